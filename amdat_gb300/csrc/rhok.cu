@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(RL_THREADS)
 
 }  // namespace amdat
 namespace amdat {
-void rhok_tc_run(amdat_ctx* ctx, const TcPlan& P, const int4* fx, int32_t n_list, int32_t n_frames,
+void rhok_tc_run(amdat_ctx* ctx, const HalfPlan& P, const int4* fx, int32_t n_list, int32_t n_frames,
                  int32_t n_k, float2* rho);
 
 struct LatticePlanDev {
@@ -515,8 +515,12 @@ struct LatticePlanDev {
   DevBuf<LatticeTile> tiles;
   DevBuf<int32_t> entry_k;
   int32_t n_tiles = 0;
-  TcPlan* tc = nullptr;  // tensor-core tiling, built at first use
-  ~LatticePlanDev() { tc_plan_free(tc); }
+  HalfPlan* half = nullptr;  // forward tensor-core tiling, built at first use
+  TcPlan* tc = nullptr;      // adjoint tensor-core tiling, built at first use
+  ~LatticePlanDev() {
+    half_plan_free(half);
+    tc_plan_free(tc);
+  }
 };
 
 void lattice_plans_free(amdat_ctx* ctx) {
@@ -683,8 +687,8 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
         int4* fx = fixed_turns(ctx, *d, e, period, d_frames);
         if (use_tensor_cores(ctx)) {
           LatticePlanDev& pw = *it->second;
-          if (!pw.tc) pw.tc = tc_plan_build(pw.kvec);
-          rhok_tc_run(ctx, *pw.tc, fx, e.n, n_frames, d->n_k, d->rho->ptr);
+          if (!pw.half) pw.half = half_plan_build(pw.kvec);
+          rhok_tc_run(ctx, *pw.half, fx, e.n, n_frames, d->n_k, d->rho->ptr);
         } else {
           dim3 grid((unsigned)P.n_tiles, (unsigned)n_frames);
           KernelTimer kt(ctx, "rhok_lattice_kernel");

@@ -34,6 +34,8 @@ namespace amdat {
 
 constexpr int SA_M = 128;                         // atoms per CTA
 constexpr int SA_KC = 32;                         // real K per chunk (16 nz, re/im)
+constexpr int SA_ROWS = 64;                       // complex rows of a tile (8 nx x 8 ny)
+constexpr int SA_NZMAX = 128;                     // widest nz window
 constexpr int SA_N = 128;                         // 64 complex rows -> Re, Im rows
 constexpr int SA_STAGES = 3;
 constexpr uint32_t SA_BPART = SA_N * SA_KC * 2;   // 8 KB: one of C hi, C lo, C' hi, C' lo
@@ -317,6 +319,71 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
     umma::tmem_dealloc(tmem, SA_TMEM_COLS);
   }
 }
+
+static bool tc_half_space(int nx, int ny, int nz) {
+  return nz > 0 || (nz == 0 && (ny > 0 || (ny == 0 && nx > 0)));
+}
+
+TcPlan* tc_plan_build(const std::vector<int32_t>& kvec) {
+  const int nk = (int)(kvec.size() / 3);
+  int nmax = 0;
+  for (int v : kvec) nmax = std::max(nmax, std::abs(v));
+  const int W = 2 * nmax + 1, H = nmax + 1;
+  std::vector<int32_t> index((size_t)W * W * H, -1);
+  for (int k = 0; k < nk; ++k) {
+    const int x = kvec[3 * k] + nmax, y = kvec[3 * k + 1] + nmax, z = kvec[3 * k + 2];
+    AMDAT_REQUIRE(z >= 0 && tc_half_space(kvec[3 * k], kvec[3 * k + 1], z), "lattice vector outside the half space");
+    index[((size_t)x * W + y) * H + z] = k;
+  }
+  // nz windows: one window of the smallest multiple of 16 covering 0..nmax, or
+  // windows of SA_NZMAX; each tile's width is trimmed to its rows' extent
+  const int nzw = std::min(SA_NZMAX, (nmax + 1 + 15) / 16 * 16);
+  const int n_zblk = (nmax + nzw) / nzw;
+  std::vector<TcTile> tiles;
+  std::vector<int32_t> entries;
+  int64_t computed = 0;
+  for (int x0 = -nmax; x0 <= nmax; x0 += 8)
+    for (int y0 = -nmax; y0 <= nmax; y0 += 8)
+      for (int zb = 0; zb < n_zblk; ++zb) {
+        int last = -1;
+        for (int r = 0; r < SA_ROWS; ++r)
+          for (int c = 0; c < nzw; ++c) {
+            const int nx = x0 + (r & 7), ny = y0 + (r >> 3), nz = zb * nzw + c;
+            if (nx > nmax || ny > nmax || nz > nmax) continue;
+            if (index[((size_t)(nx + nmax) * W + (ny + nmax)) * H + nz] >= 0) last = std::max(last, c);
+          }
+        if (last < 0) continue;
+        const int n = (last + 1 + 15) / 16 * 16;
+        const int32_t e0 = (int32_t)entries.size();
+        for (int r = 0; r < SA_ROWS; ++r)
+          for (int c = 0; c < n; ++c) {
+            const int nx = x0 + (r & 7), ny = y0 + (r >> 3), nz = zb * nzw + c;
+            int k = -1;
+            if (nx <= nmax && ny <= nmax && nz <= nmax)
+              k = index[((size_t)(nx + nmax) * W + (ny + nmax)) * H + nz];
+            entries.push_back(k);
+          }
+        tiles.push_back(TcTile{x0, y0, zb, e0, n, 0, 0, 0});
+        computed += (int64_t)SA_ROWS * n;
+      }
+  AMDAT_REQUIRE(entries.size() < (size_t)INT32_MAX, "lattice too large for the tensor-core tiling");
+  auto* p = new TcPlan();
+  p->n_tiles = (int32_t)tiles.size();
+  p->n_zblk = n_zblk;
+  p->nzw = nzw;
+  p->nmax = nmax;
+  p->entries = computed;
+  p->host_tiles = tiles;
+  p->tiles.reserve(std::max<size_t>(tiles.size(), 1));
+  p->entry_k.reserve(std::max<size_t>(entries.size(), 1));
+  if (!tiles.empty()) {
+    AMDAT_CUDA(cudaMemcpy(p->tiles.ptr, tiles.data(), tiles.size() * sizeof(TcTile), cudaMemcpyHostToDevice));
+    AMDAT_CUDA(cudaMemcpy(p->entry_k.ptr, entries.data(), entries.size() * 4, cudaMemcpyHostToDevice));
+  }
+  return p;
+}
+
+void tc_plan_free(TcPlan* p) { delete p; }
 
 size_t sa_smem_bytes(int32_t nzw) {
   const size_t a = 2 * (size_t)SA_M * 2 * nzw * 2;

@@ -90,26 +90,24 @@ def reference_shells(ms):
 
 
 def tc_tile_entries(period, kmax):
-    """Entries (complex rows x nz columns) the tensor-core tiling computes per
-    atom and frame: 8x8 (nx, ny) squares x nz windows (one window of the smallest
-    multiple of 16 covering 0..nmax, or windows of 128), each tile trimmed to a
-    multiple of 16 columns covering its rows' nz extent in the window."""
+    """Entries ((nx, ny) rows x nz columns) the tensor-core tiling computes per atom and
+    frame: squares of 8 nx >= 0 x 8 ny, each row also standing for (-nx, -ny), x nz
+    windows of equal width (at most 96), trimmed to a multiple of 8."""
     R = kmax * period / (2 * np.pi)
     nmax = int(np.floor(R))
-    nzw = min(128, (nmax + 1 + 15) // 16 * 16)
     total = 0
-    for x0 in range(-nmax, nmax + 1, 8):
+    for x0 in range(0, nmax + 1, 8):
         for y0 in range(-nmax, nmax + 1, 8):
             nx = np.arange(x0, x0 + 8)[:, None]
             ny = np.arange(y0, y0 + 8)[None, :]
             r2 = R * R - nx.astype(float) ** 2 - ny.astype(float) ** 2
-            ok = (np.abs(nx) <= nmax) & (np.abs(ny) <= nmax) & (r2 >= 0)
+            ok = (nx <= nmax) & (np.abs(ny) <= nmax) & (r2 >= 0) & ((nx > 0) | (ny >= 0))
             if not ok.any():
                 continue
-            zmax = int(np.floor(np.sqrt(r2[ok]).max()))
-            for zb in range(0, zmax // nzw + 1):
-                last = min(zmax - zb * nzw, nzw - 1)
-                total += 64 * ((last + 1 + 15) // 16 * 16)
+            ext = int(np.floor(np.sqrt(r2[ok]).max())) + 1
+            w = -(-(-(-ext // (-(-ext // 96)))) // 8) * 8
+            for z0 in range(0, ext, w):
+                total += 128 * min(w, -(-(ext - z0) // 8) * 8)
     return total
 
 
