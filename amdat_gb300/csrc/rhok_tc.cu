@@ -554,12 +554,7 @@ HalfPlan* half_plan_build(const std::vector<int32_t>& kvec) {
   int nzw = 8;
   for (int x0 = 0; x0 <= nmax; x0 += 8)
     for (int y0 = -nmax; y0 <= nmax; y0 += 8) {
-      // the vectors of (nx, ny, nz) and (-nx, -ny, nz); of nx = 0 the rows ny >= 0 carry both
-      auto images = [&](int r, int nz) {
-        const int nx = x0 + (r & 7), ny = y0 + (r >> 3);
-        if (nx == 0 && ny < 0) return make_int2(-1, -1);
-        return make_int2(index(nx, ny, nz), nx || ny ? index(-nx, -ny, nz) : -1);
-      };
+      auto images = [&](int r, int nz) { return index.images(x0 + (r & 7), y0 + (r >> 3), nz); };
       int ext = 0;  // nz extent of the 64 rows
       for (int z = nmax; z >= 0 && !ext; --z)
         for (int r = 0; r < TC_ROWS && !ext; ++r) {

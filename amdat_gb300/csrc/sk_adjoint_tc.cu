@@ -1,25 +1,34 @@
 // S(k) adjoint on the tensor cores for lattice densities (no reference
 // counterpart; the forward is Structure_Factor, src/structure_factor.cpp:201-320).
 //
-// For atom j and a tile of 64 (nx, ny) rows x n nz columns (the forward's
-// tiling), with c = u_k conj(rho_k) (u_k = 2 w_s / H_s) on the tile's vectors:
-//   T_j(row)  = sum_nz c(row, nz)      Z_j(nz)        Z_j(nz) = exp(i 2 pi nz q_z)
-//   T'_j(row) = sum_nz nz c(row, nz)   Z_j(nz)
-//   dLoss/dr_j = -(2 pi / L) Im sum_row W_j(row) (nx T, ny T, T')   W = X(nx) Y(ny)
-// T and T' are GEMMs with the atoms as M: D[atom][2m + {0,1}] = {Re, Im} T_m.
+// W(-nx,-ny) = conj W(nx,ny), so a row of half the (nx, ny) plane stands for both
+// (+-nx, +-ny).  For atom j and a tile of 64 rows (8 nx >= 0 x 8 ny) x n nz, with
+// c+- = u_k conj(rho_k) (u_k = 2 w_s / H_s) of the vectors (+-nx, +-ny, nz),
+// d = c+ - c-, e = c+ + c- and Z_j(nz) = exp(i 2 pi nz q_z) = zc + i zs:
+//   P  = sum_nz er zc - ei zs          Q  = sum_nz di zc + dr zs
+//   P' = sum_nz nz (dr zc - di zs)     Q' = sum_nz nz (ei zc + er zs)
+//   dLoss/dr_j = -(2 pi / L) sum_row (nx V, ny V, V'),
+//   V = Wr Q + Wi P, V' = Wr Q' + Wi P', W = X(nx) Y(ny):
+// eight real multiply-adds per atom and vector pair, half of the sixteen of two
+// complex sums per vector.  P, Q, P', Q' are one GEMM with the atoms as M:
+// D[atom][2m + {0,1}] = {P, Q} of row m, and {P', Q'} 128 columns on.
 // The kernel is atom-stationary: a CTA keeps Z of its 128 atoms (FP16 hi/lo,
-// K = 2 x nz window, re/im interleaved) in shared memory, streams the
-// coefficient tiles (C and nz C, FP16 hi/lo, scaled into FP16 range) in
-// chunks of 16 nz by bulk copy through a 3-stage ring, runs 12 tcgen05.mma per
-// chunk (3 split passes x 2 k-steps x {T, T'}; warp 5 issues the T and warp 6
-// the T' MMAs) into one of two TMEM accumulator pairs, and four epilogue warps (one atom per thread) read T and
-// T', form W from exact fixed-point phases and add the tile's contribution to
-// the atom's Kahan-compensated sums.  Every atom's gradient is written by one
-// thread after a fixed sequence of tiles: deterministic.
+// K = 2 x nz window, zc/zs interleaved) in shared memory, streams the
+// coefficient tiles (FP16 hi/lo, scaled into FP16 range) in chunks of 16 nz by
+// bulk copy through a ring, runs 6 tcgen05.mma of N = 256 per chunk (3 split passes
+// x 2 k-steps) into one of two 256-column accumulators, and four epilogue warps (one
+// atom per thread) read them, form W from exact fixed-point phases and add the tile's
+// contribution to the atom's Kahan-compensated sums.  Every atom's gradient is
+// written by one thread after a fixed sequence of tiles: deterministic.
 //
-// Warps 0-3: epilogue; warp 4: producer; warps 5-6: MMA issuers (T, T').  Waits are
-// bounded; a timeout makes every role stop, wait for its copies and MMAs,
-// free tensor memory and set an error word.
+// What bounds it: the MMAs' operand fetch from shared memory (A 4 KB and B 8 KB per
+// MMA).  100,000 atoms x 1.71M vectors, 2 frames: 6.41 ms, against 13.75 ms with one
+// tile per sign image and separate N = 128 MMAs for the two accumulator halves.
+//
+// Warps 0-3: epilogue; warp 4: producer; warp 5: MMA issuer.  All lanes of a warp wait
+// (one lane's wait loop would leave the warp diverged, three times the hand-off time)
+// and one elected lane issues.  Waits are bounded; a timeout makes every role stop,
+// wait for its copies and MMAs, free tensor memory and set an error word.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -36,23 +45,32 @@ constexpr int SA_M = 128;                         // atoms per CTA
 constexpr int SA_KC = 32;                         // real K per chunk (16 nz, re/im)
 constexpr int SA_ROWS = 64;                       // complex rows of a tile (8 nx x 8 ny)
 constexpr int SA_NZMAX = 128;                     // widest nz window
-constexpr int SA_N = 128;                         // 64 complex rows -> Re, Im rows
-constexpr int SA_STAGES = 3;
-constexpr uint32_t SA_BPART = SA_N * SA_KC * 2;   // 8 KB: one of C hi, C lo, C' hi, C' lo
+constexpr int SA_N = 128;                         // 64 rows -> P, Q (and P', Q') columns
+constexpr int SA_STAGES_MAX = 6;
+constexpr uint32_t SA_BPART = SA_N * SA_KC * 2;   // 8 KB: one of C hi, C' hi, C lo, C' lo
 constexpr uint32_t SA_BSTAGE = 4 * SA_BPART;      // 32 KB per chunk
-constexpr int SA_ISSUERS = 2;                    // warp 5 issues T, warp 6 issues T'
-constexpr int SA_THREADS = 32 * (5 + SA_ISSUERS);  // 224
+constexpr int SA_THREADS = 32 * 6;
+constexpr uint32_t SA_SMEM_MAX = 227 * 1024;       // dynamic shared memory per block
 constexpr uint32_t SA_WAIT = 1u << 19;             // try_wait calls of <= 1 us
-constexpr uint32_t SA_TMEM_COLS = 512;             // two (T, T') accumulator pairs
+constexpr uint32_t SA_TMEM_COLS = 512;             // two 256-column accumulators
 
 struct SaBars {
-  uint64_t full_b[SA_STAGES], empty_b[SA_STAGES];
+  uint64_t full_b[SA_STAGES_MAX], empty_b[SA_STAGES_MAX];
   uint64_t full_acc[2], empty_acc[2];
   uint64_t mma_done;
   uint32_t tmem;
   volatile int bad;
   int issued, landed;
 };
+constexpr uint32_t SA_HDR = 256;  // the barriers, behind the ring
+static_assert(sizeof(SaBars) <= SA_HDR, "the barriers must fit their slot");
+
+// shared memory: Z hi/lo of a window of nzw, then as many ring stages as fit, the barriers
+__host__ __device__ constexpr uint32_t sa_a_bytes(int nzw) { return (2u * SA_M * 2u * (uint32_t)nzw * 2u + 1023u) & ~1023u; }
+__host__ __device__ constexpr int sa_stages(int nzw) {
+  const int fit = (int)((SA_SMEM_MAX - 1024 - SA_HDR - sa_a_bytes(nzw)) / SA_BSTAGE);
+  return fit < SA_STAGES_MAX ? fit : SA_STAGES_MAX;
+}
 
 __device__ __forceinline__ void sa_split(float x, __half& hi, __half& lo) {
   hi = __float2half_rn(x);
@@ -63,15 +81,23 @@ __device__ __forceinline__ void sa_phase(int32_t ph, float* s, float* c) {
   sincospif(__fmul_rn((float)ph, 9.313225746154785e-10f), s, c);  // ph * 2^-31 turns
 }
 
+// bounded wait of a whole warp (false: give up); the block's error flag is read only
+// when the phase is not complete yet
+__device__ __forceinline__ bool sa_wait(uint64_t* mbar, uint32_t parity, volatile int* bad) {
+  if (__all_sync(0xffffffffu, umma::mbar_try_wait(mbar, parity, 1000))) return true;
+  bool ok = false;
+  for (uint32_t i = 0; i < SA_WAIT && !ok && !*bad; ++i) ok = umma::mbar_try_wait(mbar, parity, 1000);
+  return __all_sync(0xffffffffu, ok) != 0;
+}
+
 // B blobs: for frame f and chunk g (tile t = chunk_tile[g], chunk q), the
-// four 128 x 32 K-major parts [C hi | C lo | C' hi | C' lo]:
-//   row 2m   (Re T_m): k = 2z -> cr,  k = 2z+1 -> -ci
-//   row 2m+1 (Im T_m): k = 2z -> ci,  k = 2z+1 ->  cr
-// with (cr, ci) = scale * u_k conj(rho_k) of vector (nx0 + m%8, ny0 + m/8, nz),
-// and C' the same times nz (its own scale).
+// four 128 x 32 K-major parts [C hi | C' hi | C lo | C' lo]:
+//   row 2m   (P):  k = 2z -> er, k = 2z+1 -> -ei      C': nz dr, -nz di
+//   row 2m+1 (Q):  k = 2z -> di, k = 2z+1 ->  dr      C': nz ei,  nz er
+// of row (nx0 + m%8, ny0 + m/8), scaled into FP16 range (C' by its own scale).
 __global__ void __launch_bounds__(256)
     sa_blob_kernel(const float2* __restrict__ rho, int32_t n_k, const float* __restrict__ u,
-                   const TcTile* __restrict__ tiles, const int32_t* __restrict__ entry_k,
+                   const TcTile* __restrict__ tiles, const int2* __restrict__ entry_k,
                    const int32_t* __restrict__ chunk_tile, const int32_t* __restrict__ chunk_q,
                    int32_t n_chunks, int32_t nzw, float scale_c, float scale_cz,
                    unsigned char* __restrict__ blobs) {
@@ -85,26 +111,32 @@ __global__ void __launch_bounds__(256)
     const int r = e / (SA_KC / 2), z = e % (SA_KC / 2);
     const int m = r >> 1, im = r & 1;
     const int zl = q * (SA_KC / 2) + z;  // nz within the tile
-    float cr = 0.f, ci = 0.f;
+    float er = 0.f, ei = 0.f, dr = 0.f, di = 0.f;
     if (zl < T.n) {
-      const int k = entry_k[T.entry0 + m * T.n + zl];
-      if (k >= 0) {
-        const float2 rk = R[k];
-        cr = u[k] * rk.x;
-        ci = -u[k] * rk.y;
+      const int2 k = entry_k[T.entry0 + m * T.n + zl];
+      if (k.x >= 0) {
+        const float2 c = R[k.x];
+        er = dr = u[k.x] * c.x;
+        ei = di = -u[k.x] * c.y;
+      }
+      if (k.y >= 0) {
+        const float2 c = R[k.y];
+        const float cr = u[k.y] * c.x, ci = -u[k.y] * c.y;
+        er += cr, ei += ci, dr -= cr, di -= ci;
       }
     }
-    const float v0 = im ? ci : cr, v1 = im ? cr : -ci;
+    const float v0 = im ? di : er, v1 = im ? dr : -ei;
+    const float w0 = im ? ei : dr, w1 = im ? er : -di;
     const float nz = (float)(T.zblk * nzw + zl);
     __half h0, l0, h1, l1;
     const uint32_t off = umma::kmajor_offset(r, 2 * z, SA_KC);
     sa_split(v0 * scale_c, h0, l0);
     sa_split(v1 * scale_c, h1, l1);
     *reinterpret_cast<__half2*>(out + off) = __halves2half2(h0, h1);
-    *reinterpret_cast<__half2*>(out + SA_BPART + off) = __halves2half2(l0, l1);
-    sa_split(v0 * nz * scale_cz, h0, l0);
-    sa_split(v1 * nz * scale_cz, h1, l1);
-    *reinterpret_cast<__half2*>(out + 2 * SA_BPART + off) = __halves2half2(h0, h1);
+    *reinterpret_cast<__half2*>(out + 2 * SA_BPART + off) = __halves2half2(l0, l1);
+    sa_split(w0 * nz * scale_cz, h0, l0);
+    sa_split(w1 * nz * scale_cz, h1, l1);
+    *reinterpret_cast<__half2*>(out + SA_BPART + off) = __halves2half2(h0, h1);
     *reinterpret_cast<__half2*>(out + 3 * SA_BPART + off) = __halves2half2(l0, l1);
   }
 }
@@ -122,23 +154,24 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   const uint32_t a_half = (uint32_t)SA_M * KA * 2;
   unsigned char* A_hi = base;
   unsigned char* A_lo = base + a_half;
-  unsigned char* B = base + ((2 * a_half + 1023) & ~1023u);
-  SaBars& S = *reinterpret_cast<SaBars*>(B + SA_STAGES * SA_BSTAGE);
+  unsigned char* B = base + sa_a_bytes(nzw);
+  const int n_st = sa_stages(nzw);
+  SaBars& S = *reinterpret_cast<SaBars*>(B + (uint32_t)n_st * SA_BSTAGE);
   const int f = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int4* F = fx + (int64_t)f * n;
   const unsigned char* Bf = blobs + (size_t)f * n_chunks * SA_BSTAGE;
 
   if (tid == 0) {
-    for (int s = 0; s < SA_STAGES; ++s) {
+    for (int s = 0; s < n_st; ++s) {
       umma::mbar_init(&S.full_b[s], 1);
-      umma::mbar_init(&S.empty_b[s], SA_ISSUERS);
+      umma::mbar_init(&S.empty_b[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      umma::mbar_init(&S.full_acc[b], SA_ISSUERS);
-      umma::mbar_init(&S.empty_acc[b], 128);
+      umma::mbar_init(&S.full_acc[b], 1);
+      umma::mbar_init(&S.empty_acc[b], 4);
     }
-    umma::mbar_init(&S.mma_done, SA_ISSUERS);
+    umma::mbar_init(&S.mma_done, 1);
     umma::fence_mbarrier_init();
     S.bad = 0;
     S.issued = 0;
@@ -169,79 +202,77 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
 
   if (warp == 4) {
     // ---- producer: chunk blobs in tile order through the ring
-    if (lane == 0) {
-      int g = 0;
-      bool ok = true;
-      for (int ti = 0; ti < n_list_tiles && ok; ++ti) {
-        const int t = tile_list[ti];
-        const int nq = tiles[t].n / 16;
-        for (int q = 0; q < nq; ++q, ++g) {
-          const int s = g % SA_STAGES;
-          if (S.bad || !umma::mbar_wait(&S.empty_b[s], ((g / SA_STAGES) & 1) ^ 1, SA_WAIT)) {
-            ok = false;
-            break;
-          }
-          umma::mbar_expect_tx(&S.full_b[s], SA_BSTAGE);
-          umma::bulk_g2s(B + (size_t)s * SA_BSTAGE, Bf + (size_t)(tile_chunk0[t] + q) * SA_BSTAGE, SA_BSTAGE,
-                         &S.full_b[s]);
-        }
-      }
-      if (!ok) S.bad = 1;
-      S.issued = g;
-    }
-  } else if (warp == 5 || warp == 6) {
-    // ---- MMA issuers: D[atom][row] per tile, warp 5 for T and warp 6 for T'
-    // (separate accumulators, the same chunk stages: each stage and each
-    // accumulator pair is released once both issuers' MMAs on it complete)
-    const int which = warp - 5;
-    if (lane == 0) {
-      const uint32_t idesc = umma::idesc_f16_f32(SA_M, SA_N);
-      const uint32_t a_sbo = (uint32_t)(KA / 8) * 128, b_sbo = (SA_KC / 8) * 128;
-      // descriptors built once; other stages, parts and k-steps add constants
-      // to the address field (byte address >> 4)
-      const uint64_t a_hi = umma::smem_desc(umma::smem_addr(A_hi), 128, a_sbo);
-      const uint64_t a_lo = umma::smem_desc(umma::smem_addr(A_lo), 128, a_sbo);
-      const uint64_t b_desc0 = umma::smem_desc(umma::smem_addr(B), 128, b_sbo);
-      int g = 0;
-      bool ok = true;
-      for (int ti = 0; ti < n_list_tiles && ok; ++ti) {
-        const int t = tiles[tile_list[ti]].n / 16;  // chunks of this tile
-        const int buf = ti & 1;
-        if (S.bad || !umma::mbar_wait(&S.empty_acc[buf], ((ti >> 1) & 1) ^ 1, SA_WAIT)) {
+    int g = 0, st = 0;
+    uint32_t ph = 1;
+    bool ok = true;
+    for (int ti = 0; ti < n_list_tiles && ok; ++ti) {
+      const int t = tile_list[ti];
+      const int nq = tiles[t].n / 16;
+      for (int q = 0; q < nq; ++q, ++g) {
+        if (!sa_wait(&S.empty_b[st], ph, &S.bad)) {
           ok = false;
           break;
         }
-        for (int q = 0; q < t; ++q, ++g) {
-          const int s = g % SA_STAGES;
-          if (!umma::mbar_wait(&S.full_b[s], (g / SA_STAGES) & 1, SA_WAIT)) {
-            ok = false;
-            break;
-          }
-          atomicMax(&S.landed, g + 1);
-          umma::fence_after_sync();
-          const uint64_t b0 = b_desc0 + (uint64_t)(s * (SA_BSTAGE >> 4));
-          const uint64_t aq = (uint64_t)(4 * q * 8);  // K offset of chunk q: 4q core matrices of 128 B
-          {
-            const uint32_t d = tmem + (uint32_t)(buf * 256 + which * 128);
-            const uint64_t bh = b0 + (uint64_t)(2 * which * (SA_BPART >> 4));
-            const uint64_t bl = bh + (uint64_t)(SA_BPART >> 4);
-            const uint64_t ap[3] = {a_hi + aq, a_lo + aq, a_hi + aq}, bp[3] = {bl, bh, bh};
-#pragma unroll
-            for (int pass = 0; pass < 3; ++pass)
-#pragma unroll
-              for (int ks = 0; ks < 2; ++ks)
-                umma::mma_f16(d, ap[pass] + (uint64_t)(ks * 16), bp[pass] + (uint64_t)(ks * 16), idesc,
-                              (q == 0 && pass == 0 && ks == 0) ? 0u : 1u);
-          }
-          umma::mma_commit(&S.empty_b[s]);
+        if (umma::elect_one()) {
+          umma::mbar_expect_tx(&S.full_b[st], SA_BSTAGE);
+          umma::bulk_g2s(B + (size_t)st * SA_BSTAGE, Bf + (size_t)(tile_chunk0[t] + q) * SA_BSTAGE, SA_BSTAGE,
+                         &S.full_b[st]);
         }
-        if (!ok) break;
-        umma::mma_commit(&S.full_acc[buf]);
+        __syncwarp();
+        if (++st == n_st) st = 0, ph ^= 1u;
       }
-      if (!ok) S.bad = 1;
-      umma::mma_commit(&S.mma_done);
-      if (!umma::mbar_wait(&S.mma_done, 0, SA_WAIT)) S.bad = 1;
     }
+    if (!ok) S.bad = 1;
+    S.issued = g;
+  } else if (warp == 5) {
+    // ---- MMA issuer: D[atom][P Q | P' Q'] per tile
+    const uint32_t idesc = umma::idesc_f16_f32(SA_M, 2 * SA_N);
+    const uint32_t a_sbo = (uint32_t)(KA / 8) * 128, b_sbo = (SA_KC / 8) * 128;
+    // descriptors built once; other stages, parts and k-steps add constants
+    // to the address field (byte address >> 4)
+    const uint64_t a_hi = umma::smem_desc(umma::smem_addr(A_hi), 128, a_sbo);
+    const uint64_t a_lo = umma::smem_desc(umma::smem_addr(A_lo), 128, a_sbo);
+    const uint64_t b_desc0 = umma::smem_desc(umma::smem_addr(B), 128, b_sbo);
+    int g = 0, st = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int ti = 0; ti < n_list_tiles && ok; ++ti) {
+      const int nq = tiles[tile_list[ti]].n / 16;  // chunks of this tile
+      const int buf = ti & 1;
+      if (!sa_wait(&S.empty_acc[buf], ((ti >> 1) & 1) ^ 1, &S.bad)) {
+        ok = false;
+        break;
+      }
+      for (int q = 0; q < nq; ++q, ++g) {
+        if (!sa_wait(&S.full_b[st], ph, &S.bad)) {
+          ok = false;
+          break;
+        }
+        umma::fence_after_sync();
+        if (umma::elect_one()) {
+          S.landed = g + 1;
+          const uint32_t d = tmem + (uint32_t)(buf * 256);
+          const uint64_t bh = b_desc0 + (uint64_t)((uint32_t)st * (SA_BSTAGE >> 4));
+          const uint64_t bl = bh + (uint64_t)(2 * SA_BPART >> 4);
+          const uint64_t aq = (uint64_t)(4 * q * 8);  // K offset of chunk q: 4q core matrices of 128 B
+          const uint64_t ap[3] = {a_hi + aq, a_lo + aq, a_hi + aq}, bp[3] = {bl, bh, bh};
+#pragma unroll
+          for (int pass = 0; pass < 3; ++pass)
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks)
+              umma::mma_f16(d, ap[pass] + (uint64_t)(ks * 16), bp[pass] + (uint64_t)(ks * 16), idesc,
+                            (q == 0 && pass == 0 && ks == 0) ? 0u : 1u);
+          umma::mma_commit(&S.empty_b[st]);
+          if (q == nq - 1) umma::mma_commit(&S.full_acc[buf]);
+        }
+        __syncwarp();
+        if (++st == n_st) st = 0, ph ^= 1u;
+      }
+    }
+    if (!ok) S.bad = 1;
+    if (umma::elect_one()) umma::mma_commit(&S.mma_done);
+    __syncwarp();
+    if (!umma::mbar_wait(&S.mma_done, 0, SA_WAIT)) S.bad = 1;
   } else {
     // ---- epilogue: one atom per thread (TMEM lane)
     const uint32_t lanes = (uint32_t)(32 * warp) << 16;
@@ -252,9 +283,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
     for (int ti = 0; ti < n_list_tiles; ++ti) {
       const TcTile T = tiles[tile_list[ti]];
       const int buf = ti & 1;
-      bool go = true;
-      if (lane == 0) go = !S.bad && umma::mbar_wait(&S.full_acc[buf], (ti >> 1) & 1, SA_WAIT);
-      if (!__shfl_sync(0xffffffffu, go ? 1 : 0, 0)) {
+      if (!sa_wait(&S.full_acc[buf], (ti >> 1) & 1, &S.bad)) {
         ok = false;
         break;
       }
@@ -285,7 +314,8 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
         }
       }
       umma::fence_before_sync();
-      umma::mbar_arrive(&S.empty_acc[buf]);
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&S.empty_acc[buf]);
       const float part[3] = {px * inv_c, py * inv_c, pz * inv_cz};
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
@@ -309,7 +339,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   if (S.bad) {
     if (tid == 32 * 4)
       for (int g = S.landed; g < S.issued; ++g)
-        umma::mbar_wait(&S.full_b[g % SA_STAGES], (g / SA_STAGES) & 1, SA_WAIT);
+        umma::mbar_wait(&S.full_b[g % n_st], (uint32_t)(g / n_st) & 1, SA_WAIT);
     if (tid == 0) atomicExch(err, 1);
   }
   umma::fence_before_sync();
@@ -320,65 +350,49 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   }
 }
 
-static bool tc_half_space(int nx, int ny, int nz) {
-  return nz > 0 || (nz == 0 && (ny > 0 || (ny == 0 && nx > 0)));
-}
-
 TcPlan* tc_plan_build(const std::vector<int32_t>& kvec) {
-  const int nk = (int)(kvec.size() / 3);
   int nmax = 0;
   for (int v : kvec) nmax = std::max(nmax, std::abs(v));
-  const int W = 2 * nmax + 1, H = nmax + 1;
-  std::vector<int32_t> index((size_t)W * W * H, -1);
-  for (int k = 0; k < nk; ++k) {
-    const int x = kvec[3 * k] + nmax, y = kvec[3 * k + 1] + nmax, z = kvec[3 * k + 2];
-    AMDAT_REQUIRE(z >= 0 && tc_half_space(kvec[3 * k], kvec[3 * k + 1], z), "lattice vector outside the half space");
-    index[((size_t)x * W + y) * H + z] = k;
-  }
+  const LatticeIndex index(kvec, nmax);
   // nz windows: one window of the smallest multiple of 16 covering 0..nmax, or
   // windows of SA_NZMAX; each tile's width is trimmed to its rows' extent
   const int nzw = std::min(SA_NZMAX, (nmax + 1 + 15) / 16 * 16);
   const int n_zblk = (nmax + nzw) / nzw;
   std::vector<TcTile> tiles;
-  std::vector<int32_t> entries;
-  int64_t computed = 0;
-  for (int x0 = -nmax; x0 <= nmax; x0 += 8)
+  std::vector<int2> entries;
+  for (int x0 = 0; x0 <= nmax; x0 += 8)
     for (int y0 = -nmax; y0 <= nmax; y0 += 8)
       for (int zb = 0; zb < n_zblk; ++zb) {
+        auto images = [&](int r, int c) { return index.images(x0 + (r & 7), y0 + (r >> 3), zb * nzw + c); };
         int last = -1;
-        for (int r = 0; r < SA_ROWS; ++r)
-          for (int c = 0; c < nzw; ++c) {
-            const int nx = x0 + (r & 7), ny = y0 + (r >> 3), nz = zb * nzw + c;
-            if (nx > nmax || ny > nmax || nz > nmax) continue;
-            if (index[((size_t)(nx + nmax) * W + (ny + nmax)) * H + nz] >= 0) last = std::max(last, c);
+        for (int c = nzw - 1; c >= 0 && last < 0; --c)
+          for (int r = 0; r < SA_ROWS && last < 0; ++r) {
+            const int2 k = images(r, c);
+            if (k.x >= 0 || k.y >= 0) last = c;
           }
         if (last < 0) continue;
         const int n = (last + 1 + 15) / 16 * 16;
-        const int32_t e0 = (int32_t)entries.size();
+        tiles.push_back(TcTile{x0, y0, zb, (int32_t)entries.size(), n});
         for (int r = 0; r < SA_ROWS; ++r)
-          for (int c = 0; c < n; ++c) {
-            const int nx = x0 + (r & 7), ny = y0 + (r >> 3), nz = zb * nzw + c;
-            int k = -1;
-            if (nx <= nmax && ny <= nmax && nz <= nmax)
-              k = index[((size_t)(nx + nmax) * W + (ny + nmax)) * H + nz];
-            entries.push_back(k);
-          }
-        tiles.push_back(TcTile{x0, y0, zb, e0, n, 0, 0, 0});
-        computed += (int64_t)SA_ROWS * n;
+          for (int c = 0; c < n; ++c) entries.push_back(images(r, c));
+        AMDAT_REQUIRE(entries.size() < (size_t)INT32_MAX, "lattice too large for the tensor-core tiling");
       }
-  AMDAT_REQUIRE(entries.size() < (size_t)INT32_MAX, "lattice too large for the tensor-core tiling");
   auto* p = new TcPlan();
-  p->n_tiles = (int32_t)tiles.size();
-  p->n_zblk = n_zblk;
-  p->nzw = nzw;
-  p->nmax = nmax;
-  p->entries = computed;
-  p->host_tiles = tiles;
-  p->tiles.reserve(std::max<size_t>(tiles.size(), 1));
-  p->entry_k.reserve(std::max<size_t>(entries.size(), 1));
-  if (!tiles.empty()) {
-    AMDAT_CUDA(cudaMemcpy(p->tiles.ptr, tiles.data(), tiles.size() * sizeof(TcTile), cudaMemcpyHostToDevice));
-    AMDAT_CUDA(cudaMemcpy(p->entry_k.ptr, entries.data(), entries.size() * 4, cudaMemcpyHostToDevice));
+  try {
+    p->n_tiles = (int32_t)tiles.size();
+    p->n_zblk = n_zblk;
+    p->nzw = nzw;
+    p->nmax = nmax;
+    p->host_tiles = tiles;
+    p->tiles.reserve(std::max<size_t>(tiles.size(), 1));
+    p->entry_k.reserve(std::max<size_t>(entries.size(), 1));
+    if (!tiles.empty()) {
+      AMDAT_CUDA(cudaMemcpy(p->tiles.ptr, tiles.data(), tiles.size() * sizeof(TcTile), cudaMemcpyHostToDevice));
+      AMDAT_CUDA(cudaMemcpy(p->entry_k.ptr, entries.data(), entries.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    }
+  } catch (...) {
+    delete p;
+    throw;
   }
   return p;
 }
@@ -386,8 +400,7 @@ TcPlan* tc_plan_build(const std::vector<int32_t>& kvec) {
 void tc_plan_free(TcPlan* p) { delete p; }
 
 size_t sa_smem_bytes(int32_t nzw) {
-  const size_t a = 2 * (size_t)SA_M * 2 * nzw * 2;
-  return ((a + 1023) & ~(size_t)1023) + SA_STAGES * SA_BSTAGE + sizeof(SaBars) + 1024;
+  return 1024 + sa_a_bytes(nzw) + (size_t)sa_stages(nzw) * SA_BSTAGE + SA_HDR;
 }
 
 // Gradient of sum_s w_s S_raw[s] for a lattice density on the tensor cores.
@@ -397,7 +410,7 @@ void sk_adjoint_tc_run(amdat_ctx* ctx, const TcPlan& P, const int4* fx, int32_t 
                        const float2* rho, int32_t n_k, const float* d_u, float max_u, float period,
                        float* grad) {
   if (n == 0 || P.n_tiles == 0) return;
-  AMDAT_REQUIRE(sa_smem_bytes(P.nzw) <= 232448, "nz window too wide for the tensor-core adjoint");
+  AMDAT_REQUIRE(P.nzw <= SA_NZMAX && sa_stages(P.nzw) >= 2 && sa_smem_bytes(P.nzw) <= SA_SMEM_MAX, "nz window too wide for the tensor-core adjoint");
   // chunks in tile order; tile lists per nz window
   std::vector<int32_t> chunk_tile, chunk_q, tile_chunk0(P.n_tiles);
   std::vector<std::vector<int32_t>> by_zb(P.n_zblk);
@@ -411,8 +424,8 @@ void sk_adjoint_tc_run(amdat_ctx* ctx, const TcPlan& P, const int4* fx, int32_t 
     by_zb[T.zblk].push_back(t);
   }
   const int32_t n_chunks = (int32_t)chunk_tile.size();
-  // FP16 range: |c| <= max_u * n; keep the scaled values below 2^14
-  const double bound = std::max(1e-30, (double)max_u * (double)n);
+  // FP16 range: |d|, |e| <= 2 max_u * n; keep the scaled values below 2^14
+  const double bound = std::max(1e-30, 2.0 * (double)max_u * (double)n);
   const int e_c = (int)std::floor(std::log2(16384.0 / bound));
   const int e_z = e_c - (int)std::ceil(std::log2((double)P.nmax + 1.0));
   const float scale_c = (float)std::ldexp(1.0, e_c), scale_cz = (float)std::ldexp(1.0, e_z);

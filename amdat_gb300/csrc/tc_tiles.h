@@ -1,8 +1,7 @@
-// Tilings of a half-space lattice for the tensor-core kernels: the forward rho_k
-// kernel's half-plane tiles (8 nx >= 0 x 8 ny rows, each also standing for
-// (-nx, -ny), times nz windows trimmed to a multiple of 8) and the S(k) adjoint's
-// 8 x 8 (nx, ny) row blocks times nz windows, each tile trimmed to a multiple of 16
-// nz columns.
+// Tilings of a half-space lattice for the tensor-core kernels.  Both cut half the
+// (nx, ny) plane into squares of 8 nx >= 0 x 8 ny, a row standing for (nx, ny) and
+// (-nx, -ny): the forward rho_k kernel's tiles cover nz windows trimmed to a multiple
+// of 8, the S(k) adjoint's nz windows trimmed to a multiple of 16.
 #pragma once
 
 #include <cstdint>
@@ -31,6 +30,11 @@ struct LatticeIndex {
     const size_t W = 2 * (size_t)nmax + 1, H = (size_t)nmax + 1;
     return at[((size_t)(x + nmax) * W + (size_t)(y + nmax)) * H + (size_t)z];
   }
+  // the vectors (x, y, z) and (-x, -y, z) of a half-plane row x >= 0 (of x = 0 the rows y >= 0 carry both)
+  int2 images(int x, int y, int z) const {
+    if (x == 0 && y < 0) return make_int2(-1, -1);
+    return make_int2((*this)(x, y, z), x || y ? (*this)(-x, -y, z) : -1);
+  }
 };
 
 // one half-plane tile: rows (nx0 + r % 8, ny0 + r / 8), r < 64, nz = z0 + c, c < n
@@ -50,16 +54,15 @@ HalfPlan* half_plan_build(const std::vector<int32_t>& kvec);
 void half_plan_free(HalfPlan* p);
 
 struct TcTile {
-  int32_t nx0, ny0, zblk, entry0;  // entry map: 64 rows x n ints from entry0 (vector index or -1)
-  int32_t n, pad0, pad1, pad2;     // nz columns of this tile (multiple of 16, <= 128)
+  int32_t nx0, ny0, zblk, entry0;  // entry map: 64 rows x n int2 from entry0, as HalfTile's
+  int32_t n;                       // nz columns of this tile (multiple of 16, <= 128)
 };
 
 struct TcPlan {
   DevBuf<TcTile> tiles;
-  DevBuf<int32_t> entry_k;
+  DevBuf<int2> entry_k;
   std::vector<TcTile> host_tiles;
   int32_t n_tiles = 0, n_zblk = 0, nzw = 0, nmax = 0;
-  int64_t entries = 0;  // rows x columns computed per frame and atom, padding included
 };
 
 TcPlan* tc_plan_build(const std::vector<int32_t>& kvec);

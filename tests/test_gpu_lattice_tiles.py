@@ -45,3 +45,23 @@ def test_lattice_half_plane_images(eng):
         eng.wave_density_free(h)
     np.testing.assert_array_equal(out[0][..., 0], out[1][..., 0])
     np.testing.assert_array_equal(out[0][..., 1], -out[1][..., 1])
+
+
+@pytest.mark.parametrize("n_atoms,radius", [(1, 3.2), (127, 15.5), (129, 16.5), (300, 31.4), (200, 129.3)])
+def test_adjoint_tiles(eng, monkeypatch, n_atoms, radius):
+    """S(k) adjoint at the edges of its tiling (atom blocks of 128, nz chunks of 16,
+    a second nz window beyond 128) against the FP32 column kernel, 5e-4 of the
+    largest component as for the adjoint's other comparisons."""
+    box = 8.0
+    rng = np.random.default_rng(n_atoms)
+    eng.upload((rng.random((2, n_atoms, 3)) * box).astype(np.float32), [box] * 3)
+    h, nk, ns = eng.wave_density_lattice(0, radius * 2 * np.pi / box, 0.5, box, [1, 0])
+    _, off = eng.wave_density_vectors(h, nk, ns)
+    w = rng.standard_normal(ns)
+    g = eng.structure_factor_adjoint(h, off, w, 2, n_atoms)
+    monkeypatch.setenv("AMDAT_SK_ADJOINT", "columns")
+    ref = eng.structure_factor_adjoint(h, off, w, 2, n_atoms)
+    eng.wave_density_free(h)
+    assert np.isfinite(ref).all()
+    scale = np.abs(ref).max() if n_atoms > 1 else float(np.abs(w).sum() * radius)  # one atom: the gradient is zero
+    assert np.abs(g - ref).max() <= 5e-4 * scale
