@@ -5,22 +5,15 @@
 // src/van_hove_distinct.cpp:200-213, with the distance the reference meant to
 // bin: the minimum-image |r_j(t1) - r_i(t0)|).
 //
-// Every distance follows the reference's FP32 chain exactly -
-// Coordinate::length_unwrapped (src/coordinate.cpp:126-137): per axis
-// d = r_j - r_i, m = min(|d|, L - |d|); length = sqrtf((mx*mx + my*my) + mz*mz);
-// bin = int(length / bin_size) - with correctly rounded, uncontracted
-// operations, so the integer counts equal the reference's bit for bit.
-// Pairs whose squared length is safely beyond the last bin skip the square
-// root and the division; the others estimate the bin from rsqrtf and take
-// the correctly rounded chain only when the estimate lies within its error
-// bound of a bin edge.
-//
-// A block owns 512 members i of list 1 (two per thread, positions in
-// registers) and streams list 2 through shared memory in tiles of 1024.  Counts go to per-warp
-// shared-memory histograms, then once per block to the global int64
-// histogram with integer atomics (exact, order-independent).  For the RDF
-// with list1 == list2 the unordered pairs j > i are visited once and counted
-// twice (|d| is symmetric to the bit under exchange of i and j).
+// Every bin is the reference's FP32 chain exactly - Coordinate::length_unwrapped
+// (src/coordinate.cpp:126-137): per axis d = r_j - r_i, m = min(|d|, L - |d|);
+// length = sqrtf((mx*mx + my*my) + mz*mz); bin = int(length / bin_size) - with
+// correctly rounded, uncontracted operations, so the integer counts equal the
+// reference's bit for bit.  A pair's bin is first estimated (contracted square sum,
+// hardware square root, reciprocal bin size: within 1e-6 relative of the exact
+// quotient) and counted at once unless the estimate lies within its error bound of a
+// bin edge; those pairs (about one in a thousand) take the correctly rounded chain.
+// Pairs whose squared length is safely beyond the last bin are dropped before that.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -28,12 +21,13 @@
 #include <vector>
 
 #include "engine.h"
+#include "f32x2.cuh"
 
 namespace amdat {
 
 constexpr int PH_THREADS = 256;
-constexpr int PH_I_PER_BLOCK = 2 * PH_THREADS;  // two list-1 members per thread
-constexpr int PH_JT = 1024;
+constexpr int PH_WARPS = PH_THREADS / 32;
+constexpr int PH_JT = 1024;  // list-2 members staged at a time
 
 struct PHList {
   int32_t n;
@@ -62,106 +56,179 @@ struct PHParams {
   const int32_t* frame_a;  // [n_rows] frame of list-1 positions
   const int32_t* frame_b;  // [n_rows] frame of list-2 positions
   const int32_t* row_of;   // [n_rows] output row (frame index or gap)
-  int32_t symmetric;       // l1 == l2 and frame_a == frame_b: visit j > i, count 2
   float3 box;
   float bin_size;
-  float inv_bin;  // 1 / bin_size (the fast bin estimate)
+  float inv_bin;  // 1 / bin_size (the bin estimate)
+  float lim;      // 1/2 - the estimate's error bound, in bins
   float s2_cut;
   int32_t n_bins;
   unsigned long long* counts;  // [rows][n_bins]
 };
 
-// one pair: the reference's FP32 minimum-image length and its bin, counted into
-// the warp's shared histogram
-template <bool SYM>
+// the reference's chain of one pair, for estimates near a bin edge
+__device__ __noinline__ int exact_bin(float dx, float dy, float dz, float3 box, float bin_size) {
+  const float mx = min_image(dx, box.x), my = min_image(dy, box.y), mz = min_image(dz, box.z);
+  const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my)), __fmul_rn(mz, mz));
+  return (int)__fdiv_rn(__fsqrt_rn(s2), bin_size);
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Two pairs at once (packed FP32): minimum-image square sums s and bin estimates
+// x = sqrt(s) * inv_bin - 1/2, rounded to integers by adding 1.5 * 2^23: the low bits of
+// y hold the bin (PH_MAGIC_BITS + bin), r = x - bin is in [-1/2, 1/2] and its ends are
+// the bin's edges.
+constexpr float PH_MAGIC = 12582912.0f;
+constexpr uint32_t PH_MAGIC_BITS = 0x4B400000u;
+__device__ __forceinline__ void pair_estimate2(const PHParams& p, uint64_t dx, uint64_t dy, uint64_t dz, float* s,
+                                               float* y, float* r) {
+  const uint64_t d[3] = {dx, dy, dz};
+  const float L[3] = {p.box.x, p.box.y, p.box.z};
+  uint64_t s2 = 0ull;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    float d0, d1;
+    upk2(d[a], d0, d1);
+    const float m0 = fminf(fabsf(d0), __fsub_rn(L[a], fabsf(d0)));
+    const float m1 = fminf(fabsf(d1), __fsub_rn(L[a], fabsf(d1)));
+    const uint64_t m = pk2(m0, m1);
+    s2 = a == 0 ? mul2(m, m) : fma2(m, m, s2);
+  }
+  upk2(s2, s[0], s[1]);
+  const uint64_t magic = pk2(PH_MAGIC, PH_MAGIC);
+  const uint64_t x2 = fma2(pk2(sqrt_approx(s[0]), sqrt_approx(s[1])), pk2(p.inv_bin, p.inv_bin), pk2(-0.5f, -0.5f));
+  const uint64_t y2 = add2(x2, magic);
+  upk2(sub2(x2, sub2(y2, magic)), r[0], r[1]);
+  upk2(y2, y[0], y[1]);
+}
+
+// counts a pair with s < cut into the slot its estimate names; hist is the histogram's
+// shared-memory address less 4 * PH_MAGIC_BITS.  Predicated, not branched around: most
+// warps have lanes on both sides.
+__device__ __forceinline__ void count_if(float s, float cut, float y, uint32_t hist, uint32_t inc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b32 a;\n\t"
+      "setp.lt.f32 p, %0, %1;\n\t"
+      "shl.b32 a, %2, 2;\n\t"
+      "add.u32 a, a, %3;\n\t"
+      "@p red.shared.add.u32 [a], %4;\n\t}"
+      :: "f"(s), "f"(cut), "r"(__float_as_uint(y)), "r"(hist), "r"(inc));
+}
+
+// one unit of the all-pairs pass: members [i0, i0 + 256 I) of list 1 against
+// members [j0, j1) of list 2, each pair counted inc times
+struct PHUnit {
+  int32_t i0, j0, j1, inc;
+};
+
+// All-pairs pass.  A thread holds I members of list 1 in registers; list 2 streams
+// through shared memory as planes, so one 16-byte load per axis brings four members
+// for 4 I pairs.  Units are rectangles, so the work per block is even; in the
+// symmetric pass (one list, one frame) the squares on the diagonal take every ordered
+// pair once and the rectangles above it count twice (|d| is symmetric to the bit).
+// IDS: frames differ, so an atom's own pair has to be told by its index; within one
+// frame it is the pair at zero distance, which the exact path checks.
+// Bound: instruction issue, 23 per pair and warp at 69 % of the issue slots; the
+// histogram's shared-memory atomics take 2.5 wavefronts per 32 pairs (half the pairs in
+// range).  g(r) of 64,000 atoms to half the box, 50 frames: 70.6 ms, against 163 ms with
+// 35 instructions per pair (scalar chain, a branch around every count) over blocks of a
+// triangle.
+template <int I, bool IDS>
+__global__ void __launch_bounds__(PH_THREADS)
+    pair_hist_kernel(PHParams p, const PHUnit* __restrict__ units) {
+  extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins + 1], the last slot past the end
+  __shared__ __align__(16) float sx[PH_JT], sy[PH_JT], sz[PH_JT];
+  __shared__ __align__(16) int sid[PH_JT];
+  const PHUnit U = units[blockIdx.x];
+  const int q = blockIdx.y, nb1 = p.n_bins + 1;
+  const float* A = p.w + (int64_t)p.frame_a[q] * 3 * p.n_pad;
+  const float* B = p.w + (int64_t)p.frame_b[q] * 3 * p.n_pad;
+  unsigned int* whist = sh_hist + (threadIdx.x >> 5) * nb1;
+  const uint32_t hist = (uint32_t)__cvta_generic_to_shared(whist) - 4u * PH_MAGIC_BITS;
+  for (int b = threadIdx.x; b < PH_WARPS * nb1; b += PH_THREADS) sh_hist[b] = 0u;
+  const float nan = __int_as_float(0x7fffffff);  // members past the end: never within the cut
+  uint64_t xi[I], yi[I], zi[I];
+  int ai[I];
+#pragma unroll
+  for (int k = 0; k < I; ++k) {
+    const int i = U.i0 + k * PH_THREADS + threadIdx.x;
+    const bool live = i < p.l1.n;
+    ai[k] = live ? member(p.l1, i) : -1;
+    const float x = live ? A[ai[k]] : nan, y = live ? A[p.n_pad + ai[k]] : nan, z = live ? A[2 * p.n_pad + ai[k]] : nan;
+    xi[k] = pk2(x, x), yi[k] = pk2(y, y), zi[k] = pk2(z, z);
+  }
+  for (int jt = U.j0; jt < U.j1; jt += PH_JT) {
+    const int nj = min(PH_JT, U.j1 - jt);
+    __syncthreads();
+    for (int t = threadIdx.x; t < ((nj + 3) & ~3); t += PH_THREADS) {
+      const bool live = t < nj;
+      const int aj = live ? member(p.l2, jt + t) : -1;
+      sx[t] = live ? B[aj] : nan;
+      sy[t] = live ? B[p.n_pad + aj] : nan;
+      sz[t] = live ? B[2 * p.n_pad + aj] : nan;
+      sid[t] = aj;
+    }
+    __syncthreads();
+    for (int t = 0; t < nj; t += 4) {
+      const float4 X = *reinterpret_cast<const float4*>(sx + t), Y = *reinterpret_cast<const float4*>(sy + t),
+                   Z = *reinterpret_cast<const float4*>(sz + t);
+      const uint64_t xj[2] = {pk2(X.x, X.y), pk2(X.z, X.w)}, yj[2] = {pk2(Y.x, Y.y), pk2(Y.z, Y.w)},
+                     zj[2] = {pk2(Z.x, Z.y), pk2(Z.z, Z.w)};
+      int4 id = make_int4(0, 0, 0, 0);
+      if (IDS) id = *reinterpret_cast<const int4*>(sid + t);
+      const int ids[4] = {id.x, id.y, id.z, id.w};
+#pragma unroll
+      for (int k = 0; k < I; ++k) {
+        float s[4], y[4], r[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          pair_estimate2(p, sub2(xj[h], xi[k]), sub2(yj[h], yi[k]), sub2(zj[h], zi[k]), s + 2 * h, y + 2 * h, r + 2 * h);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (IDS && ids[e] == ai[k]) s[e] = nan;
+          count_if(s[e], p.s2_cut, y[e], hist, (uint32_t)U.inc);
+        }
+        // estimates within their error bound of a bin edge: the counts are put right
+        // (and an atom's own pair, at zero distance, taken out)
+        if (fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3]))) >= p.lim) {
+          const float x = __uint_as_float((uint32_t)xi[k]), yy = __uint_as_float((uint32_t)yi[k]), z = __uint_as_float((uint32_t)zi[k]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (!(s[e] < p.s2_cut) || fabsf(r[e]) < p.lim) continue;
+            const int est = (int)(__float_as_uint(y[e]) - PH_MAGIC_BITS);
+            const int b = exact_bin(__fsub_rn(sx[t + e], x), __fsub_rn(sy[t + e], yy), __fsub_rn(sz[t + e], z), p.box, p.bin_size);
+            const bool self = sid[t + e] == ai[k];
+            if (b == est && !self) continue;
+            atomicSub(whist + est, (unsigned int)U.inc);
+            if (!self && b >= 0 && b < p.n_bins) atomicAdd(whist + b, (unsigned int)U.inc);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  unsigned long long* dst = p.counts + (int64_t)p.row_of[q] * p.n_bins;
+  for (int b = threadIdx.x; b < p.n_bins; b += PH_THREADS) {
+    unsigned long long s = 0;
+    for (int w = 0; w < PH_WARPS; ++w) s += sh_hist[w * nb1 + b];
+    if (s) atomicAdd(dst + b, s);
+  }
+}
+
+// ordered pairs of the cell pass: the short exact branch
 __device__ __forceinline__ void pair_term(const PHParams& p, float4 c, float xi, float yi, float zi,
-                                          unsigned int* hist, unsigned int inc) {
+                                          unsigned int* hist) {
   const float mx = min_image(__fsub_rn(c.x, xi), p.box.x);
   const float my = min_image(__fsub_rn(c.y, yi), p.box.y);
   const float mz = min_image(__fsub_rn(c.z, zi), p.box.z);
   const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my)), __fmul_rn(mz, mz));
   if (s2 < p.s2_cut) {
-    // bin = int(sqrt_rn(s2) / bin_size), the reference's chain.  First from
-    // rsqrtf (<= 2 ulp) and the reciprocal bin size: within 1e-6 relative of
-    // the exact quotient, so its integer part is the exact one unless the
-    // quotient lies within that margin of an integer; those pairs (and s2 = 0)
-    // take the correctly rounded chain.  (The symmetric RDF pass, where most
-    // pairs are in range; the sparse distinct van Hove pass keeps the short
-    // exact branch.)
-    int b;
-    if (SYM) {
-      const float x = __fmul_rn(__fmul_rn(s2, rsqrtf(s2)), p.inv_bin);
-      b = (int)x;
-      const float frac = __fsub_rn(x, (float)b);
-      const float margin = fmaf(x, 1e-6f, 1e-6f);
-      if (!(s2 > 0.f) || frac <= margin || frac >= 1.f - margin)
-        b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-    } else {
-      b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-    }
-    if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, inc);
-  }
-}
-
-// SYM: the symmetric pass (list1 == list2, one frame): j > i, each pair counted
-// twice.  A thread holds two members of list 1 (i and i + PH_THREADS) in
-// registers, so each staged list-2 position (one 16-byte shared load: x, y, z
-// and the atom index) serves two pairs.
-template <bool SYM>
-__global__ void __launch_bounds__(PH_THREADS)
-    pair_hist_kernel(PHParams p) {
-  extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins]
-  __shared__ float4 sj[PH_JT];               // x, y, z, atom index bits
-  const int q = blockIdx.y;
-  const float* A = p.w + (int64_t)p.frame_a[q] * 3 * p.n_pad;
-  const float* B = p.w + (int64_t)p.frame_b[q] * 3 * p.n_pad;
-  const int warp = threadIdx.x >> 5;
-  unsigned int* hist = sh_hist + warp * p.n_bins;
-  for (int b = threadIdx.x; b < 8 * p.n_bins; b += blockDim.x) sh_hist[b] = 0u;
-  const int i0 = blockIdx.x * PH_I_PER_BLOCK;
-  const int ia = i0 + threadIdx.x, ib = ia + PH_THREADS;
-  const bool la = ia < p.l1.n, lb = ib < p.l1.n;
-  int aa = -1, ab = -1;
-  float xa = 0.f, ya = 0.f, za = 0.f, xb = 0.f, yb = 0.f, zb = 0.f;
-  if (la) {
-    aa = member(p.l1, ia);
-    xa = A[aa];
-    ya = A[p.n_pad + aa];
-    za = A[2 * p.n_pad + aa];
-  }
-  if (lb) {
-    ab = member(p.l1, ib);
-    xb = A[ab];
-    yb = A[p.n_pad + ab];
-    zb = A[2 * p.n_pad + ab];
-  }
-  const unsigned int inc = SYM ? 2u : 1u;
-  const int j_begin = SYM ? i0 : 0;
-  __syncthreads();
-  for (int j0 = j_begin; j0 < p.l2.n; j0 += PH_JT) {
-    const int nj = min(PH_JT, p.l2.n - j0);
-    __syncthreads();
-    for (int t = threadIdx.x; t < nj; t += blockDim.x) {
-      const int aj = member(p.l2, j0 + t);
-      sj[t] = make_float4(B[aj], B[p.n_pad + aj], B[2 * p.n_pad + aj], __int_as_float(aj));
-    }
-    __syncthreads();
-    if (!la) continue;  // lb implies la
-    // j > i for the symmetric pass (i != j is implied), i != j checked otherwise
-    const int t_begin = SYM ? max(0, ia + 1 - j0) : 0;
-    const int t_b = SYM ? ib + 1 - j0 : 0;  // the second member's first t
-    for (int t = t_begin; t < nj; ++t) {
-      const float4 c = sj[t];
-      if (SYM || __float_as_int(c.w) != aa) pair_term<SYM>(p, c, xa, ya, za, hist, inc);
-      if (lb && (SYM ? t >= t_b : __float_as_int(c.w) != ab)) pair_term<SYM>(p, c, xb, yb, zb, hist, inc);
-    }
-  }
-  __syncthreads();
-  unsigned long long* dst = p.counts + (int64_t)p.row_of[q] * p.n_bins;
-  for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x) {
-    unsigned long long s = 0;
-    for (int w = 0; w < 8; ++w) s += sh_hist[w * p.n_bins + b];
-    if (s) atomicAdd(dst + b, s);
+    const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
+    if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
   }
 }
 
@@ -286,7 +353,7 @@ __global__ void __launch_bounds__(PH_THREADS)
           const int k1 = __ldg(S2 + c + 1);
           for (int k = __ldg(S2 + c); k < k1; ++k) {
             const float4 cj = __ldg(P2 + k);
-            if (__float_as_int(cj.w) != ai) pair_term<false>(p, cj, pi.x, pi.y, pi.z, hist, 1u);
+            if (__float_as_int(cj.w) != ai) pair_term(p, cj, pi.x, pi.y, pi.z, hist);
           }
         }
       }
@@ -333,10 +400,13 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   p.frame_a = (const int32_t*)(base + o_fa);
   p.frame_b = (const int32_t*)(base + o_fb);
   p.row_of = (const int32_t*)(base + o_row);
-  p.symmetric = symmetric ? 1 : 0;
   p.box = make_float3(ctx->box[0], ctx->box[1], ctx->box[2]);
   p.bin_size = max_distance / (float)n_bins;
   p.inv_bin = 1.0f / p.bin_size;
+  // the estimate's error, in bins: the square sums differ by 6 roundings of 2^-24 (3 after
+  // the root), the root by 2^-23 and 2^-24 (the chain's), the quotient by the chain's
+  // 2^-24, the reciprocal's 2^-24 and the product's 2^-24: 9 roundings of the bin number
+  p.lim = 0.5f - 9.0f * 5.9604645e-8f * (float)(n_bins + 1) - 1e-6f;
   // squared lengths at or above this are past the last bin for sure
   const double cut = (double)max_distance * (1.0 + 1e-5);
   p.s2_cut = (float)(cut * cut);
@@ -436,16 +506,40 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     check_launch("pair_hist_cells_kernel");
     count_launch(ctx);
   } else if (n_q && l1.n > 0 && l2.n > 0) {
-    const size_t shm = (size_t)8 * n_bins * 4;
-    auto kern = symmetric ? pair_hist_kernel<true> : pair_hist_kernel<false>;
-    if (shm > 48 * 1024)
-      AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     AMDAT_REQUIRE(n_q <= 65535, "at most 65535 frames or time pairs per call");
-    dim3 grid((unsigned)ceil_div(l1.n, PH_I_PER_BLOCK), (unsigned)n_q);
-    KernelTimer kt(ctx, "pair_hist_kernel");
-    kern<<<grid, PH_THREADS, shm, ctx->stream>>>(p);
-    check_launch("pair_hist_kernel");
-    count_launch(ctx);
+    // units of 256 I members by up to seg list-2 members: wide ones while they fill
+    // the chip six times over, then fewer members per thread and shorter segments
+    const bool ids = fa != fb;
+    const int64_t want = 6 * (int64_t)ctx->n_sm;
+    auto count_units = [&](int I, int seg) {
+      const int64_t ib = ceil_div(l1.n, 256 * I), js = ceil_div(l2.n, seg);
+      return (symmetric ? (ib * js + ib) / 2 : ib * js) * (int64_t)n_q;
+    };
+    int I = 4, seg = 8192;
+    while (seg > 1024 && count_units(I, seg) < want) seg /= 2;
+    while (I > 1 && count_units(I, seg) < want) I /= 2;
+    while (seg > 128 && count_units(I, seg) < want) seg /= 2;
+    std::vector<PHUnit> units;
+    for (int i0 = 0; i0 < l1.n; i0 += 256 * I) {
+      const int i1 = std::min(l1.n, i0 + 256 * I);
+      if (symmetric)
+        for (int j = i0; j < i1; j += seg) units.push_back(PHUnit{i0, j, std::min(i1, j + seg), 1});
+      for (int j = symmetric ? i1 : 0; j < l2.n; j += seg)
+        units.push_back(PHUnit{i0, j, std::min(l2.n, j + seg), symmetric ? 2 : 1});
+    }
+    PHUnit* d_units = (PHUnit*)ctx->scratch2.reserve(units.size() * sizeof(PHUnit));
+    AMDAT_CUDA(cudaMemcpyAsync(d_units, units.data(), units.size() * sizeof(PHUnit), cudaMemcpyHostToDevice, ctx->stream));
+    const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
+    auto launch = [&](auto kern) {
+      if (shm > 32 * 1024)
+        AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+      KernelTimer kt(ctx, "pair_hist_kernel");
+      kern<<<dim3((unsigned)units.size(), (unsigned)n_q), PH_THREADS, shm, ctx->stream>>>(p, d_units);
+      check_launch("pair_hist_kernel");
+      count_launch(ctx);
+    };
+    if (ids) I == 4 ? launch(pair_hist_kernel<4, true>) : I == 2 ? launch(pair_hist_kernel<2, true>) : launch(pair_hist_kernel<1, true>);
+    else I == 4 ? launch(pair_hist_kernel<4, false>) : I == 2 ? launch(pair_hist_kernel<2, false>) : launch(pair_hist_kernel<1, false>);
   }
   AMDAT_CUDA(cudaMemcpyAsync(counts, base + o_cnt, n_out * 8,
                              out_flags == AMDAT_OUT_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
