@@ -119,6 +119,55 @@ __device__ __forceinline__ void count_if(float s, float cut, float y, uint32_t h
       :: "f"(s), "f"(cut), "r"(__float_as_uint(y)), "r"(hist), "r"(inc));
 }
 
+// how an atom's own pair is left out
+enum { PH_SELF_ZERO, PH_SELF_IDS, PH_SELF_LATER };  // one frame: the pair at zero distance; by index; by the caller
+
+// One list-1 member (x, y, z duplicated in packed pairs) against the four staged list-2
+// members at sx[0..3], ...: every pair within the cut is counted into its estimated
+// slot, then the counts of estimates within their error bound of a bin edge are put
+// right by the exact chain.
+template <int SELF>
+__device__ __forceinline__ void count4(const PHParams& p, uint64_t xi, uint64_t yi, uint64_t zi, int ai, float4 X, float4 Y,
+                                       float4 Z, const float* sx, const float* sy, const float* sz, const int* sid,
+                                       uint32_t hist, unsigned int* whist, uint32_t inc) {
+  float s[4], y[4], r[4];
+  pair_estimate2(p, sub2(pk2(X.x, X.y), xi), sub2(pk2(Y.x, Y.y), yi), sub2(pk2(Z.x, Z.y), zi), s, y, r);
+  pair_estimate2(p, sub2(pk2(X.z, X.w), xi), sub2(pk2(Y.z, Y.w), yi), sub2(pk2(Z.z, Z.w), zi), s + 2, y + 2, r + 2);
+  if (SELF == PH_SELF_IDS) {
+    const int4 id = *reinterpret_cast<const int4*>(sid);
+    const float nan = __int_as_float(0x7fffffff);
+    if (id.x == ai) s[0] = nan;
+    if (id.y == ai) s[1] = nan;
+    if (id.z == ai) s[2] = nan;
+    if (id.w == ai) s[3] = nan;
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) count_if(s[e], p.s2_cut, y[e], hist, inc);
+  if (fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3]))) >= p.lim) {
+    const float xs = __uint_as_float((uint32_t)xi), ys = __uint_as_float((uint32_t)yi), zs = __uint_as_float((uint32_t)zi);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (!(s[e] < p.s2_cut) || fabsf(r[e]) < p.lim) continue;
+      const int est = (int)(__float_as_uint(y[e]) - PH_MAGIC_BITS);
+      const int b = exact_bin(__fsub_rn(sx[e], xs), __fsub_rn(sy[e], ys), __fsub_rn(sz[e], zs), p.box, p.bin_size);
+      const bool self = SELF == PH_SELF_ZERO && sid[e] == ai;
+      if (b == est && !self) continue;
+      atomicSub(whist + est, inc);
+      if (!self && b >= 0 && b < p.n_bins) atomicAdd(whist + b, inc);
+    }
+  }
+}
+
+// a block's per-warp histograms added to the row's counts
+__device__ __forceinline__ void flush_counts(const PHParams& p, const unsigned int* hist, int row) {
+  unsigned long long* dst = p.counts + (int64_t)row * p.n_bins;
+  for (int b = threadIdx.x; b < p.n_bins; b += PH_THREADS) {
+    unsigned long long s = 0;
+    for (int w = 0; w < PH_WARPS; ++w) s += hist[w * (p.n_bins + 1) + b];
+    if (s) atomicAdd(dst + b, s);
+  }
+}
+
 // one unit of the all-pairs pass: members [i0, i0 + 256 I) of list 1 against
 // members [j0, j1) of list 2, each pair counted inc times
 struct PHUnit {
@@ -130,14 +179,12 @@ struct PHUnit {
 // for 4 I pairs.  Units are rectangles, so the work per block is even; in the
 // symmetric pass (one list, one frame) the squares on the diagonal take every ordered
 // pair once and the rectangles above it count twice (|d| is symmetric to the bit).
-// IDS: frames differ, so an atom's own pair has to be told by its index; within one
-// frame it is the pair at zero distance, which the exact path checks.
 // Bound: instruction issue, 23 per pair and warp at 69 % of the issue slots; the
 // histogram's shared-memory atomics take 2.5 wavefronts per 32 pairs (half the pairs in
 // range).  g(r) of 64,000 atoms to half the box, 50 frames: 70.6 ms, against 163 ms with
 // 35 instructions per pair (scalar chain, a branch around every count) over blocks of a
 // triangle.
-template <int I, bool IDS>
+template <int I, int SELF>
 __global__ void __launch_bounds__(PH_THREADS)
     pair_hist_kernel(PHParams p, const PHUnit* __restrict__ units) {
   extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins + 1], the last slot past the end
@@ -176,101 +223,67 @@ __global__ void __launch_bounds__(PH_THREADS)
     for (int t = 0; t < nj; t += 4) {
       const float4 X = *reinterpret_cast<const float4*>(sx + t), Y = *reinterpret_cast<const float4*>(sy + t),
                    Z = *reinterpret_cast<const float4*>(sz + t);
-      const uint64_t xj[2] = {pk2(X.x, X.y), pk2(X.z, X.w)}, yj[2] = {pk2(Y.x, Y.y), pk2(Y.z, Y.w)},
-                     zj[2] = {pk2(Z.x, Z.y), pk2(Z.z, Z.w)};
-      int4 id = make_int4(0, 0, 0, 0);
-      if (IDS) id = *reinterpret_cast<const int4*>(sid + t);
-      const int ids[4] = {id.x, id.y, id.z, id.w};
 #pragma unroll
-      for (int k = 0; k < I; ++k) {
-        float s[4], y[4], r[4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          pair_estimate2(p, sub2(xj[h], xi[k]), sub2(yj[h], yi[k]), sub2(zj[h], zi[k]), s + 2 * h, y + 2 * h, r + 2 * h);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (IDS && ids[e] == ai[k]) s[e] = nan;
-          count_if(s[e], p.s2_cut, y[e], hist, (uint32_t)U.inc);
-        }
-        // estimates within their error bound of a bin edge: the counts are put right
-        // (and an atom's own pair, at zero distance, taken out)
-        if (fmaxf(fmaxf(fabsf(r[0]), fabsf(r[1])), fmaxf(fabsf(r[2]), fabsf(r[3]))) >= p.lim) {
-          const float x = __uint_as_float((uint32_t)xi[k]), yy = __uint_as_float((uint32_t)yi[k]), z = __uint_as_float((uint32_t)zi[k]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (!(s[e] < p.s2_cut) || fabsf(r[e]) < p.lim) continue;
-            const int est = (int)(__float_as_uint(y[e]) - PH_MAGIC_BITS);
-            const int b = exact_bin(__fsub_rn(sx[t + e], x), __fsub_rn(sy[t + e], yy), __fsub_rn(sz[t + e], z), p.box, p.bin_size);
-            const bool self = sid[t + e] == ai[k];
-            if (b == est && !self) continue;
-            atomicSub(whist + est, (unsigned int)U.inc);
-            if (!self && b >= 0 && b < p.n_bins) atomicAdd(whist + b, (unsigned int)U.inc);
-          }
-        }
-      }
+      for (int k = 0; k < I; ++k)
+        count4<SELF>(p, xi[k], yi[k], zi[k], ai[k], X, Y, Z, sx + t, sy + t, sz + t, sid + t, hist, whist, (uint32_t)U.inc);
     }
   }
   __syncthreads();
-  unsigned long long* dst = p.counts + (int64_t)p.row_of[q] * p.n_bins;
-  for (int b = threadIdx.x; b < p.n_bins; b += PH_THREADS) {
-    unsigned long long s = 0;
-    for (int w = 0; w < PH_WARPS; ++w) s += sh_hist[w * nb1 + b];
-    if (s) atomicAdd(dst + b, s);
-  }
-}
-
-// ordered pairs of the cell pass: the short exact branch
-__device__ __forceinline__ void pair_term(const PHParams& p, float4 c, float xi, float yi, float zi,
-                                          unsigned int* hist) {
-  const float mx = min_image(__fsub_rn(c.x, xi), p.box.x);
-  const float my = min_image(__fsub_rn(c.y, yi), p.box.y);
-  const float mz = min_image(__fsub_rn(c.z, zi), p.box.z);
-  const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my)), __fmul_rn(mz, mz));
-  if (s2 < p.s2_cut) {
-    const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-    if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
-  }
+  flush_counts(p, sh_hist, p.row_of[q]);
 }
 
 // ---------------------------------------------------------------------------
-// cell lists for short-range ordered pair loops (the distinct van Hove pass and
-// RDFs of two different lists): when every box axis holds at least three cells
-// no narrower than the last bin edge, a pair that can fall in a bin has its
-// atoms in the same or neighbouring cells (periodic).  Per frame the list's
-// atoms are counted into cells, the counts scanned and the atoms scattered in
-// cell order as (x, y, z, atom index bits); a thread takes one list-1 member in
-// cell order at t0 and visits the 27 cells around it in the list-2 cells at t1.
-// Distances and bins are the exact chain of pair_term, counts are integer
-// atomics, so the counts equal the all-pairs kernel's bit for bit.
+// cell pass for short-range ordered pair loops (the distinct van Hove pass and RDFs
+// of two different lists), when every box axis holds at least three cutoffs.  Per
+// frame each list's atoms are counted into cells, the counts scanned and the atoms
+// scattered in cell order as (x, y, z, atom index bits).
+// List 1 is ordered along pencils: (y, z) squares about as wide as 32 atoms' cube,
+// filled with thin x cells, neighbouring pencils run in opposite directions; 32
+// consecutive atoms then fill a compact box.  A warp takes such a group.
+// List 2 is ordered in narrower pencils of x cells.  Of every pencil whose distance to
+// the group's bounding box is within the cutoff, the warp gathers the run of x cells
+// the cutoff reaches into shared memory, and each lane goes through the gathered
+// atoms (count4).  A pair within the last bin's edge is visited exactly once, so the
+// counts equal the all-pairs pass's.
+// Bound: instruction issue, as the all-pairs pass; a visited pair in five or so is
+// within the cutoff.  (One atom per thread walking its own 27 cells of the cutoff's
+// width visits twice as many pairs through scattered 16-byte loads.)
 // ---------------------------------------------------------------------------
-struct PHCells {
-  int3 nc;
-  float3 lo, inv_cell;
+struct PHGrid {
+  int3 n;
+  float3 lo, cell, inv;
   int32_t n_cells;
-  const int32_t* start;  // [slot][n_cells + 1]
-  const float4* pos;     // [slot][n]: members in cell order
-  int32_t n;             // members per slot
+  int32_t snake;  // x runs back in every other row of cells, rows run back in every other layer
+  float tol;      // atoms further than this outside the box flag the call
 };
 
 __device__ __forceinline__ int ph_cell_axis(float x, float lo, float inv_cell, int n) {
-  const int c = (int)((x - lo) * inv_cell);
+  const int c = (int)floorf((x - lo) * inv_cell);
   return min(max(c, 0), n - 1);
 }
 
 // members of list l at frame frames[s] counted into the cells of slot s
 __global__ void ph_cell_count_kernel(const float* __restrict__ w, int64_t n_pad, PHList l,
-                                     const int32_t* __restrict__ frames, int3 nc, float3 lo, float3 inv_cell,
-                                     int32_t* __restrict__ cell_of, int32_t* __restrict__ count) {
+                                     const int32_t* __restrict__ frames, PHGrid g,
+                                     int32_t* __restrict__ cell_of, int32_t* __restrict__ count, int32_t* __restrict__ out) {
   const int s = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= l.n) return;
   const float* P = w + (int64_t)frames[s] * 3 * n_pad;
   const int a = member(l, i);
-  const int c = (ph_cell_axis(P[2 * n_pad + a], lo.z, inv_cell.z, nc.z) * nc.y +
-                 ph_cell_axis(P[n_pad + a], lo.y, inv_cell.y, nc.y)) * nc.x +
-                ph_cell_axis(P[a], lo.x, inv_cell.x, nc.x);
+  const float x = P[a], y = P[n_pad + a], z = P[2 * n_pad + a];
+  int cx = ph_cell_axis(x, g.lo.x, g.inv.x, g.n.x), cy = ph_cell_axis(y, g.lo.y, g.inv.y, g.n.y);
+  const int cz = ph_cell_axis(z, g.lo.z, g.inv.z, g.n.z);
+  if (g.snake) {
+    if (cz & 1) cy = g.n.y - 1 - cy;
+    if ((cz * g.n.y + cy) & 1) cx = g.n.x - 1 - cx;
+  }
+  const int c = (cz * g.n.y + cy) * g.n.x + cx;
   cell_of[(int64_t)s * l.n + i] = c;
-  atomicAdd(count + (int64_t)s * nc.x * nc.y * nc.z + c, 1);
+  atomicAdd(count + (int64_t)s * g.n_cells + c, 1);
+  const float ex = fmaxf(g.lo.x - x, x - g.lo.x - g.cell.x * g.n.x), ey = fmaxf(g.lo.y - y, y - g.lo.y - g.cell.y * g.n.y),
+              ez = fmaxf(g.lo.z - z, z - g.lo.z - g.cell.z * g.n.z);
+  if (!(fmaxf(ex, fmaxf(ey, ez)) <= g.tol)) *out = 1;
 }
 
 // exclusive scan of one slot's cell counts (one block per slot) into start and
@@ -320,52 +333,175 @@ __global__ void ph_cell_scatter_kernel(const float* __restrict__ w, int64_t n_pa
   pos[(int64_t)s * l.n + k] = make_float4(P[a], P[n_pad + a], P[2 * n_pad + a], __int_as_float(a));
 }
 
-// ordered pairs (i at t0 from list 1, j != i at t1 from list 2) within the 27
-// cells around i; slot_a / slot_b give each row's cell slots
-__global__ void __launch_bounds__(PH_THREADS)
-    pair_hist_cells_kernel(PHParams p, PHCells C1, PHCells C2, const int32_t* __restrict__ slot_a,
-                           const int32_t* __restrict__ slot_b) {
-  extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins]
-  const int q = blockIdx.y;
-  const int warp = threadIdx.x >> 5;
-  unsigned int* hist = sh_hist + warp * p.n_bins;
-  for (int b = threadIdx.x; b < 8 * p.n_bins; b += blockDim.x) sh_hist[b] = 0u;
+__device__ __forceinline__ int wrap_index(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
+
+// group minimum and maximum of a coordinate (lanes without an atom pass NaN)
+__device__ __forceinline__ void warp_range(float v, float& lo, float& hi) {
+  lo = hi = v;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+  }
+}
+
+constexpr int PG_TILE = 128;           // gathered list-2 members gone through at a time
+constexpr int PG_BUF = PG_TILE + 32;
+
+struct PHGroups {
+  const float4* pos1;     // [slot][n1]: list-1 members in pencil order
+  int32_t n1, per_warp;   // groups per warp
+  const float4* pos2;     // [slot][n2]
+  const int32_t* start2;  // [slot][n_cells + 1]
+  int32_t n2;
+  PHGrid g2;
+  const int32_t* slot_a;  // slots of each row
+  const int32_t* slot_b;
+  float reach;            // cutoff with its margin
+  int32_t same;           // one list: each atom's own pair is taken out at the end
+  const int32_t* outside;  // set: some atom lies outside the box, nothing is counted
+};
+
+template <int SELF>
+__global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p, PHGroups G) {
+  extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins + 1]
+  __shared__ __align__(16) float sbuf[PH_WARPS][3][PG_BUF];
+  __shared__ __align__(16) int sids[PH_WARPS][SELF == PH_SELF_IDS ? PG_BUF : 4];
+  if (*G.outside) return;  // cell indexes would not wrap into the grid
+  const int q = blockIdx.y, nb1 = p.n_bins + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned int* whist = sh_hist + warp * nb1;
+  const uint32_t hist = (uint32_t)__cvta_generic_to_shared(whist) - 4u * PH_MAGIC_BITS;
+  for (int b = threadIdx.x; b < PH_WARPS * nb1; b += PH_THREADS) sh_hist[b] = 0u;
   __syncthreads();
-  const int i = blockIdx.x * PH_THREADS + threadIdx.x;
-  if (i < C1.n) {
-    const float4 pi = C1.pos[(int64_t)slot_a[q] * C1.n + i];
+  const float4* P1 = G.pos1 + (int64_t)G.slot_a[q] * G.n1;
+  const float4* P2 = G.pos2 + (int64_t)G.slot_b[q] * G.n2;
+  const int32_t* S2 = G.start2 + (int64_t)G.slot_b[q] * (G.g2.n_cells + 1);
+  const PHGrid& g = G.g2;
+  const float nan = __int_as_float(0x7fffffff);
+  float *bx = sbuf[warp][0], *by = sbuf[warp][1], *bz = sbuf[warp][2];
+  int* bid = sids[warp];
+  for (int gi = 0; gi < G.per_warp; ++gi) {
+    const int i0 = 32 * ((blockIdx.x * G.per_warp + gi) * PH_WARPS + warp);
+    if (i0 >= G.n1) break;
+    const bool live = i0 + lane < G.n1;
+    const float4 pi = live ? P1[i0 + lane] : make_float4(nan, nan, nan, __int_as_float(-1));
     const int ai = __float_as_int(pi.w);
-    const int32_t* S2 = C2.start + (int64_t)slot_b[q] * (C2.n_cells + 1);
-    const float4* P2 = C2.pos + (int64_t)slot_b[q] * C2.n;
-    const int cx = ph_cell_axis(pi.x, C2.lo.x, C2.inv_cell.x, C2.nc.x);
-    const int cy = ph_cell_axis(pi.y, C2.lo.y, C2.inv_cell.y, C2.nc.y);
-    const int cz = ph_cell_axis(pi.z, C2.lo.z, C2.inv_cell.z, C2.nc.z);
-    for (int dz = -1; dz <= 1; ++dz) {
-      int z = cz + dz;
-      z += z < 0 ? C2.nc.z : (z >= C2.nc.z ? -C2.nc.z : 0);
-      for (int dy = -1; dy <= 1; ++dy) {
-        int y = cy + dy;
-        y += y < 0 ? C2.nc.y : (y >= C2.nc.y ? -C2.nc.y : 0);
-        for (int dx = -1; dx <= 1; ++dx) {
-          int x = cx + dx;
-          x += x < 0 ? C2.nc.x : (x >= C2.nc.x ? -C2.nc.x : 0);
-          const int c = (z * C2.nc.y + y) * C2.nc.x + x;
-          const int k1 = __ldg(S2 + c + 1);
-          for (int k = __ldg(S2 + c); k < k1; ++k) {
-            const float4 cj = __ldg(P2 + k);
-            if (__float_as_int(cj.w) != ai) pair_term(p, cj, pi.x, pi.y, pi.z, hist);
+    const uint64_t xi = pk2(pi.x, pi.x), yi = pk2(pi.y, pi.y), zi = pk2(pi.z, pi.z);
+    float x0, x1, y0, y1, z0, z1;
+    warp_range(pi.x, x0, x1);
+    warp_range(pi.y, y0, y1);
+    warp_range(pi.z, z0, z1);
+    // the pencils the cutoff reaches (all of an axis once when it reaches around)
+    int ya = (int)floorf((y0 - G.reach - g.lo.y) * g.inv.y), ny = (int)floorf((y1 + G.reach - g.lo.y) * g.inv.y) - ya + 1;
+    int za = (int)floorf((z0 - G.reach - g.lo.z) * g.inv.z), nz = (int)floorf((z1 + G.reach - g.lo.z) * g.inv.z) - za + 1;
+    const bool all_y = ny >= g.n.y, all_z = nz >= g.n.z;
+    if (all_y) ya = 0, ny = g.n.y;
+    if (all_z) za = 0, nz = g.n.z;
+    int cnt = 0;  // gathered members
+    auto go = [&](int n) {  // lanes against the first n gathered members (a multiple of four)
+      __syncwarp();
+      for (int t = 0; t < n; t += 4)
+        count4<SELF>(p, xi, yi, zi, ai, *reinterpret_cast<const float4*>(bx + t), *reinterpret_cast<const float4*>(by + t),
+                     *reinterpret_cast<const float4*>(bz + t), bx + t, by + t, bz + t, bid + (SELF == PH_SELF_IDS ? t : 0),
+                     hist, whist, 1u);
+      __syncwarp();
+    };
+    auto gather = [&](int k0, int k1) {
+      for (int k = k0; k < k1; k += 32) {
+        const int m = min(32, k1 - k);
+        if (lane < m) {
+          const float4 c = __ldg(P2 + k + lane);
+          bx[cnt + lane] = c.x;
+          by[cnt + lane] = c.y;
+          bz[cnt + lane] = c.z;
+          if (SELF == PH_SELF_IDS) bid[cnt + lane] = __float_as_int(c.w);
+        }
+        cnt += m;
+        if (cnt >= PG_TILE) {
+          go(PG_TILE);
+          cnt -= PG_TILE;
+          float cx = 0.f, cy = 0.f, cz = 0.f;
+          int ci = 0;
+          if (lane < cnt) {
+            cx = bx[PG_TILE + lane], cy = by[PG_TILE + lane], cz = bz[PG_TILE + lane];
+            if (SELF == PH_SELF_IDS) ci = bid[PG_TILE + lane];
+            bx[lane] = cx, by[lane] = cy, bz[lane] = cz;
+            if (SELF == PH_SELF_IDS) bid[lane] = ci;
+          }
+          __syncwarp();
+        }
+      }
+    };
+    for (int t0 = 0; t0 < ny * nz; t0 += 32) {
+      // one pencil per lane: its run of cells, in two parts when it crosses the box's end
+      int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+      if (t0 + lane < ny * nz) {
+        const int jz = za + (t0 + lane) / ny, jy = ya + (t0 + lane) % ny;
+        const float fy = g.lo.y + (float)jy * g.cell.y, fz = g.lo.z + (float)jz * g.cell.z;
+        const float gy = all_y ? 0.f : fmaxf(0.f, fmaxf(fy - y1, y0 - (fy + g.cell.y)));
+        const float gz = all_z ? 0.f : fmaxf(0.f, fmaxf(fz - z1, z0 - (fz + g.cell.z)));
+        const float rem = G.reach * G.reach - gy * gy - gz * gz;
+        if (rem >= 0.f) {
+          const float h = sqrtf(rem);
+          const int32_t* S = S2 + (wrap_index(jz, g.n.z) * g.n.y + wrap_index(jy, g.n.y)) * g.n.x;
+          const int xa = (int)floorf((x0 - h - g.lo.x) * g.inv.x), nx = (int)floorf((x1 + h - g.lo.x) * g.inv.x) - xa + 1;
+          if (nx >= g.n.x) {
+            a0 = S[0], a1 = S[g.n.x];
+          } else {
+            const int w = wrap_index(xa, g.n.x), e = w + nx;
+            a0 = S[w], a1 = S[min(e, g.n.x)];
+            if (e > g.n.x) b0 = S[0], b1 = S[e - g.n.x];
           }
         }
       }
+      for (unsigned m = __ballot_sync(0xffffffffu, a1 > a0 || b1 > b0); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        gather(__shfl_sync(0xffffffffu, a0, src), __shfl_sync(0xffffffffu, a1, src));
+        const int k0 = __shfl_sync(0xffffffffu, b0, src), k1 = __shfl_sync(0xffffffffu, b1, src);
+        if (k1 > k0) gather(k0, k1);
+      }
     }
+    if (cnt & 3) {
+      if (lane < 4 - (cnt & 3)) {
+        bx[cnt + lane] = by[cnt + lane] = bz[cnt + lane] = nan;
+        if (SELF == PH_SELF_IDS) bid[cnt + lane] = -1;
+      }
+      cnt = (cnt + 3) & ~3;
+    }
+    go(cnt);
+    if (G.same && live) {
+      // this atom's own pair was counted when it lies within the last bin
+      const float* B = p.w + (int64_t)p.frame_b[q] * 3 * p.n_pad;
+      const float dx = __fsub_rn(B[ai], pi.x), dy = __fsub_rn(B[p.n_pad + ai], pi.y), dz = __fsub_rn(B[2 * p.n_pad + ai], pi.z);
+      const float mx = min_image(dx, p.box.x), my = min_image(dy, p.box.y), mz = min_image(dz, p.box.z);
+      if (fmaf(mz, mz, fmaf(my, my, mx * mx)) < p.s2_cut) {
+        const int b = exact_bin(dx, dy, dz, p.box, p.bin_size);
+        if (b >= 0 && b < p.n_bins) atomicSub(whist + b, 1u);
+      }
+    }
+    __syncwarp();
   }
   __syncthreads();
-  unsigned long long* dst = p.counts + (int64_t)p.row_of[q] * p.n_bins;
-  for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x) {
-    unsigned long long s = 0;
-    for (int w = 0; w < 8; ++w) s += sh_hist[w * p.n_bins + b];
-    if (s) atomicAdd(dst + b, s);
+  flush_counts(p, sh_hist, p.row_of[q]);
+}
+
+// cells of about edge_x x edge_yz x edge_yz over the box, at most 2^20
+static PHGrid make_grid(amdat_ctx* ctx, double edge_x, double edge_yz, bool snake, float tol) {
+  auto cells = [](double L, double e, int most) { return (int)std::min<double>(most, std::max(1.0, std::floor(L / e))); };
+  PHGrid g;
+  g.n = make_int3(cells(ctx->box[0], edge_x, 1024), cells(ctx->box[1], edge_yz, 1024), cells(ctx->box[2], edge_yz, 1024));
+  while ((int64_t)g.n.x * g.n.y * g.n.z > (1 << 20)) {
+    int& m = g.n.x >= g.n.y && g.n.x >= g.n.z ? g.n.x : (g.n.y >= g.n.z ? g.n.y : g.n.z);
+    m = (m + 1) / 2;
   }
+  g.n_cells = g.n.x * g.n.y * g.n.z;
+  g.lo = make_float3(ctx->box_lo[0], ctx->box_lo[1], ctx->box_lo[2]);
+  g.cell = make_float3(ctx->box[0] / g.n.x, ctx->box[1] / g.n.y, ctx->box[2] / g.n.z);
+  g.inv = make_float3((float)g.n.x / ctx->box[0], (float)g.n.y / ctx->box[1], (float)g.n.z / ctx->box[2]);
+  g.snake = snake ? 1 : 0;
+  g.tol = tol;
+  return g;
 }
 
 static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& l2, bool symmetric,
@@ -412,9 +548,7 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   p.s2_cut = (float)(cut * cut);
   p.n_bins = n_bins;
   p.counts = (unsigned long long*)(base + o_cnt);
-  // cell lists for the ordered pass when the box holds at least three cells per
-  // axis no narrower than the last bin edge (with a 1e-4 margin over the
-  // in-range cut, so a rounding of a cell index never splits an in-range pair)
+  // cell lists for the ordered pass when the box holds at least three cutoffs per axis
   const float cell_edge = (float)((double)max_distance * (1.0 + 1e-4));
   const int3 nc = make_int3((int)std::floor(ctx->box[0] / cell_edge), (int)std::floor(ctx->box[1] / cell_edge),
                             (int)std::floor(ctx->box[2] / cell_edge));
@@ -422,11 +556,9 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   const char* pc = std::getenv("AMDAT_PAIR_CELLS");  // "off": the all-pairs pass
   const bool cells = !symmetric && n_q && l1.n > 0 && l2.n >= 1024 && nc.x >= 3 && nc.y >= 3 && nc.z >= 3 &&
                      n_cells <= (1 << 20) && !(pc && std::strcmp(pc, "off") == 0);
+  bool done = false;
   if (cells) {
-    // frame slots: the distinct frames of each side; one structure when both
-    // sides are the same list
-    const bool same = &l1 == &l2;
-    std::vector<int32_t> fr1, fr2;
+    // frame slots: the distinct frames of each side
     auto slots = [](const std::vector<int32_t>& f, std::vector<int32_t>& uniq, std::vector<int32_t>& slot_of) {
       uniq = f;
       std::sort(uniq.begin(), uniq.end());
@@ -435,77 +567,93 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
       for (size_t i = 0; i < f.size(); ++i)
         slot_of[i] = (int32_t)(std::lower_bound(uniq.begin(), uniq.end(), f[i]) - uniq.begin());
     };
-    std::vector<int32_t> sa, sb;
-    if (same) {
-      std::vector<int32_t> both(fa);
-      both.insert(both.end(), fb.begin(), fb.end());
-      std::vector<int32_t> tmp;
-      slots(both, fr1, tmp);
-      sa.assign(tmp.begin(), tmp.begin() + (std::ptrdiff_t)n_q);
-      sb.assign(tmp.begin() + (std::ptrdiff_t)n_q, tmp.end());
-      fr2 = fr1;
-    } else {
-      slots(fa, fr1, sa);
-      slots(fb, fr2, sb);
-    }
-    const int n_sides = same ? 1 : 2;
+    std::vector<int32_t> fr[2], slot[2];
+    slots(fa, fr[0], slot[0]);
+    slots(fb, fr[1], slot[1]);
+    // list 1: pencils as wide as the cube of 32 atoms, x cells a quarter of that; list 2:
+    // pencils of a third of the cutoff (the runs then follow its sphere), but wide enough
+    // for runs of about 16 atoms, x cells of half a pencil or two atoms
+    const double vol = (double)ctx->box[0] * ctx->box[1] * ctx->box[2];
+    const double edge = (double)std::max(ctx->box[0], std::max(ctx->box[1], ctx->box[2]));
+    const double w1 = std::cbrt(32.0 * vol / l1.n), rho2 = l2.n / vol;
+    const double f2 = std::max((double)max_distance / 3.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
+    const float tol = (float)std::max(2e-5 * max_distance, 4e-7 * edge);
+    const PHGrid grid[2] = {make_grid(ctx, 0.25 * w1, w1, true, tol),
+                            make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol)};
     const ListEntry* lists[2] = {&l1, &l2};
-    const std::vector<int32_t>* frs[2] = {&fr1, &fr2};
     size_t need = 0;
     size_t off[2][6];
-    for (int s = 0; s < n_sides; ++s) {
-      const size_t nf = frs[s]->size(), n = (size_t)lists[s]->n;
-      off[s][0] = need; need = align(need + nf * 4);                           // frames
-      off[s][1] = need; need = align(need + nf * n * 4);                       // cell_of
-      off[s][2] = need; need = align(need + nf * (size_t)n_cells * 4);         // count
-      off[s][3] = need; need = align(need + nf * (size_t)(n_cells + 1) * 4);   // start
-      off[s][4] = need; need = align(need + nf * (size_t)n_cells * 4);         // cursor
-      off[s][5] = need; need = align(need + nf * n * sizeof(float4));          // pos
+    for (int s = 0; s < 2; ++s) {
+      const size_t nf = fr[s].size(), n = (size_t)lists[s]->n, nc1 = (size_t)grid[s].n_cells;
+      off[s][0] = need; need = align(need + nf * 4);               // frames
+      off[s][1] = need; need = align(need + nf * n * 4);           // cell_of
+      off[s][2] = need; need = align(need + nf * nc1 * 4);         // count
+      off[s][3] = need; need = align(need + nf * (nc1 + 1) * 4);   // start
+      off[s][4] = need; need = align(need + nf * nc1 * 4);         // cursor
+      off[s][5] = need; need = align(need + nf * n * sizeof(float4));  // pos
     }
-    const size_t o_sa = need; need = align(need + n_q * 4);
-    const size_t o_sb = need; need = align(need + n_q * 4);
-    unsigned char* cb = ctx->scratch2.reserve(need);
+    const size_t o_slot[2] = {need, align(need + n_q * 4)};
+    const size_t o_flag = align(o_slot[1] + n_q * 4);
+    unsigned char* cb = ctx->scratch2.reserve(o_flag + 4);
     cudaStream_t st = ctx->stream;
-    AMDAT_CUDA(cudaMemcpyAsync(cb + o_sa, sa.data(), n_q * 4, cudaMemcpyHostToDevice, st));
-    AMDAT_CUDA(cudaMemcpyAsync(cb + o_sb, sb.data(), n_q * 4, cudaMemcpyHostToDevice, st));
-    PHCells C[2];
-    for (int s = 0; s < n_sides; ++s) {
-      const int nf = (int)frs[s]->size();
+    AMDAT_CUDA(cudaMemsetAsync(cb + o_flag, 0, 4, st));
+    for (int s = 0; s < 2; ++s) {
+      const int nf = (int)fr[s].size();
       const PHList l = phview(*lists[s]);
-      PHCells& c = C[s];
-      c.nc = nc;
-      c.lo = make_float3(ctx->box_lo[0], ctx->box_lo[1], ctx->box_lo[2]);
-      c.inv_cell = make_float3((float)nc.x / ctx->box[0], (float)nc.y / ctx->box[1], (float)nc.z / ctx->box[2]);
-      c.n_cells = (int32_t)n_cells;
-      c.start = (const int32_t*)(cb + off[s][3]);
-      c.pos = (const float4*)(cb + off[s][5]);
-      c.n = l.n;
-      AMDAT_CUDA(cudaMemcpyAsync(cb + off[s][0], frs[s]->data(), (size_t)nf * 4, cudaMemcpyHostToDevice, st));
-      AMDAT_CUDA(cudaMemsetAsync(cb + off[s][2], 0, (size_t)nf * n_cells * 4, st));
+      const PHGrid& gs = grid[s];
       AMDAT_REQUIRE(nf <= 65535, "at most 65535 frames per call");
-      const dim3 g((unsigned)ceil_div(l.n, 256), (unsigned)nf);
-      ph_cell_count_kernel<<<g, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), nc, c.lo,
-                                              c.inv_cell, (int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][2]));
-      ph_cell_scan_kernel<<<(unsigned)nf, 1024, 0, st>>>((const int32_t*)(cb + off[s][2]), (int32_t)n_cells,
+      AMDAT_CUDA(cudaMemcpyAsync(cb + o_slot[s], slot[s].data(), n_q * 4, cudaMemcpyHostToDevice, st));
+      AMDAT_CUDA(cudaMemcpyAsync(cb + off[s][0], fr[s].data(), (size_t)nf * 4, cudaMemcpyHostToDevice, st));
+      AMDAT_CUDA(cudaMemsetAsync(cb + off[s][2], 0, (size_t)nf * gs.n_cells * 4, st));
+      const dim3 gn((unsigned)ceil_div(l.n, 256), (unsigned)nf);
+      ph_cell_count_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), gs,
+                                               (int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][2]), (int32_t*)(cb + o_flag));
+      ph_cell_scan_kernel<<<(unsigned)nf, 1024, 0, st>>>((const int32_t*)(cb + off[s][2]), gs.n_cells,
                                                           (int32_t*)(cb + off[s][3]), (int32_t*)(cb + off[s][4]));
-      ph_cell_scatter_kernel<<<g, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), (int32_t)n_cells,
-                                                (const int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][4]),
-                                                (float4*)(cb + off[s][5]));
+      ph_cell_scatter_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), gs.n_cells,
+                                                 (const int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][4]),
+                                                 (float4*)(cb + off[s][5]));
       check_launch("pair cell lists");
       count_launch(ctx, 3);
     }
-    if (same) C[1] = C[0];
-    const size_t shm = (size_t)8 * n_bins * 4;
-    if (shm > 48 * 1024)
-      AMDAT_CUDA(cudaFuncSetAttribute(pair_hist_cells_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
     AMDAT_REQUIRE(n_q <= 65535, "at most 65535 frames or time pairs per call");
-    dim3 grid((unsigned)ceil_div(l1.n, PH_THREADS), (unsigned)n_q);
-    KernelTimer kt(ctx, "pair_hist_cells_kernel");
-    pair_hist_cells_kernel<<<grid, PH_THREADS, shm, st>>>(p, C[0], C[1], (const int32_t*)(cb + o_sa),
-                                                          (const int32_t*)(cb + o_sb));
-    check_launch("pair_hist_cells_kernel");
-    count_launch(ctx);
-  } else if (n_q && l1.n > 0 && l2.n > 0) {
+    PHGroups G;
+    G.pos1 = (const float4*)(cb + off[0][5]);
+    G.n1 = l1.n;
+    G.pos2 = (const float4*)(cb + off[1][5]);
+    G.start2 = (const int32_t*)(cb + off[1][3]);
+    G.n2 = l2.n;
+    G.g2 = grid[1];
+    G.slot_a = (const int32_t*)(cb + o_slot[0]);
+    G.slot_b = (const int32_t*)(cb + o_slot[1]);
+    G.reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
+    G.same = &l1 == &l2 ? 1 : 0;
+    G.outside = (const int32_t*)(cb + o_flag);
+    // up to eight groups per warp (one flush of the histograms for them) while the blocks
+    // fill the chip twice over
+    const int64_t groups = ceil_div(l1.n, 32);
+    G.per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups * (int64_t)n_q / ((int64_t)ctx->n_sm * 8 * PH_WARPS)));
+    const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
+    auto launch = [&](auto kern) {
+      if (shm > 24 * 1024)
+        AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+      KernelTimer kt(ctx, "pair_hist_cells_kernel");
+      kern<<<dim3((unsigned)ceil_div(groups, (int64_t)PH_WARPS * G.per_warp), (unsigned)n_q), PH_THREADS, shm, st>>>(p, G);
+      check_launch("pair_hist_groups_kernel");
+      count_launch(ctx);
+    };
+    // lists that may share atoms tell an atom's own pair by its index
+    const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
+    if (G.same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>);
+    else launch(pair_hist_groups_kernel<PH_SELF_IDS>);
+    // atoms outside the box (wrapped coordinates given so): the all-pairs pass instead
+    int32_t outside = 0;
+    AMDAT_CUDA(cudaMemcpyAsync(&outside, cb + o_flag, 4, cudaMemcpyDeviceToHost, st));
+    AMDAT_CUDA(cudaStreamSynchronize(st));
+    done = outside == 0;
+    if (!done) AMDAT_CUDA(cudaMemsetAsync(base + o_cnt, 0, n_out * 8, st));
+  }
+  if (!done && n_q && l1.n > 0 && l2.n > 0) {
     AMDAT_REQUIRE(n_q <= 65535, "at most 65535 frames or time pairs per call");
     // units of 256 I members by up to seg list-2 members: wide ones while they fill
     // the chip six times over, then fewer members per thread and shorter segments
@@ -538,8 +686,8 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
       check_launch("pair_hist_kernel");
       count_launch(ctx);
     };
-    if (ids) I == 4 ? launch(pair_hist_kernel<4, true>) : I == 2 ? launch(pair_hist_kernel<2, true>) : launch(pair_hist_kernel<1, true>);
-    else I == 4 ? launch(pair_hist_kernel<4, false>) : I == 2 ? launch(pair_hist_kernel<2, false>) : launch(pair_hist_kernel<1, false>);
+    if (ids) I == 4 ? launch(pair_hist_kernel<4, PH_SELF_IDS>) : I == 2 ? launch(pair_hist_kernel<2, PH_SELF_IDS>) : launch(pair_hist_kernel<1, PH_SELF_IDS>);
+    else I == 4 ? launch(pair_hist_kernel<4, PH_SELF_ZERO>) : I == 2 ? launch(pair_hist_kernel<2, PH_SELF_ZERO>) : launch(pair_hist_kernel<1, PH_SELF_ZERO>);
   }
   AMDAT_CUDA(cudaMemcpyAsync(counts, base + o_cnt, n_out * 8,
                              out_flags == AMDAT_OUT_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,

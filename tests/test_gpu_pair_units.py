@@ -83,3 +83,41 @@ def test_vhd_all_pairs_units(eng, monkeypatch, n, max_d):
     for k in range(len(g)):
         ref[g[k]] += _counts(u[t0[k]], u[t1[k]], ids, ids, np.float32(box), max_d, 50)
     np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("n,box,max_d,nb,sigma", [(1100, 12.0, 3.9, 60, 0.3), (5000, 18.0, 1.2, 33, 0.5),
+                                                  (6001, 40.0, 13.0, 200, 2.0), (3000, 15.0, 4.99, 500, 0.0)])
+def test_vhd_cells(eng, monkeypatch, n, box, max_d, nb, sigma):
+    """The cell pass against the all-pairs pass: dense and sparse boxes, reaches just
+    below a third of the box and far below it, atoms that do not move (every own pair
+    at zero distance)."""
+    sc = synth.TimeScheme.linear(4, 1.0)
+    traj = synth.random_walk(n, box, sc, sigma, seed=n, time_scaled=False)
+    eng.upload(traj.unwrapped, traj.box)
+    eng.set_scheme(sc)
+    third, rest = eng.list(np.arange(0, n, 3)), eng.list(np.arange(0, n))
+    half, other = eng.list(np.arange(0, n // 2)), eng.list(np.arange(n // 2, n))
+    for l1, l2 in ((0, 0), (third, rest), (third, 0), (half, 0), (0, other), (third, third), (eng.list([5]), rest)):
+        monkeypatch.delenv("AMDAT_PAIR_CELLS", raising=False)
+        got = eng.vhd(l1, l2, max_d, nb)
+        monkeypatch.setenv("AMDAT_PAIR_CELLS", "off")
+        np.testing.assert_array_equal(got, eng.vhd(l1, l2, max_d, nb))
+
+
+def test_vhd_cells_slab_and_outside(eng, monkeypatch):
+    """A box of unequal edges and an offset origin, a list gathered in one corner; wrapped
+    coordinates that lie outside the box take the all-pairs pass."""
+    rng = np.random.default_rng(8)
+    L, lo, n = np.array([30.0, 9.5, 14.0], np.float32), np.array([-7.0, 2.0, 100.0], np.float32), 4000
+    u = (lo + rng.random((3, n, 3)) * L).astype(np.float32)
+    sc = synth.TimeScheme.linear(3, 1.0)
+    for wrapped in (None, (u + (rng.random((1, n, 1)) < 0.01) * 2.5 * L).astype(np.float32)):
+        eng.upload(u, L, lo, wrapped=wrapped)
+        eng.set_scheme(sc)
+        corner = eng.list(np.nonzero((u[0] - lo < 0.3 * L).all(1))[0])
+        for l1, l2 in ((0, 0), (corner, 0)):
+            monkeypatch.delenv("AMDAT_PAIR_CELLS", raising=False)
+            got = eng.vhd(l1, l2, 3.0, 40)
+            monkeypatch.setenv("AMDAT_PAIR_CELLS", "off")
+            np.testing.assert_array_equal(got, eng.vhd(l1, l2, 3.0, 40))
+            assert got.sum() > 0
