@@ -242,12 +242,13 @@ __global__ void __launch_bounds__(PH_THREADS)
 // consecutive atoms then fill a compact box.  A warp takes such a group.
 // List 2 is ordered in narrower pencils of x cells.  Of every pencil whose distance to
 // the group's bounding box is within the cutoff, the warp gathers the run of x cells
-// the cutoff reaches into shared memory, and each lane goes through the gathered
-// atoms (count4).  A pair within the last bin's edge is visited exactly once, so the
-// counts equal the all-pairs pass's.
-// Bound: instruction issue, as the all-pairs pass; a visited pair in five or so is
-// within the cutoff.  (One atom per thread walking its own 27 cells of the cutoff's
-// width visits twice as many pairs through scattered 16-byte loads.)
+// the cutoff reaches, keeps the atoms within the cutoff of the box in shared memory, and
+// each lane goes through them (count4).  A pair within the last bin's edge is visited
+// exactly once, so the counts equal the all-pairs pass's.
+// Bound: instruction issue, as the all-pairs pass; a visited pair in three or so is
+// within the cutoff.  G_d of 64,000 atoms over 1226 time pairs to 5.0 in a box of 42.3:
+// 93.7 ms; 118 ms with every atom of the runs visited; 331 ms with one atom per thread
+// walking its own 27 cells of the cutoff's width.
 // ---------------------------------------------------------------------------
 struct PHGrid {
   int3 n;
@@ -398,6 +399,8 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
     const bool all_y = ny >= g.n.y, all_z = nz >= g.n.z;
     if (all_y) ya = 0, ny = g.n.y;
     if (all_z) za = 0, nz = g.n.z;
+    const float xm = 0.5f * (x0 + x1), ym = 0.5f * (y0 + y1), zm = 0.5f * (z0 + z1);  // the box's centre and half edges
+    const float xh = 0.5f * (x1 - x0), yh = 0.5f * (y1 - y0), zh = 0.5f * (z1 - z0);
     int cnt = 0;  // gathered members
     auto go = [&](int n) {  // lanes against the first n gathered members (a multiple of four)
       __syncwarp();
@@ -409,15 +412,20 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
     };
     auto gather = [&](int k0, int k1) {
       for (int k = k0; k < k1; k += 32) {
-        const int m = min(32, k1 - k);
-        if (lane < m) {
-          const float4 c = __ldg(P2 + k + lane);
-          bx[cnt + lane] = c.x;
-          by[cnt + lane] = c.y;
-          bz[cnt + lane] = c.z;
-          if (SELF == PH_SELF_IDS) bid[cnt + lane] = __float_as_int(c.w);
+        // only members within reach of the group's box are kept
+        const float4 c = k + lane < k1 ? __ldg(P2 + k + lane) : make_float4(nan, nan, nan, 0.f);
+        const float gx = fmaxf(0.f, fabsf(min_image(c.x - xm, p.box.x)) - xh), gy = fmaxf(0.f, fabsf(min_image(c.y - ym, p.box.y)) - yh),
+                    gz = fmaxf(0.f, fabsf(min_image(c.z - zm, p.box.z)) - zh);
+        const bool keep = k + lane < k1 && fmaf(gz, gz, fmaf(gy, gy, gx * gx)) <= G.reach * G.reach;
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int at = cnt + __popc(kept & ((1u << lane) - 1u));
+          bx[at] = c.x;
+          by[at] = c.y;
+          bz[at] = c.z;
+          if (SELF == PH_SELF_IDS) bid[at] = __float_as_int(c.w);
         }
-        cnt += m;
+        cnt += __popc(kept);
         if (cnt >= PG_TILE) {
           go(PG_TILE);
           cnt -= PG_TILE;
@@ -570,15 +578,16 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     std::vector<int32_t> fr[2], slot[2];
     slots(fa, fr[0], slot[0]);
     slots(fb, fr[1], slot[1]);
-    // list 1: pencils as wide as the cube of 32 atoms, x cells a quarter of that; list 2:
-    // pencils of a third of the cutoff (the runs then follow its sphere), but wide enough
-    // for runs of about 16 atoms, x cells of half a pencil or two atoms
+    // list 1: pencils as wide as the cube of 32 atoms, x cells an eighth of that (a quarter
+    // leaves the groups longer: 2 % slower); list 2: pencils of half the cutoff (a third:
+    // 5 % slower, more runs; the whole: 2 %), but wide enough for runs of about 16 atoms,
+    // x cells of half a pencil or two atoms
     const double vol = (double)ctx->box[0] * ctx->box[1] * ctx->box[2];
     const double edge = (double)std::max(ctx->box[0], std::max(ctx->box[1], ctx->box[2]));
     const double w1 = std::cbrt(32.0 * vol / l1.n), rho2 = l2.n / vol;
-    const double f2 = std::max((double)max_distance / 3.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
+    const double f2 = std::max((double)max_distance / 2.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
     const float tol = (float)std::max(2e-5 * max_distance, 4e-7 * edge);
-    const PHGrid grid[2] = {make_grid(ctx, 0.25 * w1, w1, true, tol),
+    const PHGrid grid[2] = {make_grid(ctx, 0.125 * w1, w1, true, tol),
                             make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol)};
     const ListEntry* lists[2] = {&l1, &l2};
     size_t need = 0;
