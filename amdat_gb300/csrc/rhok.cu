@@ -15,8 +15,9 @@
 //
 // Kernels:
 //   rhok_list_kernel     any vector list (e.g. the reference's q-vector
-//                        shells): a block owns 1024 vectors of one frame and
-//                        streams the frame's atoms through shared memory.
+//                        shells): a block owns up to 1024 vectors of one frame
+//                        and streams a segment of the frame's atoms through
+//                        shared memory.
 //   rhok_lattice_kernel  every half-space lattice vector with |n| <= R,
 //                        factorised as rho[(nx,ny), nz] = sum_j W_j(nx,ny) Z_j(nz)
 //                        with W = X(nx) Y(ny): a complex outer-product
@@ -35,6 +36,7 @@
 #include <numeric>
 
 #include "engine.h"
+#include "f32x2.cuh"
 #include "tc_tiles.h"
 
 namespace amdat {
@@ -96,60 +98,95 @@ constexpr int RL_THREADS = 256;
 constexpr int RL_KPT = 4;                       // vectors per thread
 constexpr int RL_TILE = RL_THREADS * RL_KPT;    // vectors per block
 constexpr int RL_ATOMS = 512;                   // atoms staged per step
+constexpr int RL_FOLD = 128;                    // atoms per plain sum; segments hold whole folds
 
+// KPT vectors per thread over the atoms of segment blockIdx.z (seg atoms, whole
+// folds).  FOLDS: the plain sum of every 128 atoms is written to part [fold][frame][k]
+// and rhok_list_merge_kernel adds them up in order; else one segment holds every atom
+// and the block adds them itself.  Both give the same compensated sum bit for bit.
+// Bound: instruction issue, 38 per term and warp, 30 of them in sincospif.
+template <int KPT, bool FOLDS>
 __global__ void __launch_bounds__(RL_THREADS)
-    rhok_list_kernel(const int4* __restrict__ fx, int32_t n_list, const int4* __restrict__ kv,
-                     int32_t n_k, float2* __restrict__ rho) {
+    rhok_list_kernel(const int4* __restrict__ fx, int32_t n_list, const int4* __restrict__ kv, int32_t n_k,
+                     int32_t seg, float2* __restrict__ rho, float2* __restrict__ part) {
   __shared__ int4 s_at[RL_ATOMS];
-  const int f = blockIdx.y;
-  const int k0 = blockIdx.x * RL_TILE;
-  int4 n[RL_KPT];
-  KC acc[RL_KPT];
-  float pr[RL_KPT], pi[RL_KPT];
+  const int f = blockIdx.y, threads = blockDim.x;
+  const int k0 = blockIdx.x * threads * KPT;
+  int4 n[KPT];
+  KC acc[KPT];
+  uint64_t pp[KPT];  // plain sums (cos, sin), packed
 #pragma unroll
-  for (int j = 0; j < RL_KPT; ++j) {
-    const int k = k0 + j * RL_THREADS + threadIdx.x;
+  for (int j = 0; j < KPT; ++j) {
+    const int k = k0 + j * threads + threadIdx.x;
     n[j] = k < n_k ? kv[k] : make_int4(0, 0, 0, 0);
     acc[j] = KC{0.f, 0.f, 0.f, 0.f};
-    pr[j] = pi[j] = 0.f;
+    pp[j] = 0ull;
   }
   const int4* F = fx + (int64_t)f * n_list;
-  int since_fold = 0;
-  for (int a0 = 0; a0 < n_list; a0 += RL_ATOMS) {
-    const int na = min(RL_ATOMS, n_list - a0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < na; i += RL_THREADS) s_at[i] = F[a0 + i];
-    __syncthreads();
-    for (int a = 0; a < na; ++a) {
-      const int4 q = s_at[a];
+  const int first = blockIdx.z * seg, last = min(n_list, first + seg);
+  auto fold = [&](int at) {  // the plain sums of the fold that starts at atom `at`
 #pragma unroll
-      for (int j = 0; j < RL_KPT; ++j) {
-        const int32_t ph = (int32_t)((uint32_t)n[j].x * (uint32_t)q.x +
-                                     (uint32_t)n[j].y * (uint32_t)q.y +
-                                     (uint32_t)n[j].z * (uint32_t)q.z);
-        float s, c;
-        phase_sincos(ph, &s, &c);
-        pr[j] += c;
-        pi[j] += s;
+    for (int j = 0; j < KPT; ++j) {
+      float pr, pi;
+      upk2(pp[j], pr, pi);
+      if (FOLDS) {
+        const int k = k0 + j * threads + threadIdx.x;
+        if (k < n_k) part[((int64_t)(at / RL_FOLD) * gridDim.y + f) * n_k + k] = make_float2(pr, pi);
+      } else {
+        kc_add(acc[j], pr, pi);
       }
-      if (++since_fold == 128) {
+      pp[j] = 0ull;
+    }
+  };
+  for (int a0 = first; a0 < last; a0 += RL_ATOMS) {
+    const int na = min(RL_ATOMS, last - a0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < na; i += threads) s_at[i] = F[a0 + i];
+    __syncthreads();
+    for (int b0 = 0; b0 < na; b0 += RL_FOLD) {
+      const int b1 = min(na, b0 + RL_FOLD);
+#pragma unroll 2
+      for (int a = b0; a < b1; ++a) {
+        const int4 q = s_at[a];
 #pragma unroll
-        for (int j = 0; j < RL_KPT; ++j) {
-          kc_add(acc[j], pr[j], pi[j]);
-          pr[j] = pi[j] = 0.f;
+        for (int j = 0; j < KPT; ++j) {
+          const int32_t ph = (int32_t)((uint32_t)n[j].x * (uint32_t)q.x +
+                                       (uint32_t)n[j].y * (uint32_t)q.y +
+                                       (uint32_t)n[j].z * (uint32_t)q.z);
+          float s, c;
+          phase_sincos(ph, &s, &c);
+          pp[j] = add2(pp[j], pk2(c, s));
         }
-        since_fold = 0;
       }
+      if (FOLDS || b1 - b0 == RL_FOLD) fold(a0 + b0);
     }
   }
+  if (!FOLDS) {
+    fold(0);  // the atoms beyond the last whole fold
 #pragma unroll
-  for (int j = 0; j < RL_KPT; ++j) {
-    kc_add(acc[j], pr[j], pi[j]);
-    const int k = k0 + j * RL_THREADS + threadIdx.x;
-    if (k < n_k)
-      rho[(int64_t)f * n_k + k] = make_float2(__fsub_rn(acc[j].sr, acc[j].cr),
-                                              __fsub_rn(acc[j].si, acc[j].ci));
+    for (int j = 0; j < KPT; ++j) {
+      const int k = k0 + j * threads + threadIdx.x;
+      if (k < n_k)
+        rho[(int64_t)f * n_k + k] = make_float2(__fsub_rn(acc[j].sr, acc[j].cr), __fsub_rn(acc[j].si, acc[j].ci));
+    }
   }
+}
+
+// the folds' plain sums into the compensated sum, in order (the closing addition is the
+// partial fold's, or zero)
+__global__ void rhok_list_merge_kernel(const float2* __restrict__ part, int32_t n_whole, int32_t partial, int64_t n,
+                                       float2* __restrict__ rho) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  KC acc = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+  for (int b = 0; b < n_whole; ++b) {
+    const float2 v = __ldcs(part + b * n + i);
+    kc_add(acc, v.x, v.y);
+  }
+  const float2 v = partial ? part[n_whole * n + i] : make_float2(0.f, 0.f);
+  kc_add(acc, v.x, v.y);
+  rho[i] = make_float2(__fsub_rn(acc.sr, acc.cr), __fsub_rn(acc.si, acc.ci));
 }
 
 // ---------------------------------------------------------------------------
@@ -361,11 +398,43 @@ static void run_list_density(amdat_ctx* ctx, Density& d, float period, int32_t p
     count_launch(ctx);
   } else {
     int4* fx = fixed_turns(ctx, d, e, period, d_frames);
-    dim3 grid((unsigned)ceil_div(d.n_k, RL_TILE), (unsigned)d.n_frames);
-    KernelTimer kt(ctx, "rhok_list_kernel");
-    rhok_list_kernel<<<grid, RL_THREADS, 0, ctx->stream>>>(fx, e.n, kv.ptr, d.n_k, d.rho->ptr);
-    check_launch("rhok_list_kernel");
-    count_launch(ctx);
+    // as many vectors per thread as fill a block (four share each staged atom); atom
+    // segments until about 24 blocks per SM even out what the SMs get.  5,085 vectors x
+    // 100 frames are 500 blocks, four on some SMs and three on the others: 20.7 ms for
+    // 32,000 atoms, 17.5 ms in segments, 16.2 ms with two atoms in flight per vector.  Short lists gain more: of 85 vectors one warp in
+    // eight was busy
+    const int kpt = d.n_k > 2 * RL_THREADS ? 4 : (d.n_k > RL_THREADS ? 2 : 1);
+    const int threads = d.n_k > 128 ? RL_THREADS : (d.n_k > 64 ? 128 : 64);
+    const int64_t kb = ceil_div(d.n_k, (int64_t)threads * kpt);
+    const int64_t folds = ceil_div(e.n, RL_FOLD);
+    const int64_t want = (int64_t)24 * ctx->n_sm * (RL_THREADS / threads);
+    // frame batches keep the folds' sums within 96 MB (they stay in L2 on their way)
+    const size_t fold_bytes = (size_t)folds * d.n_k * sizeof(float2);
+    const bool split = folds > 1 && kb * d.n_frames < want;
+    const int32_t batch = split ? (int32_t)std::max<size_t>(1, std::min<size_t>(d.n_frames, (size_t)(96u << 20) / fold_bytes)) : d.n_frames;
+    const int64_t segs = split ? std::min(folds, ceil_div(want, kb * batch)) : 1;
+    const int seg = (int)(ceil_div(folds, segs) * RL_FOLD);
+    float2* part = split ? (float2*)ctx->scratch.reserve(fold_bytes * batch) : nullptr;
+    for (int32_t f0 = 0; f0 < d.n_frames; f0 += batch) {
+      const int32_t nb = std::min(batch, d.n_frames - f0);
+      float2* rho = d.rho->ptr + (int64_t)f0 * d.n_k;
+      const dim3 grid((unsigned)kb, (unsigned)nb, (unsigned)ceil_div(e.n, seg));
+      auto launch = [&](auto kern) {
+        KernelTimer kt(ctx, "rhok_list_kernel");
+        kern<<<grid, threads, 0, ctx->stream>>>(fx + (int64_t)f0 * e.n, e.n, kv.ptr, d.n_k, seg, rho, part);
+        check_launch("rhok_list_kernel");
+        count_launch(ctx);
+      };
+      if (split) kpt == 4 ? launch(rhok_list_kernel<4, true>) : kpt == 2 ? launch(rhok_list_kernel<2, true>) : launch(rhok_list_kernel<1, true>);
+      else kpt == 4 ? launch(rhok_list_kernel<4, false>) : kpt == 2 ? launch(rhok_list_kernel<2, false>) : launch(rhok_list_kernel<1, false>);
+      if (split) {
+        const int64_t n_out = (int64_t)nb * d.n_k;
+        rhok_list_merge_kernel<<<(unsigned)ceil_div(n_out, 256), 256, 0, ctx->stream>>>(
+            part, e.n / RL_FOLD, e.n % RL_FOLD ? 1 : 0, n_out, rho);
+        check_launch("rhok_list_merge_kernel");
+        count_launch(ctx);
+      }
+    }
   }
   AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
 }
