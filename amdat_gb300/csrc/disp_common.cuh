@@ -75,14 +75,21 @@ __device__ __forceinline__ KSum list_shell_sum(const int4* R, int32_t fx, int32_
   // n . (2 f) mod 2^32 is the doubled phase cos_fixed_sfu forms from n . f
   const uint32_t gx = (uint32_t)fx << 1, gy = (uint32_t)fy << 1, gz = (uint32_t)fz << 1;
   KSum acc = {0.f, 0.f};
-  for (int v0 = v_begin; v0 < v_end; v0 += 32) {
-    const int v1 = min(v0 + 32, v_end);
+  auto term = [&](int v) {
+    const int4 n = SMEM ? R[v] : __ldg(R + v);
+    return cos_turn32_sfu((int32_t)((uint32_t)n.x * gx + (uint32_t)n.y * gy + (uint32_t)n.z * gz));
+  };
+  int v0 = v_begin;
+  for (; v0 + 32 <= v_end; v0 += 32) {
+    float blk = 0.f;
+#pragma unroll
+    for (int v = 0; v < 32; ++v) blk += term(v0 + v);
+    kadd(acc, blk);
+  }
+  if (v0 < v_end) {
     float blk = 0.f;
 #pragma unroll 4
-    for (int v = v0; v < v1; ++v) {
-      const int4 n = SMEM ? R[v] : __ldg(R + v);
-      blk += cos_turn32_sfu((int32_t)((uint32_t)n.x * gx + (uint32_t)n.y * gy + (uint32_t)n.z * gz));
-    }
+    for (int v = v0; v < v_end; ++v) blk += term(v);
     kadd(acc, blk);
   }
   if ((v_end - v_begin) % 32 == 0) kadd(acc, 0.f);  // the closing (empty) block
@@ -101,22 +108,34 @@ __device__ __forceinline__ void list_shell_sum2(const int4* R, int32_t fxa, int3
   const uint64_t scale = pk2(1.4629180792671596e-09f, 1.4629180792671596e-09f);  // 2 pi / 2^32
   acc_a = KSum{0.f, 0.f};
   acc_b = KSum{0.f, 0.f};
-  for (int v0 = v_begin; v0 < v_end; v0 += 32) {
-    const int v1 = min(v0 + 32, v_end);
-    uint64_t blk = 0ull;  // (0.f, 0.f)
-#pragma unroll 4
-    for (int v = v0; v < v1; ++v) {
-      const int4 n = SMEM ? R[v] : __ldg(R + v);
-      const int32_t pa = (int32_t)((uint32_t)n.x * ax + (uint32_t)n.y * ay + (uint32_t)n.z * az);
-      const int32_t pb = (int32_t)((uint32_t)n.x * bx + (uint32_t)n.y * by + (uint32_t)n.z * bz);
-      float xa, xb;
-      upk2(mul2(pk2((float)pa, (float)pb), scale), xa, xb);
-      blk = add2(blk, pk2(__cosf(xa), __cosf(xb)));
-    }
+  auto term = [&](int v, uint64_t& blk) {
+    const int4 n = SMEM ? R[v] : __ldg(R + v);
+    const int32_t pa = (int32_t)((uint32_t)n.x * ax + (uint32_t)n.y * ay + (uint32_t)n.z * az);
+    const int32_t pb = (int32_t)((uint32_t)n.x * bx + (uint32_t)n.y * by + (uint32_t)n.z * bz);
+    float xa, xb;
+    upk2(mul2(pk2((float)pa, (float)pb), scale), xa, xb);
+    blk = add2(blk, pk2(__cosf(xa), __cosf(xb)));
+  };
+  auto close = [&](uint64_t blk) {
     float ba, bb;
     upk2(blk, ba, bb);
     kadd(acc_a, ba);
     kadd(acc_b, bb);
+  };
+  // whole blocks as straight code: 7.8 instructions and 2.8 cycles per cosine and warp,
+  // against 9.7 and 3.2 with a loop of run-time length (the SFU alone allows 2)
+  int v0 = v_begin;
+  for (; v0 + 32 <= v_end; v0 += 32) {
+    uint64_t blk = 0ull;  // (0.f, 0.f)
+#pragma unroll
+    for (int v = 0; v < 32; ++v) term(v0 + v, blk);
+    close(blk);
+  }
+  if (v0 < v_end) {
+    uint64_t blk = 0ull;
+#pragma unroll 4
+    for (int v = v0; v < v_end; ++v) term(v, blk);
+    close(blk);
   }
   if ((v_end - v_begin) % 32 == 0) {  // the closing (empty) block
     kadd(acc_a, 0.f);
