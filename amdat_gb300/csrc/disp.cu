@@ -125,6 +125,48 @@ __device__ __forceinline__ KSum octant_shell_sum(const int4* R, const float* T, 
   return acc;
 }
 
+// octant mode for two atoms at once (tables interleaved [axis][n][thread]{a, b},
+// representatives packed in 8 bytes: x | y << 16, z | weight as BF16 << 16): the sums
+// of octant_shell_sum for each, bit for bit
+__device__ __forceinline__ void octant_shell_sum2(const uint2* R, const uint64_t* T, int v_begin, int v_end, KSum& acc_a,
+                                                  KSum& acc_b) {
+  acc_a = KSum{0.f, 0.f};
+  acc_b = KSum{0.f, 0.f};
+  auto term = [&](int v, uint64_t& blk) {
+    const uint2 r = R[v];
+    const float w = __uint_as_float(r.y & 0xffff0000u);
+    blk = fma2(mul2(mul2(pk2(w, w), T[r.x & 0xffffu]), T[r.x >> 16]), T[r.y & 0xffffu], blk);
+  };
+  auto close = [&](uint64_t blk) {
+    float ba, bb;
+    upk2(blk, ba, bb);
+    kadd(acc_a, ba);
+    kadd(acc_b, bb);
+  };
+  int v0 = v_begin;
+  for (; v0 + 32 <= v_end; v0 += 32) {
+    uint64_t blk = 0ull;  // (0.f, 0.f)
+#pragma unroll
+    for (int v = 0; v < 32; ++v) term(v0 + v, blk);
+    close(blk);
+  }
+  if (v0 < v_end) {
+    uint64_t blk = 0ull;
+#pragma unroll 4
+    for (int v = v0; v < v_end; ++v) term(v, blk);
+    close(blk);
+  }
+  if ((v_end - v_begin) % 32 == 0) {  // the closing (empty) block
+    kadd(acc_a, 0.f);
+    kadd(acc_b, 0.f);
+  }
+}
+
+// MODE: 0 moments, 1 F_s by vector list, 2 F_s by octants, 3 by octants with two atoms
+// per thread.  Octants are bound by the loads of a representative and its three cosines
+// from shared memory; with two atoms per thread one 8-byte representative and three
+// 8-byte pairs serve both, and the products run packed (4,000 atoms x 1,100 pairs of 281
+// representatives: 280 -> 221 us).
 template <int MODE, bool GS>
 __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
     disp_mixed_kernel(DispParams p) {
@@ -139,8 +181,15 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
   // F_s: the pass's vectors (list mode) or representatives (octant mode, after
   // the tables) in shared memory, when they fit
   int4* reps = reinterpret_cast<int4*>(tab + (MODE == 2 ? 3 * (p.nmax + 1) * nthr : 0));
-  if (MODE != 0 && p.n_rep_smem)
+  if ((MODE == 1 || MODE == 2) && p.n_rep_smem)
     for (int i = tid; i < p.n_rep_smem; i += nthr) reps[i] = __ldg(p.kv + p.kv_off[0] + i);
+  uint64_t* tab2 = reinterpret_cast<uint64_t*>(tab);  // MODE 3: tables of two atoms, then the packed representatives
+  uint2* reps2 = reinterpret_cast<uint2*>(tab2 + (MODE == 3 ? 3 * (p.nmax + 1) * nthr : 0));
+  if (MODE == 3)
+    for (int i = tid; i < p.n_rep_smem; i += nthr) {
+      const int4 r = __ldg(p.kv + p.kv_off[0] + i);
+      reps2[i] = make_uint2((uint32_t)r.x | (uint32_t)r.y << 16, (uint32_t)r.z | (uint32_t)r.w);
+    }
 
   // the next item's counter slot is fetched while the current item is
   // processed (two slots: slot i & 1 is read after the barrier that ends item
@@ -315,6 +364,44 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
                                    p.kv_off[s + 1], acc_a, acc_b);
           kadd(fs[s], __fmul_rn(__fsub_rn(acc_a.s, acc_a.c), p.inv_count[s]));
           kadd(fs[s], __fmul_rn(__fsub_rn(acc_b.s, acc_b.c), p.inv_count[s]));
+        }
+      }
+    }
+    if (MODE == 3) {
+      // octants, two atoms per thread: a and a + nthr (the order of one atom per step)
+      const int stride = (p.nmax + 1) * nthr;
+      for (; a_start < it.a1; a_start += 2 * nthr) {
+        const int n_at = a_start + nthr < it.a1 ? 2 : 1;
+        int32_t f[2][3];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const int a = k < n_at ? a_start + k * nthr : a_start;
+          const int atom = L.idx ? __ldg(L.idx + a) : L.first + a;
+          const float dx = __fsub_rn(__ldg(X1 + atom), __ldg(X0 + atom));
+          const float dy = __fsub_rn(__ldg(X1 + p.n_pad + atom), __ldg(X0 + p.n_pad + atom));
+          const float dz = __fsub_rn(__ldg(X1 + 2 * p.n_pad + atom), __ldg(X0 + 2 * p.n_pad + atom));
+          f[k][0] = turns_fixed(dx, p.period), f[k][1] = turns_fixed(dy, p.period), f[k][2] = turns_fixed(dz, p.period);
+          if (k < n_at && p.want_moments) {
+            const float d2 = sq3(dx, dy, dz);
+            kadd(m2, d2);
+            kadd(m4, d2 * d2);
+          }
+          if (GS && k < n_at) {
+            const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+            const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
+            if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
+          }
+        }
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax)
+          for (int n = 0; n <= p.nmax; ++n)
+            tab2[ax * stride + n * nthr + tid] = pk2(cos_fixed((int32_t)((uint32_t)n * (uint32_t)f[0][ax])),
+                                                     cos_fixed((int32_t)((uint32_t)n * (uint32_t)f[1][ax])));
+        for (int s = 0; s < n_fs; ++s) {
+          KSum acc_a, acc_b;
+          octant_shell_sum2(reps2 - p.kv_off[0], tab2 + tid, p.kv_off[s], p.kv_off[s + 1], acc_a, acc_b);
+          kadd(fs[s], __fmul_rn(__fsub_rn(acc_a.s, acc_a.c), p.inv_count[s]));
+          if (n_at == 2) kadd(fs[s], __fmul_rn(__fsub_rn(acc_b.s, acc_b.c), p.inv_count[s]));
         }
       }
     }
@@ -946,6 +1033,7 @@ struct amdat_disp_plan {
   std::vector<int32_t> lu_off, lu_units;  // list -> its units (CSR, ascending)
   amdat::DevBuf<int32_t> class_idx;       // atoms of gathered classes
   int chunk = 0, blocks_per_sm = 0, n_items = 0;
+  int64_t steps1 = 0, steps2 = 0;  // block steps of the items with one and with two atoms per F_s thread
   double tuned_ms = 0.0;
   bool bulk = false;  // MSD + NGP through the bulk-copy-staged kernel
   // device: [descriptors | pair frames | item_first | counters | kv | off | inv | lu_off | lu_units |
@@ -1013,6 +1101,11 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
       for (int i = 0; i < it.n_pairs; ++i) frames.push_back(make_int2(ht0[it.pair + i], ht1[it.pair + i]));
   }
   pl.n_items = (int)items.size();
+  pl.steps1 = pl.steps2 = 0;
+  for (const DispItem& it : items) {
+    pl.steps1 += ceil_div(it.a1 - it.a0, FS_THREADS);
+    pl.steps2 += ceil_div(it.a1 - it.a0, 2 * FS_THREADS);
+  }
   pl.chunk = chunk;
   pl.blocks_per_sm = blocks_per_sm;
   auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -1101,13 +1194,26 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
     const int mode = nfs ? pl.sh.mode : 0;
     const int threads = mode ? FS_THREADS : DISP_THREADS;
     size_t shm = gs ? (size_t)((pl.NB + 3) & ~3) * 4 : 0;
-    if (mode == 2) shm += (size_t)3 * (pl.sh.nmax + 1) * threads * 4;
-    if (mode != 0) {
+    const int n_rep_pass = mode ? pl.sh.off[s0 + nfs] - pl.sh.off[s0] : 0;
+    // Octants, two atoms per thread: 4,000 atoms x 1,100 pairs, shells around q = 7.1 with
+    // components up to 11 / 19 / 22 / 29 / 34 / 45 take 95 / 227 / 350 / 757 / 1,711 / 3,707 us
+    // (one atom: 121 / 283 / 466 / 950 / 1,777 / 7,601), so wherever the tables fit a block.
+    // A step of two atoms costs 1.3 to 1.6 steps of one: items of at most a block of
+    // atoms stay with one atom (100 atoms 30 us, 38 with two; 1,000 atoms in items of
+    // 128 89 us, 124 with two).
+    const size_t two = (size_t)3 * (pl.sh.nmax + 1) * threads * 8 + (size_t)n_rep_pass * 8;
+    const bool pair_atoms = mode == 2 && 8 * pl.steps2 <= 5 * pl.steps1 && shm + two <= 220 * 1024;
+    if (pair_atoms) {
+      p.n_rep_smem = n_rep_pass;
+      shm += two;
+    } else if (mode == 2) {
+      shm += (size_t)3 * (pl.sh.nmax + 1) * threads * 4;
+    }
+    if (mode != 0 && !pair_atoms) {
       // the pass's vectors / representatives in shared memory when they take at most 32 KB
-      const int n_rep = pl.sh.off[s0 + nfs] - pl.sh.off[s0];
-      if (n_rep <= 2048) {
-        p.n_rep_smem = n_rep;
-        shm += (size_t)n_rep * sizeof(int4);
+      if (n_rep_pass <= 2048) {
+        p.n_rep_smem = n_rep_pass;
+        shm += (size_t)n_rep_pass * sizeof(int4);
       }
     }
     auto launch = [&](auto kernel) {
@@ -1148,6 +1254,7 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
       if (gs) launch(disp_mixed_kernel<0, true>); else launch(disp_mixed_kernel<0, false>);
     }
     else if (mode == 1) { if (gs) launch(disp_mixed_kernel<1, true>); else launch(disp_mixed_kernel<1, false>); }
+    else if (pair_atoms) { if (gs) launch(disp_mixed_kernel<3, true>); else launch(disp_mixed_kernel<3, false>); }
     else { if (gs) launch(disp_mixed_kernel<2, true>); else launch(disp_mixed_kernel<2, false>); }
     disp_finalize_kernel<<<(unsigned)ceil_div((int64_t)n_ug * (2 + nfs), 8), 256, 0, ctx->stream>>>(
         p.part, pl.n_out, (const int32_t*)(base + pl.o_first), (int32_t)n_ug,
