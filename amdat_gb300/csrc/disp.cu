@@ -34,6 +34,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <map>
+#include <numeric>
 #include <memory>
 #include <cmath>
 #include <cstring>
@@ -49,6 +50,10 @@ constexpr int MAX_FS = 8;         // shells per pass
 constexpr int DISP_THREADS = 256;
 constexpr int FS_THREADS = 128;
 constexpr int MAX_PAIRS_PER_ITEM = 64;
+constexpr int SLAB_BATCH = 4;                             // entries per thread
+constexpr int SLAB_ENTRIES = SLAB_BATCH * DISP_THREADS;   // members of all units per item (slab route)
+constexpr int SLAB_UNITS = 128;
+constexpr int64_t SLAB_ROWS = 16 << 20;  // rows of partials (16 bytes each)
 constexpr size_t DISP_CACHE_PLANS = 8;  // one-shot requests kept prepared
 
 struct DispItem {
@@ -481,6 +486,82 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
         if (hist[b]) atomicAdd(dst + b, (unsigned long long)hist[b]);
     }
     __syncthreads();
+  }
+}
+
+// MSD + NGP moments of several gathered units (index lists, membership classes)
+// together.  An item is up to SLAB_ENTRIES members of all units in atom order (a slab)
+// times some pairs of one gap: a warp's 32 members are close in memory whichever units
+// they belong to, where a unit alone leaves most of every 32-byte sector unused, and the
+// slab's sums go to their units once per item, not once per pair.  Each thread keeps its
+// members' compensated sums over the item's pairs, puts them at the members' places in
+// unit order in shared memory, and groups of lanes merge each unit's run.  Bound by the
+// sectors of both frames out of L2 (64 nested lists of 50,000 out of 200,000 atoms, 427
+// pairs: 160 us at 11 TB/s, 579 us unit by unit).
+__global__ void __launch_bounds__(DISP_THREADS, 3)
+    disp_slab_kernel(const float* __restrict__ u, int64_t n_pad, const DispDesc* __restrict__ desc,
+                     const int2* __restrict__ frames, const int32_t* __restrict__ atoms,   // [slab][entry]
+                     const uint16_t* __restrict__ place,                                   // [slab][entry]
+                     const uint16_t* __restrict__ run,                                     // [slab][unit + 1]
+                     int32_t n_units, int32_t n_items, double* __restrict__ part) {
+  __shared__ float4 s_sum[SLAB_ENTRIES];
+  const int tid = threadIdx.x;
+  const DispDesc it = desc[blockIdx.x];
+  const int n = it.a1 - it.a0;
+  int64_t off[SLAB_BATCH];
+  KSum m2[SLAB_BATCH], m4[SLAB_BATCH];
+#pragma unroll
+  for (int k = 0; k < SLAB_BATCH; ++k) {
+    const int a = tid + k * DISP_THREADS;
+    off[k] = __ldg(atoms + it.a0 + min(a, n - 1));
+    m2[k] = m4[k] = KSum{0.f, 0.f};
+  }
+  for (int pr = 0; pr < it.n_pairs; ++pr) {
+    const int2 tt = __ldg(frames + it.pf + pr);
+    const float* X0 = u + (int64_t)tt.x * 3 * n_pad;
+    const float* X1 = u + (int64_t)tt.y * 3 * n_pad;
+    float d[SLAB_BATCH][3];
+#pragma unroll
+    for (int k = 0; k < SLAB_BATCH; ++k)
+#pragma unroll
+      for (int ax = 0; ax < 3; ++ax)
+        d[k][ax] = __fsub_rn(__ldg(X1 + ax * n_pad + off[k]), __ldg(X0 + ax * n_pad + off[k]));
+#pragma unroll
+    for (int k = 0; k < SLAB_BATCH; ++k) {
+      const float d2 = sq3(d[k][0], d[k][1], d[k][2]);
+      // a few terms per sum, in no order of size: error-free additions (kadd's are so only
+      // while the sum is the larger part)
+      m2[k] = kmerge(m2[k], KSum{d2, 0.f});
+      m4[k] = kmerge(m4[k], KSum{d2 * d2, 0.f});
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < SLAB_BATCH; ++k) {
+    const int a = tid + k * DISP_THREADS;
+    if (a < n) s_sum[__ldg(place + it.a0 + a)] = make_float4(m2[k].s, m2[k].c, m4[k].s, m4[k].c);
+  }
+  __syncthreads();
+  // a unit's run: a whole warp where the units are few (long runs), else 8 lanes
+  const int g = n_units <= 16 ? 32 : 8, l = tid & (g - 1);
+  const uint16_t* R = run + (int64_t)it.unit * (n_units + 1);
+  for (int c0 = 0; c0 < n_units; c0 += DISP_THREADS / g) {
+    const int c = c0 + tid / g;
+    KSum a2 = {0.f, 0.f}, a4 = {0.f, 0.f};
+    if (c < n_units)
+      for (int i = R[c] + l, e = R[c + 1]; i < e; i += g) {
+        const float4 v = s_sum[i];
+        a2 = kmerge(a2, KSum{v.x, v.y});
+        a4 = kmerge(a4, KSum{v.z, v.w});
+      }
+    for (int o = g / 2; o > 0; o >>= 1) {
+      a2 = kmerge(a2, kshfl(a2, o));
+      a4 = kmerge(a4, kshfl(a4, o));
+    }
+    if (l == 0 && c < n_units) {
+      double* P = part + ((int64_t)c * n_items + it.item) * 2;
+      P[0] = (double)a2.s - (double)a2.c;
+      P[1] = (double)a4.s - (double)a4.c;
+    }
   }
 }
 
@@ -1035,6 +1116,11 @@ struct amdat_disp_plan {
   int chunk = 0, blocks_per_sm = 0, n_items = 0;
   int64_t steps1 = 0, steps2 = 0;  // block steps of the items with one and with two atoms per F_s thread
   double tuned_ms = 0.0;
+  bool slab = false;  // moments of gathered units together, by slabs of members in atom order
+  amdat::DevBuf<unsigned char> slab_dev;  // [atoms | place | run]
+  size_t o_place = 0, o_run = 0;
+  int64_t n_entries = 0;
+  int n_slabs = 0;
   bool bulk = false;  // MSD + NGP through the bulk-copy-staged kernel
   // device: [descriptors | pair frames | item_first | counters | kv | off | inv | lu_off | lu_units |
   //          part | unit d2 | d4 | fs | gs | list d2 | d4 | fs | gs]
@@ -1052,18 +1138,48 @@ struct amdat_disp_plan {
 
 namespace amdat {
 
+// Pairs per item of the slab route.  An item's units are summed once, so items are as
+// large as still fills the chip's three blocks per SM: 12 / 8 / 4 / 2 items per SM give
+// 24 / 23 / 17 / 16 us for 6,474 atoms of 2 types over 289 pairs, 65 / 51 / 44 / 40 for 64
+// nested lists of 15,000 out of 60,000.
+static int slab_pairs(const amdat_ctx* ctx, int64_t n_pairs, int64_t n_slabs) {
+  const int64_t want = (int64_t)ctx->n_sm * 2;
+  return (int)std::min<int64_t>(MAX_PAIRS_PER_ITEM, std::max<int64_t>(1, n_pairs * n_slabs / want));
+}
+
 static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P, int chunk,
                         int blocks_per_sm) {
   const int G = pl.G;
   const size_t n_ug = (size_t)pl.n_units * G, n_lg = (size_t)pl.n_lists * G;
   std::vector<DispItem> items;
   std::vector<int32_t> item_first(n_ug + 1, 0);
+  size_t n_rows = 0;         // rows of partials
   std::vector<int64_t> key;  // schedule key per item: (unit, chunk, pair)
   // moments-only passes give a unit smaller than half a chunk several pairs
   // of one gap per item (the finalize sums a (unit, gap)'s items anyway), so
   // small lists do not pay one item's fixed cost per pair
   const bool multi_pair = pl.S == 0 && pl.NB == 0;
-  for (int u = 0; u < pl.n_units; ++u) {
+  if (pl.slab) {
+    // items gap by gap, the slabs of a few pairs next to each other; a unit's rows follow
+    // the items, so (unit, gap) is a range of rows
+    const int ppi = slab_pairs(ctx, P.n_pairs, pl.n_slabs);
+    std::vector<int32_t> gap_item(G + 1, 0);
+    for (int g = 0; g < G; ++g) {
+      gap_item[g] = (int32_t)items.size();
+      for (int pr = P.gap_first[g]; pr < P.gap_first[g + 1]; pr += ppi)
+        for (int c = 0; c < pl.n_slabs; ++c) {
+          const int64_t a0 = pl.n_entries * c / pl.n_slabs, a1 = pl.n_entries * (c + 1) / pl.n_slabs;
+          key.push_back((int64_t)items.size());
+          items.push_back(DispItem{c, pr, (int32_t)a0, (int32_t)a1, std::min(ppi, P.gap_first[g + 1] - pr)});
+        }
+    }
+    gap_item[G] = (int32_t)items.size();
+    for (int u = 0; u < pl.n_units; ++u)
+      for (int g = 0; g < G; ++g)
+        item_first[(size_t)u * G + g] = (int32_t)((size_t)u * items.size() + (size_t)gap_item[g]);
+    n_rows = (size_t)pl.n_units * items.size();
+  }
+  for (int u = 0; u < pl.n_units && !pl.slab; ++u) {
     const int nch = (int)std::max<int64_t>(1, ceil_div(pl.usize[u], chunk));
     const int ppi = (multi_pair && pl.usize[u] > 0 && 2 * pl.usize[u] <= chunk)
                         ? std::min(MAX_PAIRS_PER_ITEM, chunk / pl.usize[u])
@@ -1082,7 +1198,8 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
       }
     }
   }
-  item_first[n_ug] = (int32_t)items.size();
+  if (!pl.slab) n_rows = items.size();
+  item_first[n_ug] = (int32_t)n_rows;
   // process all pairs of one (unit, atom chunk) together: the chunk's frames
   // are read from HBM once and reused from L2 by the other pairs
   std::vector<int32_t> sched(items.size());
@@ -1094,10 +1211,10 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
   std::vector<int2> frames;
   for (size_t k = 0; k < sched.size(); ++k) {
     const DispItem& it = items[sched[k]];
-    const ListDev& L = pl.udev[it.list];
+    const ListDev L = pl.slab ? ListDev{0, 0, nullptr} : pl.udev[it.list];  // a slab's members are its entries
     desc[k] = DispDesc{sched[k], it.list, it.a0, it.a1, ht0[it.pair], ht1[it.pair],
                        hgap[it.pair], L.first, L.idx, it.n_pairs, (int32_t)frames.size()};
-    if (it.n_pairs > 1)
+    if (it.n_pairs > 1 || pl.slab)
       for (int i = 0; i < it.n_pairs; ++i) frames.push_back(make_int2(ht0[it.pair + i], ht1[it.pair + i]));
   }
   pl.n_items = (int)items.size();
@@ -1120,7 +1237,7 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
   pl.o_inv = o; o = align(o + std::max<size_t>(pl.sh.inv_count.size(), 1) * 4);
   pl.o_luo = o; o = align(o + std::max<size_t>(pl.lu_off.size(), 1) * 4);
   pl.o_luu = o; o = align(o + std::max<size_t>(pl.lu_units.size(), 1) * 4);
-  pl.o_part = o; o = align(o + (size_t)std::max(pl.n_items, 1) * pl.n_out * 8);
+  pl.o_part = o; o = align(o + std::max<size_t>(n_rows, 1) * pl.n_out * 8);
   pl.o_ud2 = o; o = align(o + n_ug * 8);
   pl.o_ud4 = o; o = align(o + n_ug * 8);
   pl.o_ufs = o; o = align(o + n_ug * S1 * 8);
@@ -1236,7 +1353,15 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
       check_launch("disp_mixed_kernel");
       count_launch(ctx);
     };
-    if (mode == 0 && !gs && pl.bulk) {
+    if (pl.slab) {
+      const unsigned char* sb = pl.slab_dev.ptr;
+      KernelTimer kt(ctx, "disp_mixed_kernel");
+      disp_slab_kernel<<<(unsigned)pl.n_items, DISP_THREADS, 0, ctx->stream>>>(
+          p.u, p.n_pad, p.desc, p.frames, (const int32_t*)sb, (const uint16_t*)(sb + pl.o_place),
+          (const uint16_t*)(sb + pl.o_run), pl.n_units, pl.n_items, p.part);
+      check_launch("disp_slab_kernel");
+      count_launch(ctx);
+    } else if (mode == 0 && !gs && pl.bulk) {
       auto bulk = [&](auto kernel, size_t smem_bytes, int per_sm) {
         const size_t bshm = smem_bytes + 128;
         AMDAT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bshm));
@@ -1392,6 +1517,71 @@ static void plan_classes(amdat_ctx* ctx, amdat_disp_plan& pl, const int32_t* lis
   pl.lu_off[L] = (int32_t)pl.lu_units.size();
 }
 
+// The slab route of MSD + NGP moments over several units, taken where it reads less than
+// the units one by one.  The units' kernel reads contiguous members at 0.75 of the slab
+// kernel's time per member, gathered ones at 0.55 of it per atom of the range that they
+// are scattered over (whole 32-byte sectors, whichever atoms of them are members; 0.65 for
+// 2 units, 0.47 for 9).
+// 200,000 atoms, 427 pairs, units one by one / slabs: 2 random types 314 / 248 us, 3
+// interleaved 413 / 246, 9 random 1,063 / 259, 100 random 3,519 / 295; 8 random types in
+// half the atoms, the others contiguous 564 / 264; 2 in a quarter of them 215 / 247; 2
+// contiguous 178.  64 nested lists of up to 50,000: 579 / 160.
+// Entry tables: the members of all units in atom order (an atom of several units once for
+// each), cut into slabs of at most SLAB_ENTRIES; per entry its place in the slab's unit
+// order, per slab the units' runs there.
+static void plan_slabs(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P) {
+  const int64_t N = ctx->n_atoms;
+  std::vector<std::vector<int32_t>> idx(pl.n_units);
+  std::vector<int64_t> at(N + 1, 0);  // first entry of each atom
+  double by_unit = 0.0;               // time of the units one by one, in entries of the slab kernel
+  int64_t n = 0;
+  for (int u = 0; u < pl.n_units; ++u) {
+    const ListDev& L = pl.udev[u];
+    idx[u].resize(pl.usize[u]);
+    if (L.idx)
+      AMDAT_CUDA(cudaMemcpy(idx[u].data(), L.idx, (size_t)pl.usize[u] * 4, cudaMemcpyDeviceToHost));
+    else
+      std::iota(idx[u].begin(), idx[u].end(), L.first);
+    n += pl.usize[u];
+    if (!L.idx) {
+      by_unit += 0.75 * pl.usize[u];
+    } else if (pl.usize[u]) {
+      by_unit += 0.55 * (idx[u].back() - idx[u].front() + 1);  // lists are ascending
+    }
+  }
+  const int64_t slabs = ceil_div(n, SLAB_ENTRIES);
+  const int64_t rows = n ? pl.n_units * slabs * (pl.G + P.n_pairs / slab_pairs(ctx, P.n_pairs, slabs)) : 0;
+  if (by_unit <= (double)n || rows > SLAB_ROWS) return;
+  for (int u = 0; u < pl.n_units; ++u)
+    for (int32_t a : idx[u]) ++at[a + 1];
+  for (int64_t a = 0; a < N; ++a) at[a + 1] += at[a];
+  std::vector<int32_t> atoms(n), unit(n);
+  for (int u = 0; u < pl.n_units; ++u)
+    for (int32_t a : idx[u]) {
+      const int64_t e = at[a]++;
+      atoms[e] = a;
+      unit[e] = u;
+    }
+  pl.n_entries = n;
+  pl.n_slabs = (int)slabs;
+  std::vector<uint16_t> place(n), run((size_t)pl.n_slabs * (pl.n_units + 1), 0);
+  for (int c = 0; c < pl.n_slabs; ++c) {
+    const int64_t e0 = n * c / pl.n_slabs, e1 = n * (c + 1) / pl.n_slabs;
+    uint16_t* R = run.data() + (size_t)c * (pl.n_units + 1);
+    for (int64_t e = e0; e < e1; ++e) ++R[unit[e] + 1];
+    for (int u = 0; u < pl.n_units; ++u) R[u + 1] = (uint16_t)(R[u + 1] + R[u]);
+    std::vector<uint16_t> next(R, R + pl.n_units);
+    for (int64_t e = e0; e < e1; ++e) place[e] = next[unit[e]]++;
+  }
+  pl.o_place = (size_t)n * 4;
+  pl.o_run = pl.o_place + (size_t)n * 2;
+  unsigned char* base = pl.slab_dev.reserve(pl.o_run + run.size() * 2);
+  AMDAT_CUDA(cudaMemcpy(base, atoms.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
+  AMDAT_CUDA(cudaMemcpy(base + pl.o_place, place.data(), (size_t)n * 2, cudaMemcpyHostToDevice));
+  AMDAT_CUDA(cudaMemcpy(base + pl.o_run, run.data(), run.size() * 2, cudaMemcpyHostToDevice));
+  pl.slab = true;
+}
+
 static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* req,
                                     const int32_t* lists, int32_t n_lists, int32_t flags) {
   check_request(ctx, req);
@@ -1442,6 +1632,8 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       for (const ListDev& u : pl->udev) contiguous = contiguous && u.idx == nullptr;
       pl->bulk = kern && std::strcmp(kern, "bulk") == 0 && pl->S == 0 && pl->NB == 0 && contiguous;
     }
+    if (pl->S == 0 && pl->NB == 0 && !pl->bulk && pl->n_units > 1 && pl->n_units <= SLAB_UNITS && P.n_pairs > 0)
+      plan_slabs(ctx, *pl, P);
     // default tile: full chunks stream memory; F_s or few pairs want smaller
     // chunks to keep every SM busy
     const int64_t want_items = (int64_t)ctx->n_sm * 16;
@@ -1449,12 +1641,13 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     if (P.n_pairs > 0 && unit_atoms > 0)
       chunk = std::max<int64_t>(pl->S ? 128 : 1024,
                                 std::min<int64_t>(DISP_CHUNK, ceil_div(unit_atoms * P.n_pairs, want_items)));
+    if (pl->slab) chunk = SLAB_ENTRIES;  // its one tile
     // list-mode F_s holds few registers and only its vectors in shared memory:
     // more resident blocks hide the latency of its cosine chain
     int bps = pl->S ? (pl->sh.mode == 1 ? 8 : 4) : 8;
     char keybuf[256];
     std::snprintf(keybuf, sizeof(keybuf), "sm%d_mode%d%s_S%d_NB%d_L%d_U%d_atoms%lld_unit%lld_pairs%lld",
-                  ctx->n_sm, pl->S ? pl->sh.mode : 0, pl->bulk ? "b" : "", pl->S, pl->NB, n_lists, pl->n_units,
+                  ctx->n_sm, pl->S ? pl->sh.mode : 0, pl->bulk ? "b" : (pl->slab ? "s" : ""), pl->S, pl->NB, n_lists, pl->n_units,
                   (long long)total_atoms, (long long)unit_atoms, (long long)P.n_pairs);
     const std::string key(keybuf);
     auto hit = tune_cache().find(key);
@@ -1465,9 +1658,11 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       // time each candidate (warm-up + 3 runs, CUDA events) and keep the fastest
       // candidates: F_s is compute bound (small chunks, fewer heavier blocks);
       // MSD-only streams memory (large chunks, more resident blocks)
-      const std::vector<int> chunks = pl->S ? std::vector<int>{256, 512, 1024, 2048}
+      const std::vector<int> chunks = pl->slab ? std::vector<int>{SLAB_ENTRIES}
+                                      : pl->S ? std::vector<int>{256, 512, 1024, 2048}
                                             : std::vector<int>{1024, 2048, 4096, 8192};
-      const std::vector<int> bpss = pl->S ? (pl->sh.mode == 1 ? std::vector<int>{4, 8, 16} : std::vector<int>{2, 4, 8})
+      const std::vector<int> bpss = pl->slab ? std::vector<int>{bps}
+                                    : pl->S ? (pl->sh.mode == 1 ? std::vector<int>{4, 8, 16} : std::vector<int>{2, 4, 8})
                                           : std::vector<int>{4, 8};
       cudaEvent_t a, b;
       AMDAT_CUDA(cudaEventCreate(&a));
