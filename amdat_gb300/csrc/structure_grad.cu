@@ -118,6 +118,18 @@ __device__ __forceinline__ void gauss_bins(const SGParams& p, float r, float inv
   }
 }
 
+// Adds y >= 0, rounded to an integer, to the 64-bit sum (lo[b], hi[b]) in shared memory:
+// 32-bit integer atomics are native there, a 64-bit one is a compare-and-swap loop.
+// Exact: y * 2^-32 and the remainder are FP32 numbers, and a y with a high part is an
+// integer already.
+__device__ __forceinline__ void add_fixed(uint32_t* lo, uint32_t* hi, int b, float y) {
+  uint32_t h = __float2uint_rz(__fmul_rn(y, 2.3283064365386963e-10f));
+  const uint32_t l = __float2uint_rn(fmaf((float)h, -4294967296.0f, y));
+  const uint32_t sum = atomicAdd(lo + b, l) + l;
+  h += sum < l;  // carry
+  if (h) atomicAdd(hi + b, h);
+}
+
 constexpr int SG_WARPS = SG_THREADS / 32;
 constexpr int SG_Q = 64;  // per-warp queue of in-range pairs
 
@@ -126,18 +138,18 @@ constexpr int SG_Q = 64;  // per-warp queue of in-range pairs
 // their bins are processed 32 at a time, so the bin loop runs with every lane
 // busy.  Each Gaussian term is rounded once to a fixed-point integer (scale
 // 2^q chosen by the host so that a block's sum cannot overflow 63 bits) and
-// added with 64-bit shared-memory integer atomics: the block histogram is
+// added in shared memory with integer atomics: the block histogram is
 // exact and independent of the order of the additions, so the forward is
 // deterministic and finite differences of it see only the terms that change.
 __global__ void __launch_bounds__(SG_THREADS) gsmooth_kernel(SGParams p, float qscale) {
-  extern __shared__ double sh_d[];  // [n_bins] as unsigned 64-bit fixed point
-  unsigned long long* sh_q = reinterpret_cast<unsigned long long*>(sh_d);
+  extern __shared__ double sh_d[];  // unsigned 64-bit fixed point: low words [n_bins], high words [n_bins]
+  uint32_t *sh_lo = reinterpret_cast<uint32_t*>(sh_d), *sh_hi = sh_lo + p.n_bins;
   __shared__ float sx[SG_JT], sy[SG_JT], sz[SG_JT];
   __shared__ float q_r[SG_WARPS][SG_Q];
   const int f = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* P = p.w + (int64_t)p.frames[f] * 3 * p.n_pad;
-  for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x) sh_q[b] = 0ull;
+  for (int b = threadIdx.x; b < 2 * p.n_bins; b += blockDim.x) sh_lo[b] = 0u;
   const int i0 = blockIdx.x * SG_THREADS, i = i0 + threadIdx.x;
   const bool live = i < p.lst.n;
   float xi = 0.f, yi = 0.f, zi = 0.f;
@@ -154,7 +166,7 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_kernel(SGParams p, float q
   auto flush = [&](int count) {  // lanes < count take one queued pair each
     if (lane < count)
       gauss_bins(p, q_r[warp][lane], inv2s2, recur, [&](int b, float, float G) {
-        atomicAdd(sh_q + b, (unsigned long long)__float2ll_rn(qnorm * G));
+        add_fixed(sh_lo, sh_hi, b, qnorm * G);
       });
   };
   int qn = 0;  // warp-uniform queue length
@@ -187,7 +199,20 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_kernel(SGParams p, float q
   __syncthreads();
   const double inv_q = 1.0 / (double)qscale;
   for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x)
-    if (sh_q[b]) atomicAdd(p.h + b, (double)sh_q[b] * inv_q);
+    if (const unsigned long long v = (unsigned long long)sh_hi[b] << 32 | sh_lo[b]) atomicAdd(p.h + b, (double)v * inv_q);
+}
+
+// The entries of the queue's first `count` (<= 32) that belong to this lane, as a mask:
+// the lowest entry of each owner writes the owner's mask.
+__device__ __forceinline__ unsigned owned(const unsigned char* q_o, int count, unsigned* q_m) {
+  const int lane = threadIdx.x & 31;
+  q_m[lane] = 0u;
+  __syncwarp();
+  const int o = lane < count ? q_o[lane] : 32;
+  const unsigned m = __match_any_sync(0xffffffffu, o);
+  if (lane < count && __ffs(m) - 1 == lane) q_m[o] = m;
+  __syncwarp();
+  return q_m[lane];
 }
 
 // adjoint: each atom i gathers psi(r_ij) (r_i - r_j) / r_ij over every j != i.
@@ -201,6 +226,7 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_adjoint_kernel(SGParams p)
   __shared__ float sx[SG_JT], sy[SG_JT], sz[SG_JT];
   __shared__ float4 q_v[SG_WARPS][SG_Q];  // (dx, dy, dz, r); after a flush: (s dx, s dy, s dz, -)
   __shared__ unsigned char q_o[SG_WARPS][SG_Q];
+  __shared__ unsigned q_m[SG_WARPS][32];
   const int f = blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* P = p.w + (int64_t)p.frames[f] * 3 * p.n_pad;
@@ -231,13 +257,12 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_adjoint_kernel(SGParams p)
     __syncwarp();
     // owners add their entries in queue order (compensated)
     float part[3] = {0.f, 0.f, 0.f};
-    for (int e = 0; e < count; ++e)
-      if (q_o[warp][e] == lane) {
-        const float4 v = q_v[warp][e];
-        part[0] += v.x;
-        part[1] += v.y;
-        part[2] += v.z;
-      }
+    for (unsigned m = owned(q_o[warp], count, q_m[warp]); m; m &= m - 1) {
+      const float4 v = q_v[warp][__ffs(m) - 1];
+      part[0] += v.x;
+      part[1] += v.y;
+      part[2] += v.z;
+    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const float y = __fsub_rn(part[d], c[d]), t = __fadd_rn(g[d], y);
@@ -357,24 +382,28 @@ __global__ void cell_scatter_kernel(const int32_t* __restrict__ cell_of, int32_t
   if (i < n) order[atomicAdd(cursor + cell_of[i], 1)] = i;
 }
 
-// ascending list order inside each cell, then the sorted positions
-__global__ void cell_sort_kernel(const int32_t* __restrict__ start, int32_t n_cells, int32_t* __restrict__ order,
-                                 const float* __restrict__ P, int64_t n_pad, SGList lst, float4* __restrict__ pos) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// ascending list order inside each cell and the positions in that order: a warp per
+// cell, an atom's place being the number of the cell's list indices below its own
+__global__ void cell_sort_kernel(const int32_t* __restrict__ start, int32_t n_cells, const int32_t* __restrict__ in,
+                                 int32_t* __restrict__ order, const float* __restrict__ P, int64_t n_pad, SGList lst,
+                                 float4* __restrict__ pos) {
+  const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (c >= n_cells) return;
   const int b = start[c], e = start[c + 1];
-  for (int k = b + 1; k < e; ++k) {
-    const int v = order[k];
-    int m = k - 1;
-    while (m >= b && order[m] > v) {
-      order[m + 1] = order[m];
-      --m;
+  for (int k0 = b; k0 < e; k0 += 32) {
+    const bool own = k0 + lane < e;
+    const int v = own ? in[k0 + lane] : 0;
+    int rank = 0;
+    for (int m0 = b; m0 < e; m0 += 32) {
+      const int w = m0 + lane < e ? in[m0 + lane] : INT32_MAX;
+      const int nm = min(32, e - m0);
+      for (int m = 0; m < nm; ++m) rank += __shfl_sync(0xffffffffu, w, m) < v;
     }
-    order[m + 1] = v;
-  }
-  for (int k = b; k < e; ++k) {
-    const int a = sg_member(lst, order[k]);
-    pos[k] = make_float4(P[a], P[n_pad + a], P[2 * n_pad + a], 0.f);
+    if (own) {
+      const int a = sg_member(lst, v);
+      order[b + rank] = v;
+      pos[b + rank] = make_float4(P[a], P[n_pad + a], P[2 * n_pad + a], 0.f);
+    }
   }
 }
 
@@ -390,18 +419,23 @@ __device__ __forceinline__ int neighbour_cell(const SGCells& C, float4 p, int of
   return (cz * C.nc.y + cy) * C.nc.x + cx;
 }
 
-// forward over cells: thread per sorted slot, partners j > i (list order) in
-// the 27 cells; queue and bins as in gsmooth_kernel
+// forward over cells: thread per sorted slot, partners in the slots after its own in
+// its cell and in the 13 neighbours after it in the order of neighbour_cell (with three
+// or more cells per axis each pair of cells is met once); queue and bins as in
+// gsmooth_kernel.  SGC_PARTS lanes share a slot's cells.  Bound by issue: 6.5 tests per
+// pair in range and 25 bins of a pair (100,000 atoms, cutoff 4.12, 400 bins, per frame:
+// 1,770 us with every ordered pair tested and 64-bit atomics, 550 so).
+template <int SGC_PARTS>
 __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_kernel(SGParams p, SGCells C, float qscale) {
   extern __shared__ double sh_d[];
-  unsigned long long* sh_q = reinterpret_cast<unsigned long long*>(sh_d);
+  uint32_t *sh_lo = reinterpret_cast<uint32_t*>(sh_d), *sh_hi = sh_lo + p.n_bins;
   __shared__ float q_r[SG_WARPS][SG_Q];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x) sh_q[b] = 0ull;
+  for (int b = threadIdx.x; b < 2 * p.n_bins; b += blockDim.x) sh_lo[b] = 0u;
   __syncthreads();
-  const int slot = blockIdx.x * SG_THREADS + threadIdx.x;
+  const int slot = blockIdx.x * (SG_THREADS / SGC_PARTS) + warp * (32 / SGC_PARTS) + lane % (32 / SGC_PARTS);
+  const int part = lane / (32 / SGC_PARTS);
   const bool live = slot < p.lst.n;
-  const int i = live ? C.order[slot] : -1;
   const float4 pi = live ? C.pos[slot] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float inv2s2 = 0.5f / (p.sigma * p.sigma);
   const float qnorm = qscale * INV_SQRT_2PI / p.sigma;
@@ -410,25 +444,27 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_kernel(SGParams p, S
   auto flush = [&](int count) {
     if (lane < count)
       gauss_bins(p, q_r[warp][lane], inv2s2, recur, [&](int b, float, float G) {
-        atomicAdd(sh_q + b, (unsigned long long)__float2ll_rn(qnorm * G));
+        add_fixed(sh_lo, sh_hi, b, qnorm * G);
       });
   };
   int qn = 0;
-  for (int off = 0; off < 27; ++off) {
-    const int nb = live ? neighbour_cell(C, pi, off) : 0;
-    const int cs = live ? C.start[nb] : 0, len = live ? C.start[nb + 1] - cs : 0;
+  for (int off0 = 13; off0 < 27; off0 += SGC_PARTS) {
+    const int off = off0 + part;
+    const bool cell = live && off < 27;
+    const int nb = cell ? neighbour_cell(C, pi, off) : 0;
+    const int cs = off == 13 ? slot + 1 : (cell ? C.start[nb] : 0);
+    const int len = cell ? C.start[nb + 1] - cs : 0;
     const int maxlen = __reduce_max_sync(0xffffffffu, len);
     for (int k = 0; k < maxlen; ++k) {
       bool in = false;
       float r2 = 0.f;
       if (k < len) {
-        const int j = C.order[cs + k];
         const float4 pj = C.pos[cs + k];
         const float dx = min_image(pj.x - pi.x, p.box.x, p.inv_box.x);
         const float dy = min_image(pj.y - pi.y, p.box.y, p.inv_box.y);
         const float dz = min_image(pj.z - pi.z, p.box.z, p.inv_box.z);
         r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        in = j > i && r2 < p.cut2;
+        in = r2 < p.cut2;
       }
       const unsigned m = __ballot_sync(0xffffffffu, in);
       if (in) q_r[warp][qn + __popc(m & below)] = sqrtf(r2);
@@ -448,20 +484,25 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_kernel(SGParams p, S
   __syncthreads();
   const double inv_q = 1.0 / (double)qscale;
   for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x)
-    if (sh_q[b]) atomicAdd(p.h + b, (double)sh_q[b] * inv_q);
+    if (const unsigned long long v = (unsigned long long)sh_hi[b] << 32 | sh_lo[b]) atomicAdd(p.h + b, (double)v * inv_q);
 }
 
 // adjoint over cells: thread per sorted slot, every partner j != i in the 27
-// cells, owner-ordered sums as in gsmooth_adjoint_kernel
+// cells, owner-ordered sums as in gsmooth_adjoint_kernel, SGC_PARTS lanes per slot
+// (100,000 atoms, cutoff 4.12, per frame: 1,050 us with one lane per slot and every queue
+// entry looked at by every lane, 870 so)
+template <int SGC_PARTS>
 __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_adjoint_kernel(SGParams p, SGCells C, int32_t frame) {
   extern __shared__ double sh_d[];
   float* sh_w = (float*)sh_d;
   __shared__ float4 q_v[SG_WARPS][SG_Q];
   __shared__ unsigned char q_o[SG_WARPS][SG_Q];
+  __shared__ unsigned q_m[SG_WARPS][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int b = threadIdx.x; b < p.n_bins; b += blockDim.x) sh_w[b] = (float)p.wgt[b];
   __syncthreads();
-  const int slot = blockIdx.x * SG_THREADS + threadIdx.x;
+  const int slot = blockIdx.x * (SG_THREADS / SGC_PARTS) + warp * (32 / SGC_PARTS) + lane % (32 / SGC_PARTS);
+  const int part = lane / (32 / SGC_PARTS);
   const bool live = slot < p.lst.n;
   const int i = live ? C.order[slot] : -1;
   const float4 pi = live ? C.pos[slot] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -480,37 +521,37 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_adjoint_kernel(SGPar
       q_v[warp][lane] = make_float4(sc * v.x, sc * v.y, sc * v.z, 0.f);
     }
     __syncwarp();
-    float part[3] = {0.f, 0.f, 0.f};
-    for (int e = 0; e < count; ++e)
-      if (q_o[warp][e] == lane) {
-        const float4 v = q_v[warp][e];
-        part[0] += v.x;
-        part[1] += v.y;
-        part[2] += v.z;
-      }
+    float own[3] = {0.f, 0.f, 0.f};
+    for (unsigned m = owned(q_o[warp], count, q_m[warp]); m; m &= m - 1) {
+      const float4 v = q_v[warp][__ffs(m) - 1];
+      own[0] += v.x;
+      own[1] += v.y;
+      own[2] += v.z;
+    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const float y = __fsub_rn(part[d], c[d]), t = __fadd_rn(g[d], y);
+      const float y = __fsub_rn(own[d], c[d]), t = __fadd_rn(g[d], y);
       c[d] = __fsub_rn(__fsub_rn(t, g[d]), y);
       g[d] = t;
     }
   };
   int qn = 0;
-  for (int off = 0; off < 27; ++off) {
-    const int nb = live ? neighbour_cell(C, pi, off) : 0;
-    const int cs = live ? C.start[nb] : 0, len = live ? C.start[nb + 1] - cs : 0;
+  for (int off0 = 0; off0 < 27; off0 += SGC_PARTS) {
+    const int off = off0 + part;
+    const bool cell = live && off < 27;
+    const int nb = cell ? neighbour_cell(C, pi, off) : 0;
+    const int cs = cell ? C.start[nb] : 0, len = cell ? C.start[nb + 1] - cs : 0;
     const int maxlen = __reduce_max_sync(0xffffffffu, len);
     for (int k = 0; k < maxlen; ++k) {
       bool in = false;
       float dx = 0.f, dy = 0.f, dz = 0.f, r2 = 0.f;
       if (k < len) {
-        const int j = C.order[cs + k];
         const float4 pj = C.pos[cs + k];
         dx = min_image(pi.x - pj.x, p.box.x, p.inv_box.x);
         dy = min_image(pi.y - pj.y, p.box.y, p.inv_box.y);
         dz = min_image(pi.z - pj.z, p.box.z, p.inv_box.z);
         r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        in = j != i && r2 < p.cut2 && r2 > 0.f;
+        in = cs + k != slot && r2 < p.cut2 && r2 > 0.f;
       }
       const unsigned m = __ballot_sync(0xffffffffu, in);
       if (in) {
@@ -534,7 +575,18 @@ __global__ void __launch_bounds__(SG_THREADS) gsmooth_cells_adjoint_kernel(SGPar
   }
   __syncwarp();
   flush(qn);
-  if (live) {
+  // the slot's parts, in a fixed order (error-free sums of the leading parts)
+#pragma unroll
+  for (int o = 16; o >= 32 / SGC_PARTS; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float gb = __shfl_xor_sync(0xffffffffu, g[d], o), cb = __shfl_xor_sync(0xffffffffu, c[d], o);
+      const float t = __fadd_rn(g[d], gb), bb = __fsub_rn(t, g[d]);
+      const float err = __fadd_rn(__fsub_rn(g[d], __fsub_rn(t, bb)), __fsub_rn(gb, bb));
+      c[d] = __fsub_rn(__fadd_rn(c[d], cb), err);
+      g[d] = t;
+    }
+  if (live && part == 0) {
     float* out = p.grad + ((int64_t)frame * p.lst.n + i) * 3;
 #pragma unroll
     for (int d = 0; d < 3; ++d) out[d] = __fsub_rn(g[d], c[d]);
@@ -878,6 +930,13 @@ static bool cell_grid(amdat_ctx* ctx, const ListEntry& e, float cut, int3& nc) {
   return e.n >= 1024 && nc.x >= 3 && nc.y >= 3 && nc.z >= 3 && cells <= (1 << 22);
 }
 
+// Lanes per slot of the cell kernels: enough warps to fill the chip, but lanes of one warp
+// in fewer cells are closer in length.  Per frame, forward / adjoint, 1, 4 and 8 lanes:
+// 3,000 atoms 674 / 860, 214 / 276, 128 / 165 us; 20,000 683 / 859, 236 / 316, 171 / 309;
+// 100,000 702 / 966, 554 / 866, 541 / 905; 400,000 1,793 / 2,842, 1,810 / 2,909, 1,893 /
+// 3,190.
+static int cell_parts(const ListEntry& e) { return e.n < 40000 ? 8 : 4; }
+
 // builds one frame's cell lists in ctx->scratch2 and returns their view
 static SGCells build_cells(amdat_ctx* ctx, const ListEntry& e, int32_t frame, int3 nc) {
   const int n = e.n, n_cells = nc.x * nc.y * nc.z;
@@ -886,6 +945,7 @@ static SGCells build_cells(amdat_ctx* ctx, const ListEntry& e, int32_t frame, in
   const size_t o_cnt = o; o = align256(o + (size_t)n_cells * 4);
   const size_t o_start = o; o = align256(o + (size_t)(n_cells + 1) * 4);
   const size_t o_cur = o; o = align256(o + (size_t)n_cells * 4);
+  const size_t o_in = o; o = align256(o + (size_t)n * 4);
   const size_t o_ord = o; o = align256(o + (size_t)n * 4);
   const size_t o_pos = o; o = align256(o + (size_t)n * sizeof(float4));
   unsigned char* b = ctx->scratch2.reserve(o);
@@ -899,15 +959,15 @@ static SGCells build_cells(amdat_ctx* ctx, const ListEntry& e, int32_t frame, in
   C.pos = (const float4*)(b + o_pos);
   cudaStream_t st = ctx->stream;
   AMDAT_CUDA(cudaMemsetAsync(b + o_cnt, 0, (size_t)n_cells * 4, st));
-  const unsigned gn = (unsigned)ceil_div(n, 256), gc = (unsigned)ceil_div(n_cells, 256);
+  const unsigned gn = (unsigned)ceil_div(n, 256), gc = (unsigned)ceil_div(n_cells, 8);
   cell_assign_kernel<<<gn, 256, 0, st>>>(P, ctx->n_pad, sglist(e), C.lo, C.inv_cell, nc, (int32_t*)(b + o_cell),
                                          (int32_t*)(b + o_cnt));
   cell_scan_kernel<<<1, 1024, 0, st>>>((const int32_t*)(b + o_cnt), n_cells, (int32_t*)(b + o_start),
                                        (int32_t*)(b + o_cur));
   cell_scatter_kernel<<<gn, 256, 0, st>>>((const int32_t*)(b + o_cell), n, (int32_t*)(b + o_cur),
-                                          (int32_t*)(b + o_ord));
-  cell_sort_kernel<<<gc, 256, 0, st>>>((const int32_t*)(b + o_start), n_cells, (int32_t*)(b + o_ord), P,
-                                       ctx->n_pad, sglist(e), (float4*)(b + o_pos));
+                                          (int32_t*)(b + o_in));
+  cell_sort_kernel<<<gc, 256, 0, st>>>((const int32_t*)(b + o_start), n_cells, (const int32_t*)(b + o_in),
+                                       (int32_t*)(b + o_ord), P, ctx->n_pad, sglist(e), (float4*)(b + o_pos));
   check_launch("cell lists");
   count_launch(ctx, 4);
   return C;
@@ -951,11 +1011,13 @@ amdat_status amdat_gsmooth_run(amdat_ctx* ctx, int32_t list, const int32_t* fram
       const size_t shm = (size_t)n_bins * 8;
       int3 nc;
       if (cell_grid(ctx, e, std::sqrt(p.cut2), nc)) {
-        set_smem((const void*)gsmooth_cells_kernel, shm);
+        const int parts = cell_parts(e);
+        auto kernel = parts == 8 ? gsmooth_cells_kernel<8> : gsmooth_cells_kernel<4>;
+        set_smem((const void*)kernel, shm);
         for (int f = 0; f < n_frames; ++f) {
           const SGCells C = build_cells(ctx, e, frames[f], nc);
           KernelTimer kt(ctx, "gsmooth_kernel");
-          gsmooth_cells_kernel<<<(unsigned)ceil_div(e.n, SG_THREADS), SG_THREADS, shm, ctx->stream>>>(p, C, qscale);
+          kernel<<<(unsigned)ceil_div(e.n, SG_THREADS / parts), SG_THREADS, shm, ctx->stream>>>(p, C, qscale);
           check_launch("gsmooth_cells_kernel");
           count_launch(ctx);
         }
@@ -998,11 +1060,13 @@ amdat_status amdat_gsmooth_adjoint(amdat_ctx* ctx, int32_t list, const int32_t* 
       const size_t shm = (size_t)n_bins * 4;
       int3 nc;
       if (cell_grid(ctx, e, std::sqrt(p.cut2), nc)) {
-        set_smem((const void*)gsmooth_cells_adjoint_kernel, shm);
+        const int parts = cell_parts(e);
+        auto kernel = parts == 8 ? gsmooth_cells_adjoint_kernel<8> : gsmooth_cells_adjoint_kernel<4>;
+        set_smem((const void*)kernel, shm);
         for (int f = 0; f < n_frames; ++f) {
           const SGCells C = build_cells(ctx, e, frames[f], nc);
           KernelTimer kt(ctx, "gsmooth_adjoint_kernel");
-          gsmooth_cells_adjoint_kernel<<<(unsigned)ceil_div(e.n, SG_THREADS), SG_THREADS, shm, ctx->stream>>>(
+          kernel<<<(unsigned)ceil_div(e.n, SG_THREADS / parts), SG_THREADS, shm, ctx->stream>>>(
               p, C, f);
           check_launch("gsmooth_cells_adjoint_kernel");
           count_launch(ctx);
