@@ -132,7 +132,7 @@ struct Density {
   int32_t n_list = 0;              // list size when the density was computed
   std::string lattice_key;         // lattice densities: the plan key (kmax, dk, period)
   std::vector<int32_t> frames;     // system frame of each row
-  std::vector<int32_t> kvec;       // [3*n_k] (lattice mode: shell-sorted)
+  std::shared_ptr<const std::vector<int32_t>> kvec;  // [3*n_k] (lattice mode: shell-sorted, the plan's)
   std::vector<int32_t> shell_off;  // lattice mode
   DevBuf<float2>* rho = nullptr;   // [n_frames][n_k], from the context's pool
 };

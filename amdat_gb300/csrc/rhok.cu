@@ -377,7 +377,7 @@ static void run_list_density(amdat_ctx* ctx, Density& d, float period, int32_t p
   kv.reserve(std::max(d.n_k, 1));
   std::vector<int4> hk(d.n_k);
   for (int k = 0; k < d.n_k; ++k)
-    hk[k] = make_int4(d.kvec[3 * k], d.kvec[3 * k + 1], d.kvec[3 * k + 2], 0);
+    hk[k] = make_int4((*d.kvec)[3 * k], (*d.kvec)[3 * k + 1], (*d.kvec)[3 * k + 2], 0);
   if (d.n_k) AMDAT_CUDA(cudaMemcpyAsync(kv.ptr, hk.data(), d.n_k * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
   DevBuf<int32_t> d_frames;
   if (e.n == 0 || d.n_k == 0) {
@@ -580,7 +580,8 @@ void rhok_tc_run(amdat_ctx* ctx, const HalfPlan& P, const int4* fx, int32_t n_li
                  int32_t n_k, float2* rho);
 
 struct LatticePlanDev {
-  std::vector<int32_t> kvec, shell_off;
+  std::shared_ptr<const std::vector<int32_t>> kvec;  // shared with the densities made from the plan
+  std::vector<int32_t> shell_off;
   DevBuf<LatticeTile> tiles;
   DevBuf<int32_t> entry_k;
   int32_t n_tiles = 0;
@@ -600,7 +601,7 @@ void lattice_plans_free(amdat_ctx* ctx) {
 TcPlan* lattice_tc_plan(amdat_ctx* ctx, const std::string& lattice_key) {
   auto it = ctx->lattice_plans.find(lattice_key);
   AMDAT_REQUIRE(it != ctx->lattice_plans.end(), "lattice plan not found");
-  if (!it->second->tc) it->second->tc = tc_plan_build(it->second->kvec);
+  if (!it->second->tc) it->second->tc = tc_plan_build(*it->second->kvec);
   return it->second->tc;
 }
 
@@ -695,7 +696,7 @@ amdat_status amdat_wave_density(amdat_ctx* ctx, int32_t list, const int32_t* kve
     d->period = period;
     d->n_list = list_entry(ctx, list).n;
     d->frames.assign(frames, frames + n_frames);
-    d->kvec.assign(kvec_n, kvec_n + 3 * (size_t)n_k);
+    d->kvec = std::make_shared<const std::vector<int32_t>>(kvec_n, kvec_n + 3 * (size_t)n_k);
     try {
       run_list_density(ctx, *d, period, precision);
     } catch (...) {
@@ -726,7 +727,7 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
     if (it == ctx->lattice_plans.end()) {
       LatticePlan P = plan_lattice(kmax, dk, period);
       auto* pd = new LatticePlanDev();
-      pd->kvec = std::move(P.kvec);
+      pd->kvec = std::make_shared<const std::vector<int32_t>>(std::move(P.kvec));
       pd->shell_off = std::move(P.shell_off);
       pd->n_tiles = (int32_t)P.tiles.size();
       pd->tiles.reserve(P.tiles.size());
@@ -738,7 +739,7 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
     const LatticePlanDev& P = *it->second;
     auto* d = new Density();
     d->list = list;
-    d->n_k = (int32_t)(P.kvec.size() / 3);
+    d->n_k = (int32_t)(P.kvec->size() / 3);
     d->n_frames = n_frames;
     d->n_shells = (int32_t)P.shell_off.size() - 1;
     d->period = period;
@@ -756,7 +757,7 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
         int4* fx = fixed_turns(ctx, *d, e, period, d_frames);
         if (use_tensor_cores(ctx)) {
           LatticePlanDev& pw = *it->second;
-          if (!pw.half) pw.half = half_plan_build(pw.kvec);
+          if (!pw.half) pw.half = half_plan_build(*pw.kvec);
           rhok_tc_run(ctx, *pw.half, fx, e.n, n_frames, d->n_k, d->rho->ptr);
         } else {
           dim3 grid((unsigned)P.n_tiles, (unsigned)n_frames);
@@ -784,7 +785,7 @@ amdat_status amdat_wave_density_vectors(amdat_ctx* ctx, int32_t handle, int32_t*
   return guarded([&] {
     check_ctx(ctx);
     Density& d = density(ctx, handle);
-    if (kvec_n) std::memcpy(kvec_n, d.kvec.data(), d.kvec.size() * 4);
+    if (kvec_n) std::memcpy(kvec_n, d.kvec->data(), d.kvec->size() * 4);
     if (shell_offsets && !d.shell_off.empty())
       std::memcpy(shell_offsets, d.shell_off.data(), d.shell_off.size() * 4);
   });

@@ -609,6 +609,20 @@ __device__ __forceinline__ void kahan3(float (&acc)[3], float (&cmp)[3], const f
   }
 }
 
+// u[k] = the value of the shell that holds vector k, 0 outside the shells
+__global__ void shell_values_kernel(const int32_t* __restrict__ off, const float* __restrict__ value, int32_t n_shells,
+                                    int32_t n_k, float* __restrict__ u) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n_k) return;
+  int lo = -1, hi = n_shells + 1;  // off[lo] <= k < off[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (off[mid] <= k) lo = mid;
+    else hi = mid;
+  }
+  u[k] = lo >= 0 && lo < n_shells ? value[lo] : 0.f;
+}
+
 // c[f][slot(k)] = u_k conj(rho[f][k]); holes of the slot table stay zero
 __global__ void sk_coef_kernel(const float2* __restrict__ rho, int32_t n_k, int32_t n_frames,
                                const int32_t* __restrict__ slot, const float* __restrict__ u,
@@ -1111,11 +1125,25 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
       AMDAT_CUDA(cudaMemcpy(w.data(), dl_ds, (size_t)n_shells * 8, cudaMemcpyDeviceToHost));
     else
       std::memcpy(w.data(), dl_ds, (size_t)n_shells * 8);
-    std::vector<float> u(std::max(nk, 1), 0.f);
+    // (expanded on the device from the shells' values: [offsets | values])
+    std::vector<int32_t> shells(2 * (size_t)n_shells + 1, 0);
+    float max_u = 0.f;
     for (int s = 0; s < n_shells; ++s) {
       const int cnt = shell_offsets[s + 1] - shell_offsets[s];
-      for (int k = shell_offsets[s]; k < shell_offsets[s + 1]; ++k) u[k] = (float)(2.0 * w[s] / cnt);
+      const float us = cnt ? (float)(2.0 * w[s] / cnt) : 0.f;
+      max_u = std::max(max_u, std::fabs(us));
+      shells[s] = shell_offsets[s];
+      std::memcpy(&shells[(size_t)n_shells + 1 + s], &us, 4);
     }
+    shells[n_shells] = shell_offsets[n_shells];
+    const size_t sbytes = shells.size() * 4;
+    auto expand = [&](unsigned char* d_shells, unsigned char* d_u) {
+      AMDAT_CUDA(cudaMemcpyAsync(d_shells, shells.data(), sbytes, cudaMemcpyHostToDevice, ctx->stream));
+      shell_values_kernel<<<(unsigned)ceil_div(nk, 256), 256, 0, ctx->stream>>>(
+          (const int32_t*)d_shells, (const float*)d_shells + n_shells + 1, n_shells, nk, (float*)d_u);
+      check_launch("shell_values_kernel");
+      count_launch(ctx);
+    };
     if (n == 0 || nk == 0) {
       if (gbytes) {
         if (dev) AMDAT_CUDA(cudaMemsetAsync(grad, 0, gbytes, ctx->stream));
@@ -1129,14 +1157,12 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
     const char* sel = std::getenv("AMDAT_SK_ADJOINT");
     if (!d.lattice_key.empty() && tc_enabled(ctx) && !(sel && std::strcmp(sel, "columns") == 0)) {
       TcPlan* tp = lattice_tc_plan(ctx, d.lattice_key);
-      float max_u = 0.f;
-      for (int k = 0; k < nk; ++k) max_u = std::max(max_u, std::fabs(u[k]));
-      const size_t o_fr = 0, o_u = align256((size_t)F * 4), o_fx = align256(o_u + (size_t)nk * 4);
+      const size_t o_fr = 0, o_sh = align256((size_t)F * 4), o_u = align256(o_sh + sbytes), o_fx = align256(o_u + (size_t)nk * 4);
       const size_t o_g = align256(o_fx + (size_t)F * n * sizeof(int4));
       unsigned char* base = ctx->scratch.reserve(o_g + (dev ? 0 : gbytes));
       cudaStream_t st = ctx->stream;
       AMDAT_CUDA(cudaMemcpyAsync(base + o_fr, d.frames.data(), (size_t)F * 4, cudaMemcpyHostToDevice, st));
-      AMDAT_CUDA(cudaMemcpyAsync(base + o_u, u.data(), (size_t)nk * 4, cudaMemcpyHostToDevice, st));
+      expand(base + o_sh, base + o_u);
       fixed_turns_launch(ctx, (const int32_t*)(base + o_fr), F, e, d.period, (int4*)(base + o_fx));
       float* d_g = dev ? grad : (float*)(base + o_g);
       sk_adjoint_tc_run(ctx, *tp, (const int4*)(base + o_fx), n, F, d.rho->ptr, nk, (const float*)(base + o_u),
@@ -1151,15 +1177,16 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
     if (!d.lattice_key.empty()) {
       auto it = ctx->sk_adjoint_plans.find(d.lattice_key);
       if (it == ctx->sk_adjoint_plans.end())
-        it = ctx->sk_adjoint_plans.emplace(d.lattice_key, sk_adjoint_plan_build(d.kvec)).first;
+        it = ctx->sk_adjoint_plans.emplace(d.lattice_key, sk_adjoint_plan_build(*d.kvec)).first;
       A = it->second;
     } else {
-      own.reset(sk_adjoint_plan_build(d.kvec));
+      own.reset(sk_adjoint_plan_build(*d.kvec));
       A = own.get();
     }
     const int64_t n_slots = A->n_slots;
     size_t o = 0;
     const size_t o_fr = o; o = align256(o + (size_t)F * 4);
+    const size_t o_sh = o; o = align256(o + sbytes);
     const size_t o_u = o; o = align256(o + (size_t)nk * 4);
     const size_t o_fx = o; o = align256(o + (size_t)F * n * sizeof(int4));
     const size_t o_c = o; o = align256(o + (size_t)F * n_slots * sizeof(float2));
@@ -1167,7 +1194,7 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
     unsigned char* base = ctx->scratch.reserve(o);
     cudaStream_t st = ctx->stream;
     AMDAT_CUDA(cudaMemcpyAsync(base + o_fr, d.frames.data(), (size_t)F * 4, cudaMemcpyHostToDevice, st));
-    AMDAT_CUDA(cudaMemcpyAsync(base + o_u, u.data(), (size_t)nk * 4, cudaMemcpyHostToDevice, st));
+    expand(base + o_sh, base + o_u);
     float2* coef = (float2*)(base + o_c);
     if (A->columns) AMDAT_CUDA(cudaMemsetAsync(coef, 0, (size_t)F * n_slots * sizeof(float2), st));
     const int64_t tot = (int64_t)F * nk;
