@@ -98,7 +98,8 @@ struct DispParams {
   unsigned long long* gs;  // [list][gap][bin]
   int32_t n_gaps;
   int32_t n_bins;
-  float bin_size;
+  float bin_size, inv_bin;
+  float gs_lim;  // 1/2 - the bin estimate's error bound, in bins
   // F_s
   int32_t n_fs;              // shells in this pass (<= MAX_FS)
   int32_t fs_mode;           // 0 none, 1 list, 2 octant
@@ -109,6 +110,26 @@ struct DispParams {
   float period;              // L of k = 2 pi n / L
   int32_t n_rep_smem;        // F_s vectors (list) or representatives (octant) of the pass in shared memory (0: read from kv)
 };
+
+__device__ __noinline__ int gs_exact_bin(float s2, float bin_size) {
+  return (int)__fdiv_rn(__fsqrt_rn(s2), bin_size);
+}
+
+// Counts a displacement into its G_s bin, the reference's FP32 chain
+// sqrt((dx*dx + dy*dy) + dz*dz) / bin_size.  The bin is estimated from the approximate
+// root, x = sqrt * inv_bin - 1/2 rounded to an integer by adding 1.5 * 2^23; an estimate
+// within its error bound of the bin's edges (|r| near 1/2), and anything not finite, takes
+// the chain itself.
+__device__ __forceinline__ void gs_count(const DispParams& p, unsigned int* hist, float dx, float dy, float dz) {
+  constexpr float magic = 12582912.0f;
+  const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+  float root;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(root) : "f"(s2));
+  const float x = fmaf(root, p.inv_bin, -0.5f), y = __fadd_rn(x, magic);
+  int b = (int)(__float_as_uint(y) - 0x4b400000u);
+  if (!(fabsf(__fsub_rn(x, __fsub_rn(y, magic))) < p.gs_lim)) b = gs_exact_bin(s2, p.bin_size);
+  if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
+}
 
 // octant mode: the compensated sum over one shell's representatives (blocks of
 // 32 terms, each block added to the sum), reading the representatives from
@@ -279,12 +300,7 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
         const float e = sq3(dx, dy, dz);
         kadd(m2, e);
         kadd(m4, e * e);
-        if (GS) {
-          // the reference's FP32 chain: sqrt((dx*dx + dy*dy) + dz*dz) / bin_size
-          const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-          const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-          if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
-        }
+        if (GS) gs_count(p, hist, dx, dy, dz);
       };
       const int lo = L.first + it.a0, hi = L.first + it.a1;
       const int v0 = (lo + 3) >> 2, v1 = hi >> 2;  // whole quads [v0, v1)
@@ -391,11 +407,7 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
             kadd(m2, d2);
             kadd(m4, d2 * d2);
           }
-          if (GS && k < n_at) {
-            const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-            const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-            if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
-          }
+          if (GS && k < n_at) gs_count(p, hist, dx, dy, dz);
         }
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax)
@@ -420,12 +432,7 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
         kadd(m2, d2);
         kadd(m4, d2 * d2);
       }
-      if (GS) {
-        // the reference's FP32 chain: sqrt((dx*dx + dy*dy) + dz*dz) / bin_size
-        const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-        const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
-        if (b >= 0 && b < p.n_bins) atomicAdd(hist + b, 1u);
-      }
+      if (GS) gs_count(p, hist, dx, dy, dz);
       if (MODE == 1) {
         const int32_t fx = turns_fixed(dx, p.period);
         const int32_t fy = turns_fixed(dy, p.period);
@@ -1300,6 +1307,10 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
     p.n_gaps = pl.G;
     p.n_bins = pass == 0 ? pl.NB : 0;
     p.bin_size = pl.NB ? pl.bin_max / (float)pl.NB : 1.0f;
+    p.inv_bin = 1.0f / p.bin_size;
+    // the estimate's error, in roundings of 2^-24 of the bin number: the approximate root 2,
+    // the chain's root and quotient 1 each, the reciprocal and the product 1 each
+    p.gs_lim = 0.5f - 6.0f * 5.9604645e-8f * (float)(pl.NB + 1) - 1e-6f;
     p.n_fs = nfs;
     p.fs_mode = pl.S ? pl.sh.mode : 0;
     p.kv = (const int4*)(base + pl.o_kv);
