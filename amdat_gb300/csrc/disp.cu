@@ -45,7 +45,7 @@
 
 namespace amdat {
 
-constexpr int DISP_CHUNK = 4096;  // list members per item
+constexpr int DISP_CHUNK = 4096;  // list members per item (moments and G_s up to four times as many)
 constexpr int MAX_FS = 8;         // shells per pass
 constexpr int DISP_THREADS = 256;
 constexpr int FS_THREADS = 128;
@@ -1645,13 +1645,32 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     }
     if (pl->S == 0 && pl->NB == 0 && !pl->bulk && pl->n_units > 1 && pl->n_units <= SLAB_UNITS && P.n_pairs > 0)
       plan_slabs(ctx, *pl, P);
-    // default tile: full chunks stream memory; F_s or few pairs want smaller
-    // chunks to keep every SM busy
-    const int64_t want_items = (int64_t)ctx->n_sm * 16;
+    // Default tile.  Every item ends with a block reduction, so moments take chunks of up
+    // to 16,384 members while that leaves ten items per SM and the chunk's atoms in all
+    // frames fit half the L2 (its pairs run one after the other).  4,096 / 16,384 members,
+    // moments and with 200 G_s bins: 64,000 atoms x 1,226 pairs 123 / 95, 214 / 169 us;
+    // 500,000 x 1,226 957 / 676, 1,558 / 1,072; 200,000 x 427 176 / 150, 298 / 257; a third
+    // of those 200,000 atoms, gathered (196 MB of sectors), 155 / 152, 214 / 232.  32,000
+    // atoms x 187 pairs in 2,460 / 4,096 / 8,192 25 / 20 / 23, 42 / 36 / 42.
+    // F_s is compute bound and keeps smaller chunks.
     int64_t chunk = DISP_CHUNK;
-    if (P.n_pairs > 0 && unit_atoms > 0)
-      chunk = std::max<int64_t>(pl->S ? 128 : 1024,
-                                std::min<int64_t>(DISP_CHUNK, ceil_div(unit_atoms * P.n_pairs, want_items)));
+    if (P.n_pairs > 0 && unit_atoms > 0) {
+      if (pl->S || pl->bulk) {
+        const int64_t want_items = (int64_t)ctx->n_sm * 16;
+        chunk = std::max<int64_t>(pl->S ? 128 : 1024,
+                                  std::min<int64_t>(DISP_CHUNK, ceil_div(unit_atoms * P.n_pairs, want_items)));
+      } else {
+        int64_t span = 0;  // atoms that the units are spread over
+        for (const ListDev& u : pl->udev) span += u.idx ? ctx->n_atoms : u.n;
+        const int64_t in_l2 = (int64_t)(64 << 20) / ((int64_t)ctx->n_frames * 12) * unit_atoms / std::max<int64_t>(span, 1);
+        const int64_t top = std::min<int64_t>(4 * DISP_CHUNK, std::max<int64_t>(DISP_CHUNK, in_l2));
+        const int64_t want_items = (int64_t)ctx->n_sm * 10;
+        // whole rounds of the block's 16-byte loads (6,474 atoms x 289 pairs: 1,079-atom items
+        // 19.1 us, 1,024 18.3, 1,618 16.3)
+        chunk = std::max<int64_t>(1, std::min(top, ceil_div(unit_atoms * P.n_pairs, want_items)));
+        chunk = ceil_div(chunk, 1024) * 1024;
+      }
+    }
     if (pl->slab) chunk = SLAB_ENTRIES;  // its one tile
     // list-mode F_s holds few registers and only its vectors in shared memory:
     // more resident blocks hide the latency of its cosine chain
@@ -1671,7 +1690,7 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       // MSD-only streams memory (large chunks, more resident blocks)
       const std::vector<int> chunks = pl->slab ? std::vector<int>{SLAB_ENTRIES}
                                       : pl->S ? std::vector<int>{256, 512, 1024, 2048}
-                                            : std::vector<int>{1024, 2048, 4096, 8192};
+                                            : std::vector<int>{1024, 2048, 4096, 8192, 16384};
       const std::vector<int> bpss = pl->slab ? std::vector<int>{bps}
                                     : pl->S ? (pl->sh.mode == 1 ? std::vector<int>{4, 8, 16} : std::vector<int>{2, 4, 8})
                                           : std::vector<int>{4, 8};
