@@ -194,6 +194,7 @@ amdat_ctx::~amdat_ctx() {
   }
   for (auto* b : rho_pool) delete b;
   for (auto& kv : bin_maps) delete kv.second;
+  if (result) cudaFreeHost(result);
   amdat::lattice_plans_free(this);
   amdat::sk_adjoint_plans_free(this);
   for (auto& r : prof_pending) {
@@ -321,6 +322,10 @@ amdat_status amdat_create(int32_t device, amdat_ctx** out) {
       AMDAT_CUDA(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
       c->stream = c->own_stream;
       c->lists.push_back(new ListEntry());
+      if (cudaMallocHost((void**)&c->result, amdat_ctx::RESULT_BYTES) != cudaSuccess) {
+        cudaGetLastError();
+        c->result = nullptr;
+      }
     } catch (...) {
       delete c;
       throw;

@@ -1772,10 +1772,27 @@ static void plan_read(amdat_ctx* ctx, amdat_disp_plan* pl, int32_t out_flags, do
   AMDAT_REQUIRE(out_flags == AMDAT_OUT_HOST || out_flags == AMDAT_OUT_DEVICE, "bad out_flags");
   const size_t n_lg = (size_t)pl->n_lists * pl->G;
   unsigned char* base = pl->dev.ptr;
-  to_out(ctx, sum_d2, (const double*)(base + pl->o_d2), n_lg, out_flags);
-  to_out(ctx, sum_d4, (const double*)(base + pl->o_d4), n_lg, out_flags);
-  if (pl->S) to_out(ctx, fs_sum, (const double*)(base + pl->o_fs), n_lg * pl->S, out_flags);
-  if (pl->NB) to_out(ctx, (unsigned long long*)gs_counts, (const unsigned long long*)(base + pl->o_gs), n_lg * pl->NB, out_flags);
+  // results to host arrays: one copy of all outputs (they lie one after the other) into
+  // pinned memory while they fit it, instead of a pageable copy with its own wait for each
+  // (500 atoms: 47 -> 39 us a call)
+  const size_t fs_bytes = pl->S ? n_lg * pl->S * 8 : 0, gs_bytes = pl->NB ? n_lg * pl->NB * 8 : 0;
+  const size_t end = gs_bytes ? pl->o_gs + gs_bytes : (fs_bytes ? pl->o_fs + fs_bytes : pl->o_d4 + n_lg * 8);
+  if (out_flags == AMDAT_OUT_HOST && ctx->result && end - pl->o_d2 <= amdat_ctx::RESULT_BYTES) {
+    AMDAT_CUDA(cudaMemcpyAsync(ctx->result, base + pl->o_d2, end - pl->o_d2, cudaMemcpyDeviceToHost, ctx->stream));
+    AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
+    auto take = [&](void* dst, size_t from, size_t n) {
+      if (dst && n) std::memcpy(dst, ctx->result + (from - pl->o_d2), n);
+    };
+    take(sum_d2, pl->o_d2, n_lg * 8);
+    take(sum_d4, pl->o_d4, n_lg * 8);
+    take(fs_sum, pl->o_fs, fs_bytes);
+    take(gs_counts, pl->o_gs, gs_bytes);
+  } else {
+    to_out(ctx, sum_d2, (const double*)(base + pl->o_d2), n_lg, out_flags);
+    to_out(ctx, sum_d4, (const double*)(base + pl->o_d4), n_lg, out_flags);
+    if (pl->S) to_out(ctx, fs_sum, (const double*)(base + pl->o_fs), n_lg * pl->S, out_flags);
+    if (pl->NB) to_out(ctx, (unsigned long long*)gs_counts, (const unsigned long long*)(base + pl->o_gs), n_lg * pl->NB, out_flags);
+  }
   if (atom_pairs) {
     if (out_flags == AMDAT_OUT_DEVICE)
       AMDAT_CUDA(cudaMemcpyAsync(atom_pairs, pl->pairs.data(), n_lg * 8, cudaMemcpyHostToDevice, ctx->stream));

@@ -179,6 +179,8 @@ struct amdat_ctx {
   amdat::DevBuf<unsigned char> scratch;
   amdat::DevBuf<unsigned char> scratch2;
   amdat::DevBuf<unsigned char> staging;
+  static constexpr size_t RESULT_BYTES = 256 << 10;
+  unsigned char* result = nullptr;  // pinned, RESULT_BYTES: results on their way to host arrays (null: none to be had)
   std::vector<amdat::DevBuf<float2>*> rho_pool;        // released density tables
   std::map<std::string, amdat::LatticePlanDev*> lattice_plans;
   std::map<std::string, amdat::SkAdjointPlan*> sk_adjoint_plans;  // by lattice key
