@@ -39,6 +39,32 @@ __device__ __forceinline__ void ksadd(KSumF& k, float v) {
   k.s = t;
 }
 
+// Sums of NV values over groups of KT lanes, each in the order of a shuffle tree (lane l
+// adds lane l + KT/2, then + KT/4, ...): at each of the first steps half of the lanes take
+// one half of the values and the others the other half, so NV trees cost NV - 1 additions
+// of a warp and then one per step, not NV per step: FP64 additions, at a small fraction of
+// the FP32 rate, bound the correlator of few frames (20 frames, 80,000 tiles: 925 us with a
+// tree per gap, 565 with four gaps per tree).
+// The sum of value v ends in lane (v's bits from the top) of the group, returned as `slot`.
+template <int KT, int NV>
+__device__ __forceinline__ double fold(double (&v)[NV], int lane, int* slot) {
+  int off = KT / 2, base = 0;
+#pragma unroll
+  for (int h = NV / 2; h >= 1; h /= 2) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+    base += up ? h : 0;
+    off /= 2;
+  }
+  for (; off > 0; off /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+  *slot = base;
+  return v[0];
+}
+
 template <int KT>
 __global__ void __launch_bounds__(256)
     isf_pairs_kernel(const float2* __restrict__ rho1, const float2* __restrict__ rho2,
@@ -62,19 +88,25 @@ __global__ void __launch_bounds__(256)
   const int grp = threadIdx.x / KT, n_grp = blockDim.x / KT;
   // the loop bound is uniform across the block, so every lane of a warp
   // reaches each shuffle together even when several groups share a warp
-  for (int gb = 0; gb < n_gaps; gb += n_grp) {
-    const int g = gb + grp;
-    KSumF acc = {0.f, 0.f};
-    if (g < n_gaps) {
-      for (int p = gap_first[g]; p < gap_first[g + 1]; ++p) {
-        const float2 a = s1[t0[p] * KT + kk], b = s2[t1[p] * KT + kk];
-        ksadd(acc, fmaf(a.x, b.x, a.y * b.y));
-      }
-    }
-    double v = (double)acc.s - (double)acc.c;
+  constexpr int NV = KT < 4 ? KT : 4;  // gaps folded together
+  for (int gb = 0; gb < n_gaps; gb += NV * n_grp) {
+    double v[NV];
 #pragma unroll
-    for (int off = KT / 2; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off, KT);
-    if (kk == 0 && g < n_gaps) part[(int64_t)blockIdx.x * n_gaps + g] = v;
+    for (int j = 0; j < NV; ++j) {
+      const int g = gb + j * n_grp + grp;
+      KSumF acc = {0.f, 0.f};
+      if (g < n_gaps) {
+        for (int p = gap_first[g]; p < gap_first[g + 1]; ++p) {
+          const float2 a = s1[t0[p] * KT + kk], b = s2[t1[p] * KT + kk];
+          ksadd(acc, fmaf(a.x, b.x, a.y * b.y));
+        }
+      }
+      v[j] = (double)acc.s - (double)acc.c;
+    }
+    int j;
+    const double sum = fold<KT, NV>(v, kk, &j);
+    const int g = gb + j * n_grp + grp;
+    if (kk % (KT / NV) == 0 && g < n_gaps) part[(int64_t)blockIdx.x * n_gaps + g] = sum;
   }
 }
 
@@ -159,16 +191,21 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// the tiles of each (column, shell) summed by a warp: lanes stride over the tiles, then a
+// shuffle tree (200 shells of 80,000 tiles x 20 columns: 18 us; a thread per sum, waiting for
+// each addition, 190)
 __global__ void tile_finalize_kernel(const double* __restrict__ part, int32_t n_cols,
                                      const int32_t* __restrict__ shell_tile_first,
                                      const float* __restrict__ inv_count, int32_t n_shells,
                                      double* __restrict__ out /* [col][shell] */) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (i >= (int64_t)n_shells * n_cols) return;
-  const int s = (int)(i % n_shells), col = (int)(i / n_shells);
+  const int s = (int)(i / n_cols), col = (int)(i % n_cols);
   double acc = 0.0;
-  for (int t = shell_tile_first[s]; t < shell_tile_first[s + 1]; ++t) acc += part[(int64_t)t * n_cols + col];
-  out[(int64_t)col * n_shells + s] = acc * (double)inv_count[s];
+  for (int t = shell_tile_first[s] + lane; t < shell_tile_first[s + 1]; t += 32) acc += part[(int64_t)t * n_cols + col];
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+  if (lane == 0) out[(int64_t)col * n_shells + s] = acc * (double)inv_count[s];
 }
 
 __global__ void __launch_bounds__(256)
@@ -304,7 +341,7 @@ amdat_status amdat_isf_run(amdat_ctx* ctx, int32_t h1, int32_t h2, int32_t fullb
       AMDAT_CUDA(cudaMemsetAsync(part, 0, G * 8, ctx->stream));
     }
     const int64_t n_out = (int64_t)G * n_shells;
-    tile_finalize_kernel<<<(unsigned)ceil_div(n_out, 256), 256, 0, ctx->stream>>>(
+    tile_finalize_kernel<<<(unsigned)ceil_div(n_out, 8), 256, 0, ctx->stream>>>(
         part, G, (const int32_t*)(base + o_stf), (const float*)(base + o_inv), n_shells, out);
     check_launch("tile_finalize_kernel");
     count_launch(ctx);
@@ -355,7 +392,7 @@ amdat_status amdat_structure_factor_run(amdat_ctx* ctx, int32_t h1, int32_t h2,
       check_launch("sk_frames_kernel");
       count_launch(ctx);
     }
-    tile_finalize_kernel<<<(unsigned)ceil_div(n_shells, 256), 256, 0, ctx->stream>>>(
+    tile_finalize_kernel<<<(unsigned)ceil_div(n_shells, 8), 256, 0, ctx->stream>>>(
         part, 1, (const int32_t*)(base + o_stf), (const float*)(base + o_inv), n_shells, out);
     check_launch("tile_finalize_kernel");
     count_launch(ctx);
