@@ -158,10 +158,18 @@ __device__ __forceinline__ void octant_shell_sum2(const uint2* R, const uint64_t
                                                   KSum& acc_b) {
   acc_a = KSum{0.f, 0.f};
   acc_b = KSum{0.f, 0.f};
+  // the representatives run through y and z of one x after the other (225 -> 217 us with
+  // x's cosines kept, at 4,000 atoms x 316 pairs of 281 representatives)
+  uint32_t x_at = ~0u;
+  uint64_t tx = 0ull;
   auto term = [&](int v, uint64_t& blk) {
     const uint2 r = R[v];
     const float w = __uint_as_float(r.y & 0xffff0000u);
-    blk = fma2(mul2(mul2(pk2(w, w), T[r.x & 0xffffu]), T[r.x >> 16]), T[r.y & 0xffffu], blk);
+    if ((r.x & 0xffffu) != x_at) {
+      x_at = r.x & 0xffffu;
+      tx = T[x_at];
+    }
+    blk = fma2(mul2(mul2(pk2(w, w), tx), T[r.x >> 16]), T[r.y & 0xffffu], blk);
   };
   auto close = [&](uint64_t blk) {
     float ba, bb;
@@ -191,8 +199,8 @@ __device__ __forceinline__ void octant_shell_sum2(const uint2* R, const uint64_t
 // MODE: 0 moments, 1 F_s by vector list, 2 F_s by octants, 3 by octants with two atoms
 // per thread.  Octants are bound by the loads of a representative and its three cosines
 // from shared memory; with two atoms per thread one 8-byte representative and three
-// 8-byte pairs serve both, and the products run packed (4,000 atoms x 1,100 pairs of 281
-// representatives: 280 -> 221 us).
+// 8-byte pairs serve both, and the products run packed (4,000 atoms x 316 pairs of 281
+// representatives: 280 -> 217 us).
 template <int MODE, bool GS>
 __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
     disp_mixed_kernel(DispParams p) {
@@ -1323,8 +1331,8 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
     const int threads = mode ? FS_THREADS : DISP_THREADS;
     size_t shm = gs ? (size_t)((pl.NB + 3) & ~3) * 4 : 0;
     const int n_rep_pass = mode ? pl.sh.off[s0 + nfs] - pl.sh.off[s0] : 0;
-    // Octants, two atoms per thread: 4,000 atoms x 1,100 pairs, shells around q = 7.1 with
-    // components up to 11 / 19 / 22 / 29 / 34 / 45 take 95 / 227 / 350 / 757 / 1,711 / 3,707 us
+    // Octants, two atoms per thread: 4,000 atoms x 316 pairs, shells around q = 7.1 with
+    // components up to 11 / 19 / 22 / 29 / 34 / 45 take 95 / 217 / 331 / 729 / 1,712 / 3,725 us
     // (one atom: 121 / 283 / 466 / 950 / 1,777 / 7,601), so wherever the tables fit a block.
     // A step of two atoms costs 1.3 to 1.6 steps of one: items of at most a block of
     // atoms stay with one atom (100 atoms 30 us, 38 with two; 1,000 atoms in items of
