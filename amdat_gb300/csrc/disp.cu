@@ -53,6 +53,8 @@ constexpr int MAX_PAIRS_PER_ITEM = 64;
 constexpr int SLAB_BATCH = 4;                             // entries per thread
 constexpr int SLAB_ENTRIES = SLAB_BATCH * DISP_THREADS;   // members of all units per item (slab route)
 constexpr int SLAB_UNITS = 128;
+constexpr double SLAB_MEAN = 8192.0;  // mean list size, weighted by members
+constexpr int SLAB_PAIRS = 32;
 constexpr int64_t SLAB_ROWS = 16 << 20;  // rows of partials (16 bytes each)
 constexpr size_t DISP_CACHE_PLANS = 8;  // one-shot requests kept prepared
 
@@ -1536,15 +1538,22 @@ static void plan_classes(amdat_ctx* ctx, amdat_disp_plan& pl, const int32_t* lis
   pl.lu_off[L] = (int32_t)pl.lu_units.size();
 }
 
+// the size of a member's list (unit), averaged over members
+static double mean_size(const std::vector<int32_t>& sizes) {
+  double members = 0.0, squares = 0.0;
+  for (int32_t m : sizes) members += m, squares += (double)m * m;
+  return members > 0.0 ? squares / members : 0.0;
+}
+
 // The slab route of MSD + NGP moments over several units, taken where it reads less than
 // the units one by one.  The units' kernel reads contiguous members at 0.75 of the slab
 // kernel's time per member, gathered ones at 0.55 of it per atom of the range that they
 // are scattered over (whole 32-byte sectors, whichever atoms of them are members; 0.65 for
 // 2 units, 0.47 for 9).
 // 200,000 atoms, 427 pairs, units one by one / slabs: 2 random types 314 / 248 us, 3
-// interleaved 413 / 246, 9 random 1,063 / 259, 100 random 3,519 / 295; 8 random types in
-// half the atoms, the others contiguous 564 / 264; 2 in a quarter of them 215 / 247; 2
-// contiguous 178.  64 nested lists of up to 50,000: 579 / 160.
+// interleaved 413 / 246, 9 random 1,063 / 259; 8 random types in half the atoms, the others
+// contiguous 564 / 264; 2 in a quarter of them 215 / 247; 2 contiguous 178.  64 nested lists
+// of up to 50,000: 579 / 160.
 // Entry tables: the members of all units in atom order (an atom of several units once for
 // each), cut into slabs of at most SLAB_ENTRIES; per entry its place in the slab's unit
 // order, per slab the units' runs there.
@@ -1571,6 +1580,11 @@ static void plan_slabs(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P) 
   const int64_t slabs = ceil_div(n, SLAB_ENTRIES);
   const int64_t rows = n ? pl.n_units * slabs * (pl.G + P.n_pairs / slab_pairs(ctx, P.n_pairs, slabs)) : 0;
   if (by_unit <= (double)n || rows > SLAB_ROWS) return;
+  // Small lists and few pairs stay with the units' kernel: its sums are not error-free
+  // (each thread adds its terms by Kahan's scheme, a few in no order of size), and there
+  // the slabs' exact sums differ from them by up to 2e-9, from these sizes on by less
+  // than 6e-10.
+  if (P.n_pairs < SLAB_PAIRS || mean_size(pl.lsize) < SLAB_MEAN) return;
   for (int u = 0; u < pl.n_units; ++u)
     for (int32_t a : idx[u]) ++at[a + 1];
   for (int64_t a = 0; a < N; ++a) at[a + 1] += at[a];
@@ -1660,10 +1674,11 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     // 500,000 x 1,226 957 / 676, 1,558 / 1,072; 200,000 x 427 176 / 150, 298 / 257; a third
     // of those 200,000 atoms, gathered (196 MB of sectors), 155 / 152, 214 / 232.  32,000
     // atoms x 187 pairs in 2,460 / 4,096 / 8,192 25 / 20 / 23, 42 / 36 / 42.
-    // F_s is compute bound and keeps smaller chunks.
+    // F_s is compute bound and keeps smaller chunks; so do several small units, whose sums
+    // of a few terms per thread depend on the items' cut.
     int64_t chunk = DISP_CHUNK;
     if (P.n_pairs > 0 && unit_atoms > 0) {
-      if (pl->S || pl->bulk) {
+      if (pl->S || pl->bulk || (pl->n_units > 1 && mean_size(pl->usize) < SLAB_MEAN)) {
         const int64_t want_items = (int64_t)ctx->n_sm * 16;
         chunk = std::max<int64_t>(pl->S ? 128 : 1024,
                                   std::min<int64_t>(DISP_CHUNK, ceil_div(unit_atoms * P.n_pairs, want_items)));

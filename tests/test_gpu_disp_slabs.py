@@ -2,8 +2,9 @@
 sums equal the exact sums of the FP32 terms to 1e-9 (the kernel's additions are
 error-free but for the last bits of their corrections) and the oracle's to 1e-6, over
 slab edges, unit counts on both sides of the
-lane groups' rule and up to the route's limit, empty lists, contiguous
-units among gathered ones and repeated atoms across lists."""
+lane groups' rule and up to the route's limit, units of one atom and up, empty lists,
+contiguous units among gathered ones and repeated atoms across lists.  A list of all
+atoms brings the lists' mean size over the route's lower limit."""
 import numpy as np
 import pytest
 
@@ -13,15 +14,19 @@ from oracle import oracle as orc
 pytestmark = pytest.mark.gpu
 
 
-def _sets(kind, n, rng):
-    perm = rng.permutation(n)
+def _sets(kind, n, m, rng):
+    """Lists over m scattered atoms, then the list of all n."""
+    some = np.sort(rng.permutation(n)[:m])
+    perm = rng.permutation(some)
     if kind.startswith("types"):
-        return [np.sort(x) for x in np.array_split(perm, int(kind[5:]))]
-    if kind == "nested":
-        return [np.sort(perm[:m]) for m in (1, 3, n // 9, n // 3, n)]
-    if kind == "mixed":
-        return [np.arange(n // 2), np.zeros(0, int)] + [n // 2 + np.arange(i, n - n // 2, 7) for i in range(7)]
-    return [np.sort(rng.choice(n, n // 2, replace=False)) for _ in range(9)]  # overlapping
+        out = [np.sort(x) for x in np.array_split(perm, int(kind[5:]))]
+    elif kind == "nested":
+        out = [np.sort(perm[:k]) for k in (1, 3, m // 9 + 1, m // 3 + 1, m)]
+    elif kind == "mixed":
+        out = [np.arange(m), np.zeros(0, int)] + [m + np.arange(i, n - m, 7) for i in range(6)]
+    else:  # overlapping
+        out = [np.sort(rng.choice(some, m // 2 + 1, replace=False)) for _ in range(9)]
+    return out + [np.arange(n)]
 
 
 def _exact(scheme, u, fb, members):
@@ -41,14 +46,14 @@ def _exact(scheme, u, fb, members):
     return out
 
 
-@pytest.mark.parametrize("n", [5, 127, 1023, 1024, 1025, 3000])
-@pytest.mark.parametrize("kind", ["types2", "types16", "types17", "types128", "nested", "mixed", "overlap"])
-def test_slabs_match_exact_sums(eng, n, kind):
-    scheme = synth.TimeScheme.exponential(3, 7, 1.4, 0, 0, 0.005)
+@pytest.mark.parametrize("n,m", [(16383, 5), (16384, 127), (16385, 1023), (16900, 1500)])
+@pytest.mark.parametrize("kind", ["types2", "types15", "types16", "types127", "nested", "mixed", "overlap"])
+def test_slabs_match_exact_sums(eng, n, m, kind):
+    scheme = synth.TimeScheme.exponential(4, 8, 1.4, 0, 0, 0.005)
     traj = synth.random_walk(n, 15.0, scheme, 0.5, seed=n)
     eng.upload(traj.unwrapped, traj.box)
     eng.set_scheme(scheme)
-    sets = _sets(kind, n, np.random.default_rng(n))
+    sets = _sets(kind, n, m, np.random.default_rng(n))
     handles = [eng.list(s.astype(np.int32)) for s in sets]
     for flags, fb in ((0, 0), (2, 1)):  # plain and replayed as a graph; default and full-block pairs
         plan = eng.plan(handles, flags=flags, fullblock=fb)
