@@ -40,10 +40,10 @@ PEAKS_FILE = os.path.join(HERE, "MEASURED_PEAKS.json")
 FP32_LANES_PER_SM = 128
 # DRAM bytes (read + write) per frame of one rhok_tc_kernel launch on the headline
 # lattice (N=32000, |k|<=20, L=33.6), from one ncu capture of a 2-frame launch of
-# this kernel (941.9 MB read + 42.7 MB written).  Every stream of the launch is per
+# this kernel (898.6 MB read + 50.8 MB written).  Every stream of the launch is per
 # frame (X/Y phase tables, Z operands, rho rows), so a launch over f frames moves f
 # times this.
-TC_DRAM_BYTES_PER_FRAME = (941.943e6 + 42.651e6) / 2
+TC_DRAM_BYTES_PER_FRAME = (898.555e6 + 50.796e6) / 2
 # DRAM bytes (read + write) of one launch of the per-list MSD + NGP plan over the 64
 # nested lists, from one ncu capture of disp_mixed_kernel on that workload
 PERLIST_DRAM_BYTES = 2.33e9
@@ -989,7 +989,7 @@ def main():
                                gd_rate=npairs_gd * n * (n - 1) / gd_s, gd_ms=1e3 * gd_s,
                                gd_kernel_ms=ms_gd, gd_pairs=npairs_gd, rdf_total=int(counts.sum()),
                                gd_all_ms=1e3 * gd_all_s, gd_all_kernel_ms=ms_gd_all, gd_same=gd_same,
-                               gd_cells=int(math.floor(42.3 / (5.0 * (1 + 1e-4)))) ** 3)
+                               gd_total=int(gd_counts.sum()))
 
     if args.only in ("", "structure"):
         result["structure"] = structure_bench(torch, stream, local, args)
@@ -1213,9 +1213,7 @@ def main():
         fp32_peak = 2 * FP32_LANES_PER_SM * sm_count * float(peaks.get("sm_max_mhz", 2070.0)) * 1e6 / 1e12
         n = 64000.0
         rdf_fl = 10.0 * q["frames"] * n * (n - 1) / 2 / (q["rdf_kernel_ms"] / 1e3) / 1e12
-        # the cell pass visits each atom's 27 neighbour cells: ~27 / cells of the pairs
-        gd_visited = q["gd_pairs"] * n * n * 27.0 / q["gd_cells"]
-        gd_fl = 10.0 * gd_visited / (q["gd_kernel_ms"] / 1e3) / 1e12
+        gd_fl = 10.0 * q["gd_total"] / (q["gd_kernel_ms"] / 1e3) / 1e12
         gd_all_fl = 10.0 * q["gd_pairs"] * n * (n - 1) / (q["gd_all_kernel_ms"] / 1e3) / 1e12
         pair_rule = ("algorithmic: 10 FP32 flops per visited pair (3 differences, 3 minimum-image "
                      "corrections, 3 multiply-adds of |r|^2, 1 bin division); peak = FP32 FMA peak "
@@ -1235,9 +1233,8 @@ def main():
                     "unit_rule": "every ordered pair of every time pair (the reference's loop), per second",
                     "roofline": {"bound": "fp32", "achieved": gd_fl, "peak": fp32_peak, "unit": "TFLOP/s",
                                  "frac": gd_fl / fp32_peak, "kernel": "pair_hist_cells_kernel",
-                                 "rule": pair_rule + f"; visited pairs = time pairs x N^2 x 27 / "
-                                                     f"{q['gd_cells']} cells (each atom's 27 neighbour "
-                                                     f"cells of width >= 5.0)"},
+                                 "rule": pair_rule + "; pairs = those within the last bin (counted), which "
+                                                     "a pass over cells cannot leave out"},
                     "all_pairs": {"ms_per_step": q["gd_all_ms"], "kernel_ms": q["gd_all_kernel_ms"],
                                   "counts_equal": q["gd_same"],
                                   "roofline_frac": gd_all_fl / fp32_peak,
