@@ -28,6 +28,12 @@ void check_launch(const char* what) {
     throw Error(AMDAT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+void upload_tables(amdat_ctx* ctx, std::initializer_list<TableCopy> tables) {
+  for (const TableCopy& t : tables)
+    if (t.bytes) AMDAT_CUDA(cudaMemcpyAsync(t.dst, t.src, t.bytes, cudaMemcpyHostToDevice, ctx->stream));
+  AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
+}
+
 amdat_ctx* check_ctx(amdat_ctx* ctx) {
   if (!ctx) throw Error(AMDAT_ERR_ARGUMENT, "null context");
   AMDAT_CUDA(cudaSetDevice(ctx->device));
@@ -72,9 +78,7 @@ const PairTable& pair_table(amdat_ctx* ctx, bool fullblock, bool loop_order) {
   t->h_t0 = p.t0;
   t->h_t1 = p.t1;
   t->h_gap = p.gap;
-  AMDAT_CUDA(cudaMemcpy(t->t0.ptr, p.t0.data(), n * 4, cudaMemcpyHostToDevice));
-  AMDAT_CUDA(cudaMemcpy(t->t1.ptr, p.t1.data(), n * 4, cudaMemcpyHostToDevice));
-  AMDAT_CUDA(cudaMemcpy(t->gap.ptr, p.gap.data(), n * 4, cudaMemcpyHostToDevice));
+  upload_tables(ctx, {{t->t0.ptr, p.t0.data(), n * 4}, {t->t1.ptr, p.t1.data(), n * 4}, {t->gap.ptr, p.gap.data(), n * 4}});
   ctx->pair_cache[key] = t;
   return *t;
 }
@@ -405,7 +409,7 @@ amdat_status amdat_list_create(amdat_ctx* ctx, const int32_t* atoms, int32_t n, 
     e->first = n ? atoms[0] : 0;
     if (!e->contiguous) {
       e->idx.reserve(n);
-      AMDAT_CUDA(cudaMemcpy(e->idx.ptr, atoms, sizeof(int32_t) * n, cudaMemcpyHostToDevice));
+      upload_tables(ctx, {{e->idx.ptr, atoms, sizeof(int32_t) * n}});
     }
     ctx->lists.push_back(e);
     *handle = (int32_t)ctx->lists.size() - 1;

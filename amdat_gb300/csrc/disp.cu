@@ -1518,7 +1518,7 @@ static void plan_classes(amdat_ctx* ctx, amdat_disp_plan& pl, const int32_t* lis
   pl.usize.assign(n_cls, 0);
   pl.udev.assign(n_cls, ListDev{0, 0, nullptr});
   pl.class_idx.reserve(std::max<size_t>(members.size(), 1));
-  AMDAT_CUDA(cudaMemcpy(pl.class_idx.ptr, members.data(), members.size() * 4, cudaMemcpyHostToDevice));
+  upload_tables(ctx, {{pl.class_idx.ptr, members.data(), members.size() * 4}});
   std::vector<std::vector<int32_t>> per_list(L);
   for (int c = 0; c < n_cls; ++c) {
     const int32_t b = start[c], e = start[c + 1];
@@ -1609,9 +1609,8 @@ static void plan_slabs(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P) 
   pl.o_place = (size_t)n * 4;
   pl.o_run = pl.o_place + (size_t)n * 2;
   unsigned char* base = pl.slab_dev.reserve(pl.o_run + run.size() * 2);
-  AMDAT_CUDA(cudaMemcpy(base, atoms.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
-  AMDAT_CUDA(cudaMemcpy(base + pl.o_place, place.data(), (size_t)n * 2, cudaMemcpyHostToDevice));
-  AMDAT_CUDA(cudaMemcpy(base + pl.o_run, run.data(), run.size() * 2, cudaMemcpyHostToDevice));
+  upload_tables(ctx, {{base, atoms.data(), (size_t)n * 4}, {base + pl.o_place, place.data(), (size_t)n * 2},
+                      {base + pl.o_run, run.data(), run.size() * 2}});
   pl.slab = true;
 }
 

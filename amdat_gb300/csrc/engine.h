@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <stdexcept>
@@ -199,6 +200,16 @@ const PairTable& pair_table(amdat_ctx* ctx, bool fullblock, bool loop_order);
 const ListEntry& list_entry(amdat_ctx* ctx, int32_t handle);
 Density& density(amdat_ctx* ctx, int32_t handle);
 void ensure_fp64(amdat_ctx* ctx);
+// Host tables to the device, complete on return.  They are copied on the context's
+// stream: a cudaMemcpy is ordered with the legacy stream, which the context's
+// (non-blocking) stream does not wait for, and from pageable memory it may return before
+// the data has arrived.
+struct TableCopy {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+void upload_tables(amdat_ctx* ctx, std::initializer_list<TableCopy> tables);
 void count_launch(amdat_ctx* ctx, int n = 1);
 void check_launch(const char* what);
 DevBuf<float2>* rho_acquire(amdat_ctx* ctx, size_t count);

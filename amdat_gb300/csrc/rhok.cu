@@ -601,7 +601,7 @@ void lattice_plans_free(amdat_ctx* ctx) {
 TcPlan* lattice_tc_plan(amdat_ctx* ctx, const std::string& lattice_key) {
   auto it = ctx->lattice_plans.find(lattice_key);
   AMDAT_REQUIRE(it != ctx->lattice_plans.end(), "lattice plan not found");
-  if (!it->second->tc) it->second->tc = tc_plan_build(*it->second->kvec);
+  if (!it->second->tc) it->second->tc = tc_plan_build(ctx, *it->second->kvec);
   return it->second->tc;
 }
 
@@ -732,8 +732,8 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
       pd->n_tiles = (int32_t)P.tiles.size();
       pd->tiles.reserve(P.tiles.size());
       pd->entry_k.reserve(P.entry_k.size());
-      AMDAT_CUDA(cudaMemcpy(pd->tiles.ptr, P.tiles.data(), P.tiles.size() * sizeof(LatticeTile), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(pd->entry_k.ptr, P.entry_k.data(), P.entry_k.size() * 4, cudaMemcpyHostToDevice));
+      upload_tables(ctx, {{pd->tiles.ptr, P.tiles.data(), P.tiles.size() * sizeof(LatticeTile)},
+                          {pd->entry_k.ptr, P.entry_k.data(), P.entry_k.size() * 4}});
       it = ctx->lattice_plans.emplace(key, pd).first;
     }
     const LatticePlanDev& P = *it->second;
@@ -757,7 +757,7 @@ amdat_status amdat_wave_density_lattice(amdat_ctx* ctx, int32_t list, float kmax
         int4* fx = fixed_turns(ctx, *d, e, period, d_frames);
         if (use_tensor_cores(ctx)) {
           LatticePlanDev& pw = *it->second;
-          if (!pw.half) pw.half = half_plan_build(*pw.kvec);
+          if (!pw.half) pw.half = half_plan_build(ctx, *pw.kvec);
           rhok_tc_run(ctx, *pw.half, fx, e.n, n_frames, d->n_k, d->rho->ptr);
         } else {
           dim3 grid((unsigned)P.n_tiles, (unsigned)n_frames);

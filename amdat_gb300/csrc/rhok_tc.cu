@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // ---------------------------------------------------------------------------
 // host: tile plan over the shell-sorted vector list, launches per frame batch
 // ---------------------------------------------------------------------------
-HalfPlan* half_plan_build(const std::vector<int32_t>& kvec) {
+HalfPlan* half_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec) {
   int nmax = 0;
   for (int v : kvec) nmax = std::max(nmax, std::abs(v));
   const LatticeIndex index(kvec, nmax);
@@ -583,10 +583,8 @@ HalfPlan* half_plan_build(const std::vector<int32_t>& kvec) {
     p->nmax = nmax;
     p->tiles.reserve(std::max<size_t>(tiles.size(), 1));
     p->entry_k.reserve(std::max<size_t>(entries.size(), 1));
-    if (!tiles.empty()) {
-      AMDAT_CUDA(cudaMemcpy(p->tiles.ptr, tiles.data(), tiles.size() * sizeof(HalfTile), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(p->entry_k.ptr, entries.data(), entries.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    }
+    upload_tables(ctx, {{p->tiles.ptr, tiles.data(), tiles.size() * sizeof(HalfTile)},
+                        {p->entry_k.ptr, entries.data(), entries.size() * sizeof(int2)}});
   } catch (...) {
     delete p;
     throw;

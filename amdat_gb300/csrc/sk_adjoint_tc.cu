@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(SA_THREADS, 1)
   }
 }
 
-TcPlan* tc_plan_build(const std::vector<int32_t>& kvec) {
+TcPlan* tc_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec) {
   int nmax = 0;
   for (int v : kvec) nmax = std::max(nmax, std::abs(v));
   const LatticeIndex index(kvec, nmax);
@@ -386,10 +386,8 @@ TcPlan* tc_plan_build(const std::vector<int32_t>& kvec) {
     p->host_tiles = tiles;
     p->tiles.reserve(std::max<size_t>(tiles.size(), 1));
     p->entry_k.reserve(std::max<size_t>(entries.size(), 1));
-    if (!tiles.empty()) {
-      AMDAT_CUDA(cudaMemcpy(p->tiles.ptr, tiles.data(), tiles.size() * sizeof(TcTile), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(p->entry_k.ptr, entries.data(), entries.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    }
+    upload_tables(ctx, {{p->tiles.ptr, tiles.data(), tiles.size() * sizeof(TcTile)},
+                        {p->entry_k.ptr, entries.data(), entries.size() * sizeof(int2)}});
   } catch (...) {
     delete p;
     throw;

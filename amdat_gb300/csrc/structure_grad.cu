@@ -867,7 +867,7 @@ void sk_adjoint_plans_free(amdat_ctx* ctx) {
   ctx->sk_adjoint_plans.clear();
 }
 
-static SkAdjointPlan* sk_adjoint_plan_build(const std::vector<int32_t>& kvec) {
+static SkAdjointPlan* sk_adjoint_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec) {
   const int nk = (int)(kvec.size() / 3);
   auto* A = new SkAdjointPlan();
   try {
@@ -879,9 +879,9 @@ static SkAdjointPlan* sk_adjoint_plan_build(const std::vector<int32_t>& kvec) {
       A->n_chunks = (int32_t)plan.chunks.size();
       A->cols.reserve(std::max<size_t>(plan.cols.size(), 1));
       A->chunks.reserve(std::max<size_t>(plan.chunks.size(), 1));
-      AMDAT_CUDA(cudaMemcpy(A->cols.ptr, plan.cols.data(), plan.cols.size() * sizeof(SkColumn), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(A->chunks.ptr, plan.chunks.data(), plan.chunks.size() * sizeof(SkChunk), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(A->slot.ptr, plan.slot.data(), (size_t)nk * 4, cudaMemcpyHostToDevice));
+      upload_tables(ctx, {{A->cols.ptr, plan.cols.data(), plan.cols.size() * sizeof(SkColumn)},
+                          {A->chunks.ptr, plan.chunks.data(), plan.chunks.size() * sizeof(SkChunk)},
+                          {A->slot.ptr, plan.slot.data(), (size_t)nk * 4}});
     } else {
       A->n_slots = nk;
       std::vector<int32_t> slot(nk);
@@ -891,8 +891,7 @@ static SkAdjointPlan* sk_adjoint_plan_build(const std::vector<int32_t>& kvec) {
         hk[k] = make_int4(kvec[3 * (size_t)k], kvec[3 * (size_t)k + 1], kvec[3 * (size_t)k + 2], 0);
       }
       A->kv.reserve(std::max(nk, 1));
-      AMDAT_CUDA(cudaMemcpy(A->kv.ptr, hk.data(), (size_t)nk * sizeof(int4), cudaMemcpyHostToDevice));
-      AMDAT_CUDA(cudaMemcpy(A->slot.ptr, slot.data(), (size_t)nk * 4, cudaMemcpyHostToDevice));
+      upload_tables(ctx, {{A->kv.ptr, hk.data(), (size_t)nk * sizeof(int4)}, {A->slot.ptr, slot.data(), (size_t)nk * 4}});
     }
   } catch (...) {
     delete A;
@@ -1177,10 +1176,10 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
     if (!d.lattice_key.empty()) {
       auto it = ctx->sk_adjoint_plans.find(d.lattice_key);
       if (it == ctx->sk_adjoint_plans.end())
-        it = ctx->sk_adjoint_plans.emplace(d.lattice_key, sk_adjoint_plan_build(*d.kvec)).first;
+        it = ctx->sk_adjoint_plans.emplace(d.lattice_key, sk_adjoint_plan_build(ctx, *d.kvec)).first;
       A = it->second;
     } else {
-      own.reset(sk_adjoint_plan_build(*d.kvec));
+      own.reset(sk_adjoint_plan_build(ctx, *d.kvec));
       A = own.get();
     }
     const int64_t n_slots = A->n_slots;

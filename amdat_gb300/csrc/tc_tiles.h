@@ -50,7 +50,7 @@ struct HalfPlan {
   int32_t n_tiles = 0, nzw = 0, nmax = 0;  // nzw: the widest tile's n
 };
 
-HalfPlan* half_plan_build(const std::vector<int32_t>& kvec);
+HalfPlan* half_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec);
 void half_plan_free(HalfPlan* p);
 
 struct TcTile {
@@ -65,7 +65,7 @@ struct TcPlan {
   int32_t n_tiles = 0, n_zblk = 0, nzw = 0, nmax = 0;
 };
 
-TcPlan* tc_plan_build(const std::vector<int32_t>& kvec);
+TcPlan* tc_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec);
 void tc_plan_free(TcPlan* p);
 // the tensor-core tiling of a lattice density's plan (built at first use)
 TcPlan* lattice_tc_plan(amdat_ctx* ctx, const std::string& lattice_key);
