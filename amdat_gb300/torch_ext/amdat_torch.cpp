@@ -28,7 +28,9 @@ void check(amdat_status st, const char* what) {
   TORCH_CHECK(st == AMDAT_OK, what, ": ", amdat_last_error());
 }
 
-// one engine context per device, on the caller's current stream
+// one engine context per device, on the caller's current stream (torch's default stream is
+// the legacy one, whose null handle would stand for the context's own stream, and that does
+// not wait for the kernels that make the inputs)
 amdat_ctx* engine(int device) {
   static std::mutex mu;
   static std::map<int, amdat_ctx*> ctxs;
@@ -39,7 +41,8 @@ amdat_ctx* engine(int device) {
     check(amdat_create(device, &c), "amdat_create");
     it = ctxs.emplace(device, c).first;
   }
-  check(amdat_set_stream(it->second, at::cuda::getCurrentCUDAStream(device).stream()), "amdat_set_stream");
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(device).stream();
+  check(amdat_set_stream(it->second, stream ? stream : cudaStreamLegacy), "amdat_set_stream");
   return it->second;
 }
 
