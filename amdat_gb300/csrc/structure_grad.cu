@@ -1120,10 +1120,12 @@ amdat_status amdat_structure_factor_adjoint(amdat_ctx* ctx, int32_t density_hand
     const size_t gbytes = (size_t)F * n * 3 * sizeof(float);
     // per-vector weights u_k = 2 w_s / H_s (zero outside the shells)
     std::vector<double> w(n_shells);
-    if (dev)
-      AMDAT_CUDA(cudaMemcpy(w.data(), dl_ds, (size_t)n_shells * 8, cudaMemcpyDeviceToHost));
-    else
+    if (dev) {
+      AMDAT_CUDA(cudaMemcpyAsync(w.data(), dl_ds, (size_t)n_shells * 8, cudaMemcpyDeviceToHost, ctx->stream));
+      AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
+    } else {
       std::memcpy(w.data(), dl_ds, (size_t)n_shells * 8);
+    }
     // (expanded on the device from the shells' values: [offsets | values])
     std::vector<int32_t> shells(2 * (size_t)n_shells + 1, 0);
     float max_u = 0.f;

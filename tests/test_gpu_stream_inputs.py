@@ -1,6 +1,9 @@
 """Device inputs made by kernels that are still queued when the call is made: the autograd
-functions on torch's default stream and on a stream of its own.  The result is that of the
-finished inputs, to the order of the FP64 additions."""
+functions on torch's default stream and on a stream of its own, and the structure factor's
+adjoint on the stream set with amdat_set_stream.  The result is that of the finished
+inputs, to the order of the FP64 additions."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -39,3 +42,32 @@ def test_autograd_waits_for_its_inputs(engine_mod, side, what):
     torch.cuda.synchronize()
     np.testing.assert_allclose(got.cpu().numpy(), want.cpu().numpy(), rtol=1e-12)
     np.testing.assert_array_equal(got_grad.cpu().numpy(), want_grad.cpu().numpy())
+
+
+def test_adjoint_reads_its_weights_on_the_context_stream(engine_mod):
+    eng = engine_mod.Engine(0)
+    stream = torch.cuda.Stream()
+    try:
+        pos = _pos(3)
+        torch.cuda.synchronize()
+        eng.upload_device(pos.data_ptr(), 2, N, [L] * 3)
+        eng.set_stream(stream.cuda_stream)
+        h, nk, ns = eng.wave_density_lattice(0, 4.0, 0.2, L, [0, 1])
+        off = eng.wave_density_vectors(h, nk, ns)[1]
+        weights = torch.cos(torch.arange(ns, device="cuda", dtype=torch.float64))
+        late = weights.clone()
+        weights.zero_()
+        grad = torch.zeros((2, N, 3), device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(WAIT)
+            weights.copy_(late)
+        engine_mod._check(engine_mod.lib().amdat_structure_factor_adjoint(
+            eng.handle, h, C.c_void_p(off.ctypes.data), ns, C.c_void_p(weights.data_ptr()), engine_mod.OUT_DEVICE,
+            C.c_void_p(grad.data_ptr())))
+        eng.synchronize()
+        want = eng.structure_factor_adjoint(h, off, late.cpu().numpy(), 2, N)
+        assert np.abs(want).max() > 0
+        np.testing.assert_array_equal(grad.cpu().numpy(), want)
+    finally:
+        eng.close()
