@@ -389,13 +389,16 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
     const float4 pi = live ? P1[i0 + lane] : make_float4(nan, nan, nan, __int_as_float(-1));
     const int ai = __float_as_int(pi.w);
     const uint64_t xi = pk2(pi.x, pi.x), yi = pk2(pi.y, pi.y), zi = pk2(pi.z, pi.z);
+    // the group's box, relative to the periodic box's origin (as every length below that
+    // only selects members: the origin may lie at any distance, and coordinates far from
+    // zero round by more than the cutoff's margin)
     float x0, x1, y0, y1, z0, z1;
-    warp_range(pi.x, x0, x1);
-    warp_range(pi.y, y0, y1);
-    warp_range(pi.z, z0, z1);
+    warp_range(pi.x - g.lo.x, x0, x1);
+    warp_range(pi.y - g.lo.y, y0, y1);
+    warp_range(pi.z - g.lo.z, z0, z1);
     // the pencils the cutoff reaches (all of an axis once when it reaches around)
-    int ya = (int)floorf((y0 - G.reach - g.lo.y) * g.inv.y), ny = (int)floorf((y1 + G.reach - g.lo.y) * g.inv.y) - ya + 1;
-    int za = (int)floorf((z0 - G.reach - g.lo.z) * g.inv.z), nz = (int)floorf((z1 + G.reach - g.lo.z) * g.inv.z) - za + 1;
+    int ya = (int)floorf((y0 - G.reach) * g.inv.y), ny = (int)floorf((y1 + G.reach) * g.inv.y) - ya + 1;
+    int za = (int)floorf((z0 - G.reach) * g.inv.z), nz = (int)floorf((z1 + G.reach) * g.inv.z) - za + 1;
     const bool all_y = ny >= g.n.y, all_z = nz >= g.n.z;
     if (all_y) ya = 0, ny = g.n.y;
     if (all_z) za = 0, nz = g.n.z;
@@ -414,8 +417,9 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
       for (int k = k0; k < k1; k += 32) {
         // only members within reach of the group's box are kept
         const float4 c = k + lane < k1 ? __ldg(P2 + k + lane) : make_float4(nan, nan, nan, 0.f);
-        const float gx = fmaxf(0.f, fabsf(min_image(c.x - xm, p.box.x)) - xh), gy = fmaxf(0.f, fabsf(min_image(c.y - ym, p.box.y)) - yh),
-                    gz = fmaxf(0.f, fabsf(min_image(c.z - zm, p.box.z)) - zh);
+        const float gx = fmaxf(0.f, fabsf(min_image(c.x - g.lo.x - xm, p.box.x)) - xh),
+                    gy = fmaxf(0.f, fabsf(min_image(c.y - g.lo.y - ym, p.box.y)) - yh),
+                    gz = fmaxf(0.f, fabsf(min_image(c.z - g.lo.z - zm, p.box.z)) - zh);
         const bool keep = k + lane < k1 && fmaf(gz, gz, fmaf(gy, gy, gx * gx)) <= G.reach * G.reach;
         const unsigned kept = __ballot_sync(0xffffffffu, keep);
         if (keep) {
@@ -446,14 +450,14 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
       int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
       if (t0 + lane < ny * nz) {
         const int jz = za + (t0 + lane) / ny, jy = ya + (t0 + lane) % ny;
-        const float fy = g.lo.y + (float)jy * g.cell.y, fz = g.lo.z + (float)jz * g.cell.z;
+        const float fy = (float)jy * g.cell.y, fz = (float)jz * g.cell.z;
         const float gy = all_y ? 0.f : fmaxf(0.f, fmaxf(fy - y1, y0 - (fy + g.cell.y)));
         const float gz = all_z ? 0.f : fmaxf(0.f, fmaxf(fz - z1, z0 - (fz + g.cell.z)));
         const float rem = G.reach * G.reach - gy * gy - gz * gz;
         if (rem >= 0.f) {
           const float h = sqrtf(rem);
           const int32_t* S = S2 + (wrap_index(jz, g.n.z) * g.n.y + wrap_index(jy, g.n.y)) * g.n.x;
-          const int xa = (int)floorf((x0 - h - g.lo.x) * g.inv.x), nx = (int)floorf((x1 + h - g.lo.x) * g.inv.x) - xa + 1;
+          const int xa = (int)floorf((x0 - h) * g.inv.x), nx = (int)floorf((x1 + h) * g.inv.x) - xa + 1;
           if (nx >= g.n.x) {
             a0 = S[0], a1 = S[g.n.x];
           } else {
