@@ -258,9 +258,12 @@ struct PHGrid {
   float tol;      // atoms further than this outside the box flag the call
 };
 
-__device__ __forceinline__ int ph_cell_axis(float x, float lo, float inv_cell, int n) {
+__device__ __forceinline__ int wrap_index(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
+
+// the cell of a coordinate; outside the box its image's (wrap) or the nearest one
+__device__ __forceinline__ int ph_cell_axis(float x, float lo, float inv_cell, int n, bool wrap) {
   const int c = (int)floorf((x - lo) * inv_cell);
-  return min(max(c, 0), n - 1);
+  return min(max(wrap ? wrap_index(c, n) : c, 0), n - 1);
 }
 
 // members of list l at frame frames[s] counted into the cells of slot s
@@ -273,8 +276,10 @@ __global__ void ph_cell_count_kernel(const float* __restrict__ w, int64_t n_pad,
   const float* P = w + (int64_t)frames[s] * 3 * n_pad;
   const int a = member(l, i);
   const float x = P[a], y = P[n_pad + a], z = P[2 * n_pad + a];
-  int cx = ph_cell_axis(x, g.lo.x, g.inv.x, g.n.x), cy = ph_cell_axis(y, g.lo.y, g.inv.y, g.n.y);
-  const int cz = ph_cell_axis(z, g.lo.z, g.inv.z, g.n.z);
+  // list 1 (snake) keeps an atom beside its neighbours, list 2 is looked up by image
+  const bool wrap = !g.snake;
+  int cx = ph_cell_axis(x, g.lo.x, g.inv.x, g.n.x, wrap), cy = ph_cell_axis(y, g.lo.y, g.inv.y, g.n.y, wrap);
+  const int cz = ph_cell_axis(z, g.lo.z, g.inv.z, g.n.z, wrap);
   if (g.snake) {
     if (cz & 1) cy = g.n.y - 1 - cy;
     if ((cz * g.n.y + cy) & 1) cx = g.n.x - 1 - cx;
@@ -334,8 +339,6 @@ __global__ void ph_cell_scatter_kernel(const float* __restrict__ w, int64_t n_pa
   pos[(int64_t)s * l.n + k] = make_float4(P[a], P[n_pad + a], P[2 * n_pad + a], __int_as_float(a));
 }
 
-__device__ __forceinline__ int wrap_index(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
-
 // group minimum and maximum of a coordinate (lanes without an atom pass NaN)
 __device__ __forceinline__ void warp_range(float v, float& lo, float& hi) {
   lo = hi = v;
@@ -360,7 +363,7 @@ struct PHGroups {
   const int32_t* slot_b;
   float reach;            // cutoff with its margin
   int32_t same;           // one list: each atom's own pair is taken out at the end
-  const int32_t* outside;  // set: some atom lies outside the box, nothing is counted
+  const int32_t* outside;  // set: some atom lies far outside the box, nothing is counted
 };
 
 template <int SELF>
@@ -590,7 +593,10 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     const double edge = (double)std::max(ctx->box[0], std::max(ctx->box[1], ctx->box[2]));
     const double w1 = std::cbrt(32.0 * vol / l1.n), rho2 = l2.n / vol;
     const double f2 = std::max((double)max_distance / 2.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
-    const float tol = (float)std::max(2e-5 * max_distance, 4e-7 * edge);
+    // wrapped coordinates need not lie in the box (read from a file so, or rounded there
+    // from far unwrapped ones).  Up to an eighth of it the cells wrap and L - |d| is still
+    // the distance to the nearest image; beyond, the all-pairs pass gives the chain's value
+    const float tol = 0.125f * std::min(ctx->box[0], std::min(ctx->box[1], ctx->box[2]));
     const PHGrid grid[2] = {make_grid(ctx, 0.125 * w1, w1, true, tol),
                             make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol)};
     const ListEntry* lists[2] = {&l1, &l2};
@@ -659,7 +665,7 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
     if (G.same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>);
     else launch(pair_hist_groups_kernel<PH_SELF_IDS>);
-    // atoms outside the box (wrapped coordinates given so): the all-pairs pass instead
+    // atoms far outside the box: the all-pairs pass instead
     int32_t outside = 0;
     AMDAT_CUDA(cudaMemcpyAsync(&outside, cb + o_flag, 4, cudaMemcpyDeviceToHost, st));
     AMDAT_CUDA(cudaStreamSynchronize(st));

@@ -32,3 +32,20 @@ def test_vhd_cells_far_origin(eng, monkeypatch, lo, max_d):
     for l1, l2 in ((0, 0), (few, many), (many, 0)):
         got, want = _both(eng, monkeypatch, l1, l2, max_d, 49)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("out,cells", [(1e-5, True), (1e-2, True), (0.4, True), (1.8, True), (3.5, False)])
+def test_vhd_cells_outside_the_box(eng, monkeypatch, out, cells):
+    """Wrapped coordinates up to an eighth of the box outside it stay with the cell pass."""
+    rng = np.random.default_rng(3)
+    L, n = np.array([15.0, 16.0, 27.0], np.float32), 6000
+    w = (rng.random((3, n, 3)) * (L + 2 * out) - out).astype(np.float32)
+    eng.upload(w, L, wrapped=w)
+    eng.set_scheme(synth.TimeScheme.linear(3, 1.0))
+    some = eng.list(np.arange(0, n, 2))
+    for l1, l2 in ((0, 0), (some, 0), (0, some)):
+        eng.profile_reset()
+        eng.vhd(l1, l2, 4.9, 49)
+        assert (eng.profile_kernel("pair_hist_kernel")[0] == 0) == cells
+        got, want = _both(eng, monkeypatch, l1, l2, 4.9, 49)
+        np.testing.assert_array_equal(got, want)
