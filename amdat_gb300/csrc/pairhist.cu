@@ -293,37 +293,50 @@ __global__ void ph_cell_count_kernel(const float* __restrict__ w, int64_t n_pad,
 }
 
 // exclusive scan of one slot's cell counts (one block per slot) into start and
-// the scatter cursors
-__global__ void __launch_bounds__(1024) ph_cell_scan_kernel(const int32_t* __restrict__ count, int32_t n_cells,
-                                                            int32_t* __restrict__ start, int32_t* __restrict__ cursor) {
-  __shared__ int32_t s_part[1024];
-  __shared__ int32_t s_carry;
-  const int s = blockIdx.x;
+// the scatter cursors: four cells per thread, shuffle scans of a warp and of the warps
+// (50,000 cells: 15 us; a scan over 1,024 cells at a time in shared memory, ten barriers
+// each, 110)
+constexpr int PS_THREADS = 1024, PS_ITEMS = 4;
+__device__ __forceinline__ int32_t warp_scan(int32_t v, int lane) {  // inclusive
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, v, off);
+    if (lane >= off) v += u;
+  }
+  return v;
+}
+__global__ void __launch_bounds__(PS_THREADS) ph_cell_scan_kernel(const int32_t* __restrict__ count, int32_t n_cells,
+                                                                  int32_t* __restrict__ start, int32_t* __restrict__ cursor) {
+  __shared__ int32_t s_warp[2][32];
+  const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t* C = count + (int64_t)s * n_cells;
   int32_t* S = start + (int64_t)s * (n_cells + 1);
   int32_t* U = cursor + (int64_t)s * n_cells;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (int base = 0; base < n_cells; base += 1024) {
-    const int i = base + threadIdx.x;
-    s_part[threadIdx.x] = i < n_cells ? C[i] : 0;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-      const int v = threadIdx.x >= off ? s_part[threadIdx.x - off] : 0;
-      __syncthreads();
-      s_part[threadIdx.x] += v;
-      __syncthreads();
+  int32_t carry = 0;
+  for (int base = 0, it = 0; base < n_cells; base += PS_THREADS * PS_ITEMS, ++it) {
+    const int i0 = base + PS_ITEMS * threadIdx.x;
+    int32_t v[PS_ITEMS], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PS_ITEMS; ++j) {
+      v[j] = i0 + j < n_cells ? C[i0 + j] : 0;
+      sum += v[j];
     }
-    if (i < n_cells) {
-      const int excl = s_carry + s_part[threadIdx.x] - C[i];
-      S[i] = excl;
-      U[i] = excl;
-    }
+    const int32_t incl = warp_scan(sum, lane);
+    int32_t* T = s_warp[it & 1];  // written again after the next iteration's barrier
+    if (lane == 31) T[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) s_carry += s_part[1023];
-    __syncthreads();
+    const int32_t totals = warp_scan(T[lane], lane);  // every warp scans the warps' totals
+    int32_t excl = carry + incl - sum + (warp ? __shfl_sync(0xffffffffu, totals, warp - 1) : 0);
+    carry += __shfl_sync(0xffffffffu, totals, 31);
+#pragma unroll
+    for (int j = 0; j < PS_ITEMS; ++j)
+      if (i0 + j < n_cells) {
+        S[i0 + j] = excl;
+        U[i0 + j] = excl;
+        excl += v[j];
+      }
   }
-  if (threadIdx.x == 0) S[n_cells] = s_carry;
+  if (threadIdx.x == 0) S[n_cells] = carry;
 }
 
 __global__ void ph_cell_scatter_kernel(const float* __restrict__ w, int64_t n_pad, PHList l,
@@ -519,6 +532,29 @@ static PHGrid make_grid(amdat_ctx* ctx, double edge_x, double edge_yz, bool snak
   return g;
 }
 
+// units of the all-pairs pass, 256 I members by up to seg list-2 members: wide ones while
+// they fill the chip six times over, then fewer members per thread and shorter segments
+static std::vector<PHUnit> pair_units(const amdat_ctx* ctx, int n1, int n2, bool symmetric, int64_t n_q, int* per_thread) {
+  const int64_t want = 6 * (int64_t)ctx->n_sm;
+  auto count_units = [&](int I, int seg) {
+    const int64_t ib = ceil_div(n1, 256 * I), js = ceil_div(n2, seg);
+    return (symmetric ? (ib * js + ib) / 2 : ib * js) * n_q;
+  };
+  int I = 4, seg = 8192;
+  while (seg > 1024 && count_units(I, seg) < want) seg /= 2;
+  while (I > 1 && count_units(I, seg) < want) I /= 2;
+  while (seg > 128 && count_units(I, seg) < want) seg /= 2;
+  std::vector<PHUnit> units;
+  for (int i0 = 0; i0 < n1; i0 += 256 * I) {
+    const int i1 = std::min(n1, i0 + 256 * I);
+    if (symmetric)
+      for (int j = i0; j < i1; j += seg) units.push_back(PHUnit{i0, j, std::min(i1, j + seg), 1});
+    for (int j = symmetric ? i1 : 0; j < n2; j += seg) units.push_back(PHUnit{i0, j, std::min(n2, j + seg), symmetric ? 2 : 1});
+  }
+  *per_thread = I;
+  return units;
+}
+
 static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& l2, bool symmetric,
                           const std::vector<int32_t>& fa, const std::vector<int32_t>& fb,
                           const std::vector<int32_t>& row, int32_t n_rows_out, float max_distance,
@@ -528,21 +564,48 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   AMDAT_REQUIRE(counts != nullptr, "null output");
   const size_t n_q = fa.size();
   const size_t n_out = (size_t)n_rows_out * n_bins;
+  const bool any = n_q && l1.n > 0 && l2.n > 0;
+  AMDAT_REQUIRE(!any || n_q <= 65535, "at most 65535 frames or time pairs per call");
+  // cell lists for the ordered pass when the box holds at least three cutoffs per axis
+  const float cell_edge = (float)((double)max_distance * (1.0 + 1e-4));
+  const int3 nc = make_int3((int)std::floor(ctx->box[0] / cell_edge), (int)std::floor(ctx->box[1] / cell_edge),
+                            (int)std::floor(ctx->box[2] / cell_edge));
+  const int64_t n_cells = (int64_t)nc.x * nc.y * nc.z;
+  const char* pc = std::getenv("AMDAT_PAIR_CELLS");  // "off": the all-pairs pass
+  const bool cells = !symmetric && any && l2.n >= 1024 && nc.x >= 3 && nc.y >= 3 && nc.z >= 3 &&
+                     n_cells <= (1 << 20) && !(pc && std::strcmp(pc, "off") == 0);
+  // the host's tables go to the device in one copy
   auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  size_t o = 0;
-  const size_t o_fa = o; o = align(o + std::max<size_t>(n_q, 1) * 4);
-  const size_t o_fb = o; o = align(o + std::max<size_t>(n_q, 1) * 4);
-  const size_t o_row = o; o = align(o + std::max<size_t>(n_q, 1) * 4);
-  const size_t o_cnt = o; o = align(o + n_out * 8);
-  unsigned char* base = ctx->scratch.reserve(o);
-  std::vector<unsigned char> host(o_cnt, 0);
-  if (n_q) {
-    std::memcpy(host.data() + o_fa, fa.data(), n_q * 4);
-    std::memcpy(host.data() + o_fb, fb.data(), n_q * 4);
-    std::memcpy(host.data() + o_row, row.data(), n_q * 4);
+  std::vector<unsigned char> host;
+  auto table = [&](const auto& v) {
+    const size_t at = host.size(), bytes = v.size() * sizeof(v[0]);
+    host.resize(align(at + bytes));
+    if (bytes) std::memcpy(host.data() + at, v.data(), bytes);
+    return at;
+  };
+  const size_t o_fa = table(fa), o_fb = table(fb), o_row = table(row);
+  std::vector<int32_t> fr[2], slot[2];  // the distinct frames of each side and each row's place among them
+  size_t o_fr[2] = {0, 0}, o_slot[2] = {0, 0}, o_units = 0;
+  std::vector<PHUnit> units;
+  int per_thread = 1;
+  if (cells) {
+    for (int s = 0; s < 2; ++s) {
+      const std::vector<int32_t>& f = s ? fb : fa;
+      fr[s] = f;
+      std::sort(fr[s].begin(), fr[s].end());
+      fr[s].erase(std::unique(fr[s].begin(), fr[s].end()), fr[s].end());
+      for (int32_t x : f) slot[s].push_back((int32_t)(std::lower_bound(fr[s].begin(), fr[s].end(), x) - fr[s].begin()));
+      o_fr[s] = table(fr[s]);
+      o_slot[s] = table(slot[s]);
+    }
+  } else if (any) {
+    units = pair_units(ctx, l1.n, l2.n, symmetric, (int64_t)n_q, &per_thread);
+    o_units = table(units);
   }
-  AMDAT_CUDA(cudaMemcpyAsync(base, host.data(), o_cnt, cudaMemcpyHostToDevice, ctx->stream));
-  AMDAT_CUDA(cudaMemsetAsync(base + o_cnt, 0, n_out * 8, ctx->stream));
+  const size_t o_flag = host.size(), o_cnt = align(o_flag + 4);
+  unsigned char* base = ctx->scratch.reserve(o_cnt + n_out * 8);
+  if (!host.empty()) AMDAT_CUDA(cudaMemcpyAsync(base, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
+  AMDAT_CUDA(cudaMemsetAsync(base + o_flag, 0, o_cnt - o_flag + n_out * 8, ctx->stream));
   PHParams p{};
   p.w = ctx->w.ptr;
   p.n_pad = ctx->n_pad;
@@ -563,28 +626,7 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   p.s2_cut = (float)(cut * cut);
   p.n_bins = n_bins;
   p.counts = (unsigned long long*)(base + o_cnt);
-  // cell lists for the ordered pass when the box holds at least three cutoffs per axis
-  const float cell_edge = (float)((double)max_distance * (1.0 + 1e-4));
-  const int3 nc = make_int3((int)std::floor(ctx->box[0] / cell_edge), (int)std::floor(ctx->box[1] / cell_edge),
-                            (int)std::floor(ctx->box[2] / cell_edge));
-  const int64_t n_cells = (int64_t)nc.x * nc.y * nc.z;
-  const char* pc = std::getenv("AMDAT_PAIR_CELLS");  // "off": the all-pairs pass
-  const bool cells = !symmetric && n_q && l1.n > 0 && l2.n >= 1024 && nc.x >= 3 && nc.y >= 3 && nc.z >= 3 &&
-                     n_cells <= (1 << 20) && !(pc && std::strcmp(pc, "off") == 0);
-  bool done = false;
   if (cells) {
-    // frame slots: the distinct frames of each side
-    auto slots = [](const std::vector<int32_t>& f, std::vector<int32_t>& uniq, std::vector<int32_t>& slot_of) {
-      uniq = f;
-      std::sort(uniq.begin(), uniq.end());
-      uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
-      slot_of.resize(f.size());
-      for (size_t i = 0; i < f.size(); ++i)
-        slot_of[i] = (int32_t)(std::lower_bound(uniq.begin(), uniq.end(), f[i]) - uniq.begin());
-    };
-    std::vector<int32_t> fr[2], slot[2];
-    slots(fa, fr[0], slot[0]);
-    slots(fb, fr[1], slot[1]);
     // list 1: pencils as wide as the cube of 32 atoms, x cells an eighth of that (a quarter
     // leaves the groups longer: 2 % slower); list 2: pencils of half the cutoff (a third:
     // 5 % slower, more runs; the whole: 2 %), but wide enough for runs of about 16 atoms,
@@ -601,53 +643,45 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
                             make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol)};
     const ListEntry* lists[2] = {&l1, &l2};
     size_t need = 0;
-    size_t off[2][6];
+    size_t off[2][5];
     for (int s = 0; s < 2; ++s) {
       const size_t nf = fr[s].size(), n = (size_t)lists[s]->n, nc1 = (size_t)grid[s].n_cells;
-      off[s][0] = need; need = align(need + nf * 4);               // frames
-      off[s][1] = need; need = align(need + nf * n * 4);           // cell_of
-      off[s][2] = need; need = align(need + nf * nc1 * 4);         // count
-      off[s][3] = need; need = align(need + nf * (nc1 + 1) * 4);   // start
-      off[s][4] = need; need = align(need + nf * nc1 * 4);         // cursor
-      off[s][5] = need; need = align(need + nf * n * sizeof(float4));  // pos
+      off[s][0] = need; need = align(need + nf * n * 4);           // cell_of
+      off[s][1] = need; need = align(need + nf * nc1 * 4);         // count
+      off[s][2] = need; need = align(need + nf * (nc1 + 1) * 4);   // start
+      off[s][3] = need; need = align(need + nf * nc1 * 4);         // cursor
+      off[s][4] = need; need = align(need + nf * n * sizeof(float4));  // pos
     }
-    const size_t o_slot[2] = {need, align(need + n_q * 4)};
-    const size_t o_flag = align(o_slot[1] + n_q * 4);
-    unsigned char* cb = ctx->scratch2.reserve(o_flag + 4);
+    unsigned char* cb = ctx->scratch2.reserve(need);
     cudaStream_t st = ctx->stream;
-    AMDAT_CUDA(cudaMemsetAsync(cb + o_flag, 0, 4, st));
     for (int s = 0; s < 2; ++s) {
       const int nf = (int)fr[s].size();
       const PHList l = phview(*lists[s]);
       const PHGrid& gs = grid[s];
-      AMDAT_REQUIRE(nf <= 65535, "at most 65535 frames per call");
-      AMDAT_CUDA(cudaMemcpyAsync(cb + o_slot[s], slot[s].data(), n_q * 4, cudaMemcpyHostToDevice, st));
-      AMDAT_CUDA(cudaMemcpyAsync(cb + off[s][0], fr[s].data(), (size_t)nf * 4, cudaMemcpyHostToDevice, st));
-      AMDAT_CUDA(cudaMemsetAsync(cb + off[s][2], 0, (size_t)nf * gs.n_cells * 4, st));
+      const int32_t* frames = (const int32_t*)(base + o_fr[s]);
+      AMDAT_CUDA(cudaMemsetAsync(cb + off[s][1], 0, (size_t)nf * gs.n_cells * 4, st));
       const dim3 gn((unsigned)ceil_div(l.n, 256), (unsigned)nf);
-      ph_cell_count_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), gs,
-                                               (int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][2]), (int32_t*)(cb + o_flag));
-      ph_cell_scan_kernel<<<(unsigned)nf, 1024, 0, st>>>((const int32_t*)(cb + off[s][2]), gs.n_cells,
-                                                          (int32_t*)(cb + off[s][3]), (int32_t*)(cb + off[s][4]));
-      ph_cell_scatter_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, (const int32_t*)(cb + off[s][0]), gs.n_cells,
-                                                 (const int32_t*)(cb + off[s][1]), (int32_t*)(cb + off[s][4]),
-                                                 (float4*)(cb + off[s][5]));
+      ph_cell_count_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, frames, gs, (int32_t*)(cb + off[s][0]),
+                                               (int32_t*)(cb + off[s][1]), (int32_t*)(base + o_flag));
+      ph_cell_scan_kernel<<<(unsigned)nf, PS_THREADS, 0, st>>>((const int32_t*)(cb + off[s][1]), gs.n_cells,
+                                                               (int32_t*)(cb + off[s][2]), (int32_t*)(cb + off[s][3]));
+      ph_cell_scatter_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, frames, gs.n_cells, (const int32_t*)(cb + off[s][0]),
+                                                 (int32_t*)(cb + off[s][3]), (float4*)(cb + off[s][4]));
       check_launch("pair cell lists");
       count_launch(ctx, 3);
     }
-    AMDAT_REQUIRE(n_q <= 65535, "at most 65535 frames or time pairs per call");
     PHGroups G;
-    G.pos1 = (const float4*)(cb + off[0][5]);
+    G.pos1 = (const float4*)(cb + off[0][4]);
     G.n1 = l1.n;
-    G.pos2 = (const float4*)(cb + off[1][5]);
-    G.start2 = (const int32_t*)(cb + off[1][3]);
+    G.pos2 = (const float4*)(cb + off[1][4]);
+    G.start2 = (const int32_t*)(cb + off[1][2]);
     G.n2 = l2.n;
     G.g2 = grid[1];
-    G.slot_a = (const int32_t*)(cb + o_slot[0]);
-    G.slot_b = (const int32_t*)(cb + o_slot[1]);
+    G.slot_a = (const int32_t*)(base + o_slot[0]);
+    G.slot_b = (const int32_t*)(base + o_slot[1]);
     G.reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
     G.same = &l1 == &l2 ? 1 : 0;
-    G.outside = (const int32_t*)(cb + o_flag);
+    G.outside = (const int32_t*)(base + o_flag);
     // up to eight groups per warp (one flush of the histograms for them) while the blocks
     // fill the chip twice over
     const int64_t groups = ceil_div(l1.n, 32);
@@ -665,37 +699,9 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
     if (G.same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>);
     else launch(pair_hist_groups_kernel<PH_SELF_IDS>);
-    // atoms far outside the box: the all-pairs pass instead
-    int32_t outside = 0;
-    AMDAT_CUDA(cudaMemcpyAsync(&outside, cb + o_flag, 4, cudaMemcpyDeviceToHost, st));
-    AMDAT_CUDA(cudaStreamSynchronize(st));
-    done = outside == 0;
-    if (!done) AMDAT_CUDA(cudaMemsetAsync(base + o_cnt, 0, n_out * 8, st));
   }
-  if (!done && n_q && l1.n > 0 && l2.n > 0) {
-    AMDAT_REQUIRE(n_q <= 65535, "at most 65535 frames or time pairs per call");
-    // units of 256 I members by up to seg list-2 members: wide ones while they fill
-    // the chip six times over, then fewer members per thread and shorter segments
+  auto all_pairs = [&](const PHUnit* d_units) {
     const bool ids = fa != fb;
-    const int64_t want = 6 * (int64_t)ctx->n_sm;
-    auto count_units = [&](int I, int seg) {
-      const int64_t ib = ceil_div(l1.n, 256 * I), js = ceil_div(l2.n, seg);
-      return (symmetric ? (ib * js + ib) / 2 : ib * js) * (int64_t)n_q;
-    };
-    int I = 4, seg = 8192;
-    while (seg > 1024 && count_units(I, seg) < want) seg /= 2;
-    while (I > 1 && count_units(I, seg) < want) I /= 2;
-    while (seg > 128 && count_units(I, seg) < want) seg /= 2;
-    std::vector<PHUnit> units;
-    for (int i0 = 0; i0 < l1.n; i0 += 256 * I) {
-      const int i1 = std::min(l1.n, i0 + 256 * I);
-      if (symmetric)
-        for (int j = i0; j < i1; j += seg) units.push_back(PHUnit{i0, j, std::min(i1, j + seg), 1});
-      for (int j = symmetric ? i1 : 0; j < l2.n; j += seg)
-        units.push_back(PHUnit{i0, j, std::min(l2.n, j + seg), symmetric ? 2 : 1});
-    }
-    PHUnit* d_units = (PHUnit*)ctx->scratch2.reserve(units.size() * sizeof(PHUnit));
-    AMDAT_CUDA(cudaMemcpyAsync(d_units, units.data(), units.size() * sizeof(PHUnit), cudaMemcpyHostToDevice, ctx->stream));
     const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
     auto launch = [&](auto kern) {
       if (shm > 32 * 1024)
@@ -705,13 +711,30 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
       check_launch("pair_hist_kernel");
       count_launch(ctx);
     };
+    const int I = per_thread;
     if (ids) I == 4 ? launch(pair_hist_kernel<4, PH_SELF_IDS>) : I == 2 ? launch(pair_hist_kernel<2, PH_SELF_IDS>) : launch(pair_hist_kernel<1, PH_SELF_IDS>);
     else I == 4 ? launch(pair_hist_kernel<4, PH_SELF_ZERO>) : I == 2 ? launch(pair_hist_kernel<2, PH_SELF_ZERO>) : launch(pair_hist_kernel<1, PH_SELF_ZERO>);
+  };
+  auto read = [&] {
+    AMDAT_CUDA(cudaMemcpyAsync(counts, base + o_cnt, n_out * 8,
+                               out_flags == AMDAT_OUT_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                               ctx->stream));
+    AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
+  };
+  if (any && !cells) all_pairs((const PHUnit*)(base + o_units));
+  int32_t here = 0, *outside = ctx->result ? (int32_t*)ctx->result : &here;
+  *outside = 0;
+  if (cells) AMDAT_CUDA(cudaMemcpyAsync(outside, base + o_flag, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  read();
+  if (*outside) {
+    // atoms far outside the box: the all-pairs pass instead
+    units = pair_units(ctx, l1.n, l2.n, symmetric, (int64_t)n_q, &per_thread);
+    PHUnit* d_units = (PHUnit*)ctx->scratch2.reserve(units.size() * sizeof(PHUnit));
+    AMDAT_CUDA(cudaMemcpyAsync(d_units, units.data(), units.size() * sizeof(PHUnit), cudaMemcpyHostToDevice, ctx->stream));
+    AMDAT_CUDA(cudaMemsetAsync(base + o_cnt, 0, n_out * 8, ctx->stream));
+    all_pairs(d_units);
+    read();
   }
-  AMDAT_CUDA(cudaMemcpyAsync(counts, base + o_cnt, n_out * 8,
-                             out_flags == AMDAT_OUT_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                             ctx->stream));
-  AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
 }  // namespace amdat

@@ -49,3 +49,17 @@ def test_vhd_cells_outside_the_box(eng, monkeypatch, out, cells):
         assert (eng.profile_kernel("pair_hist_kernel")[0] == 0) == cells
         got, want = _both(eng, monkeypatch, l1, l2, 4.9, 49)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("n,box,max_d", [(40000, 34.0, 1.0), (1024, 300.0, 0.9), (30000, (200.0, 9.5, 3.2), 1.05)])
+def test_vhd_cells_many_cells(eng, monkeypatch, n, box, max_d):
+    """More cells than the scan takes at a time, and mostly empty ones."""
+    rng = np.random.default_rng(n)
+    L = np.broadcast_to(np.float32(box), 3).astype(np.float32)
+    eng.upload((rng.random((2, n, 3)) * L).astype(np.float32), L)
+    eng.set_scheme(synth.TimeScheme.linear(2, 1.0))
+    for l1, l2 in ((0, 0), (eng.list(np.arange(1, n, 9)), 0)):
+        monkeypatch.delenv("AMDAT_PAIR_CELLS", raising=False)
+        got = eng.vhd(l1, l2, max_d, 30)
+        monkeypatch.setenv("AMDAT_PAIR_CELLS", "off")
+        np.testing.assert_array_equal(got, eng.vhd(l1, l2, max_d, 30))
