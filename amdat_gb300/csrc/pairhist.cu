@@ -514,6 +514,59 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
   flush_counts(p, sh_hist, p.row_of[q]);
 }
 
+// The walk: list-1 members too sparse for compact groups (a few atoms of a solute, cutoffs
+// below the atoms' spacing).  PARTS lanes per list-1 member go through the 27 cells around
+// its own, cells at least as wide as the cutoff, a cell per lane at a time; every pair takes
+// the exact chain.  Bound by the latency of its scattered loads.
+struct PHWalk {
+  const float4* pos1;     // [slot][n1] in cell order
+  int32_t n1;
+  const float4* pos2;     // [slot][n2]
+  const int32_t* start2;  // [slot][n_cells + 1]
+  int32_t n2;
+  PHGrid g;
+  const int32_t* slot_a;
+  const int32_t* slot_b;
+  const int32_t* outside;
+};
+
+template <int PARTS>
+__global__ void __launch_bounds__(PH_THREADS) pair_hist_walk_kernel(PHParams p, PHWalk W) {
+  extern __shared__ unsigned int sh_hist[];  // [8 warps][n_bins + 1]
+  if (*W.outside) return;
+  const int q = blockIdx.y, nb1 = p.n_bins + 1;
+  unsigned int* whist = sh_hist + (threadIdx.x >> 5) * nb1;
+  for (int b = threadIdx.x; b < PH_WARPS * nb1; b += PH_THREADS) sh_hist[b] = 0u;
+  __syncthreads();
+  const int i = blockIdx.x * (PH_THREADS / PARTS) + threadIdx.x / PARTS;
+  if (i < W.n1) {
+    const PHGrid& g = W.g;
+    const float4 pi = W.pos1[(int64_t)W.slot_a[q] * W.n1 + i];
+    const int32_t* S2 = W.start2 + (int64_t)W.slot_b[q] * (g.n_cells + 1);
+    const float4* P2 = W.pos2 + (int64_t)W.slot_b[q] * W.n2;
+    const int cx = ph_cell_axis(pi.x, g.lo.x, g.inv.x, g.n.x, true), cy = ph_cell_axis(pi.y, g.lo.y, g.inv.y, g.n.y, true),
+              cz = ph_cell_axis(pi.z, g.lo.z, g.inv.z, g.n.z, true);
+    for (int off = threadIdx.x % PARTS; off < 27; off += PARTS) {
+      const int x = wrap_index(cx + off % 3 - 1, g.n.x), y = wrap_index(cy + off / 3 % 3 - 1, g.n.y),
+                z = wrap_index(cz + off / 9 - 1, g.n.z);
+      const int c = (z * g.n.y + y) * g.n.x + x;
+      const int k1 = __ldg(S2 + c + 1);
+      for (int k = __ldg(S2 + c); k < k1; ++k) {
+        const float4 cj = __ldg(P2 + k);
+        const float mx = min_image(__fsub_rn(cj.x, pi.x), p.box.x), my = min_image(__fsub_rn(cj.y, pi.y), p.box.y),
+                    mz = min_image(__fsub_rn(cj.z, pi.z), p.box.z);
+        const float s2 = __fadd_rn(__fadd_rn(__fmul_rn(mx, mx), __fmul_rn(my, my)), __fmul_rn(mz, mz));
+        if (s2 < p.s2_cut && __float_as_int(cj.w) != __float_as_int(pi.w)) {
+          const int b = (int)__fdiv_rn(__fsqrt_rn(s2), p.bin_size);
+          if (b < p.n_bins) atomicAdd(whist + b, 1u);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  flush_counts(p, sh_hist, p.row_of[q]);
+}
+
 // cells of about edge_x x edge_yz x edge_yz over the box, at most 2^20
 static PHGrid make_grid(amdat_ctx* ctx, double edge_x, double edge_yz, bool snake, float tol) {
   auto cells = [](double L, double e, int most) { return (int)std::min<double>(most, std::max(1.0, std::floor(L / e))); };
@@ -588,10 +641,52 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   size_t o_fr[2] = {0, 0}, o_slot[2] = {0, 0}, o_units = 0;
   std::vector<PHUnit> units;
   int per_thread = 1;
+  PHGrid grid[2];
+  bool walk = false;
+  int lanes = 1;  // of the walk, per list-1 member
+  const double edge = (double)std::max(ctx->box[0], std::max(ctx->box[1], ctx->box[2]));
+  const bool same = &l1 == &l2;
+  int sides = 2;
   if (cells) {
+    // list 1: pencils as wide as the cube of 32 atoms, x cells an eighth of that (a quarter
+    // leaves the groups longer: 2 % slower); list 2: pencils of half the cutoff (a third:
+    // 5 % slower, more runs; the whole: 2 %), but wide enough for runs of about 16 atoms,
+    // x cells of half a pencil or two atoms
+    const double vol = (double)ctx->box[0] * ctx->box[1] * ctx->box[2];
+    const double w1 = std::cbrt(32.0 * vol / l1.n), rho2 = l2.n / vol;
+    const double f2 = std::max((double)max_distance / 2.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
+    // wrapped coordinates need not lie in the box (read from a file so, or rounded there
+    // from far unwrapped ones).  Up to an eighth of it the cells wrap and L - |d| is still
+    // the distance to the nearest image; beyond, the all-pairs pass gives the chain's value
+    const float tol = 0.125f * std::min(ctx->box[0], std::min(ctx->box[1], ctx->box[2]));
+    grid[0] = make_grid(ctx, 0.125 * w1, w1, true, tol);
+    grid[1] = make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol);
+    // The walk instead of the groups where these would gather far more members.  Gathered
+    // for a group: the members of its box (as the cube of its atoms) widened by the cutoff.
+    // Walked for an atom: the members of 27 cells, each cell costing as much as 0.7 of them.
+    // G_d of n1 atoms to n2, groups / walk: 10 to 64,000 (r 3.0, 12 frames) 3,677 / 122 us
+    // (428 with a thread per atom, as before the groups), 1,000 to 200,000 (2.0, 2 frames)
+    // 1,706 / 166; 16,000 to 200,000 (2.0, 12 frames) 1,942 / 900.  At the line: 64,000 to
+    // 200,000 (2.0, 12 frames) 2,723 / 2,547 at 2.4 times the walk's members, 64,000 to
+    // themselves (2.0, 12 frames) 1,606 / 2,138 at 1.4; few atoms, 32 lanes each: 1,000 to 3,000 (3.0,
+    // 12 frames) 209 / 217 at 1.3, 1,000 to 20,000 (5.0) 649 / 778 at 1.2.
+    const double ew = std::max((double)max_distance * (1.0 + 1e-4) + 1e-6 * edge, std::cbrt(2.0 / rho2));
+    const PHGrid gw = make_grid(ctx, ew, ew, false, tol);
+    const double c = max_distance, w = l1.n > 1 ? std::min(w1, std::cbrt(vol)) : 0.0;
+    const double by_group = std::min<double>(l2.n, rho2 * (w * w * w + 6.0 * w * w * c + 9.42 * w * c * c + 4.19 * c * c * c));
+    const double by_walk = 27.0 * ((double)l2.n / gw.n_cells + 0.7);
+    // lanes per atom while there are too few to fill the chip (10 to 64,000 as above: 427 /
+    // 169 / 122 us with 1, 8 and 32; 4,000 to 64,000: 374 / 332 / 367)
+    const int64_t members = (int64_t)l1.n * (int64_t)n_q;
+    lanes = members <= 512 * (int64_t)ctx->n_sm ? 32 : (members <= 2048 * (int64_t)ctx->n_sm ? 8 : 1);
+    walk = gw.n.x >= 3 && gw.n.y >= 3 && gw.n.z >= 3 && by_group > (lanes == 32 ? 1.2 : 2.4) * by_walk;
+    if (walk) grid[0] = grid[1] = gw;
+    // the walk of one list has one set of tables
+    if (walk && same) sides = 1;
     for (int s = 0; s < 2; ++s) {
       const std::vector<int32_t>& f = s ? fb : fa;
       fr[s] = f;
+      if (sides == 1) fr[s].insert(fr[s].end(), s ? fa.begin() : fb.begin(), s ? fa.end() : fb.end());
       std::sort(fr[s].begin(), fr[s].end());
       fr[s].erase(std::unique(fr[s].begin(), fr[s].end()), fr[s].end());
       for (int32_t x : f) slot[s].push_back((int32_t)(std::lower_bound(fr[s].begin(), fr[s].end(), x) - fr[s].begin()));
@@ -627,24 +722,10 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   p.n_bins = n_bins;
   p.counts = (unsigned long long*)(base + o_cnt);
   if (cells) {
-    // list 1: pencils as wide as the cube of 32 atoms, x cells an eighth of that (a quarter
-    // leaves the groups longer: 2 % slower); list 2: pencils of half the cutoff (a third:
-    // 5 % slower, more runs; the whole: 2 %), but wide enough for runs of about 16 atoms,
-    // x cells of half a pencil or two atoms
-    const double vol = (double)ctx->box[0] * ctx->box[1] * ctx->box[2];
-    const double edge = (double)std::max(ctx->box[0], std::max(ctx->box[1], ctx->box[2]));
-    const double w1 = std::cbrt(32.0 * vol / l1.n), rho2 = l2.n / vol;
-    const double f2 = std::max((double)max_distance / 2.0, std::sqrt(16.0 / (rho2 * (1.6 * max_distance + w1))));
-    // wrapped coordinates need not lie in the box (read from a file so, or rounded there
-    // from far unwrapped ones).  Up to an eighth of it the cells wrap and L - |d| is still
-    // the distance to the nearest image; beyond, the all-pairs pass gives the chain's value
-    const float tol = 0.125f * std::min(ctx->box[0], std::min(ctx->box[1], ctx->box[2]));
-    const PHGrid grid[2] = {make_grid(ctx, 0.125 * w1, w1, true, tol),
-                            make_grid(ctx, std::max(0.5 * f2, 2.0 / (f2 * f2 * rho2)), f2, false, tol)};
     const ListEntry* lists[2] = {&l1, &l2};
     size_t need = 0;
     size_t off[2][5];
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < sides; ++s) {
       const size_t nf = fr[s].size(), n = (size_t)lists[s]->n, nc1 = (size_t)grid[s].n_cells;
       off[s][0] = need; need = align(need + nf * n * 4);           // cell_of
       off[s][1] = need; need = align(need + nf * nc1 * 4);         // count
@@ -654,7 +735,7 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     }
     unsigned char* cb = ctx->scratch2.reserve(need);
     cudaStream_t st = ctx->stream;
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < sides; ++s) {
       const int nf = (int)fr[s].size();
       const PHList l = phview(*lists[s]);
       const PHGrid& gs = grid[s];
@@ -670,35 +751,39 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
       check_launch("pair cell lists");
       count_launch(ctx, 3);
     }
-    PHGroups G;
-    G.pos1 = (const float4*)(cb + off[0][4]);
-    G.n1 = l1.n;
-    G.pos2 = (const float4*)(cb + off[1][4]);
-    G.start2 = (const int32_t*)(cb + off[1][2]);
-    G.n2 = l2.n;
-    G.g2 = grid[1];
-    G.slot_a = (const int32_t*)(base + o_slot[0]);
-    G.slot_b = (const int32_t*)(base + o_slot[1]);
-    G.reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
-    G.same = &l1 == &l2 ? 1 : 0;
-    G.outside = (const int32_t*)(base + o_flag);
-    // up to eight groups per warp (one flush of the histograms for them) while the blocks
-    // fill the chip twice over
-    const int64_t groups = ceil_div(l1.n, 32);
-    G.per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups * (int64_t)n_q / ((int64_t)ctx->n_sm * 8 * PH_WARPS)));
     const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
-    auto launch = [&](auto kern) {
+    auto launch = [&](auto kern, const auto& view, int64_t blocks) {
       if (shm > 24 * 1024)
         AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
       KernelTimer kt(ctx, "pair_hist_cells_kernel");
-      kern<<<dim3((unsigned)ceil_div(groups, (int64_t)PH_WARPS * G.per_warp), (unsigned)n_q), PH_THREADS, shm, st>>>(p, G);
-      check_launch("pair_hist_groups_kernel");
+      kern<<<dim3((unsigned)blocks, (unsigned)n_q), PH_THREADS, shm, st>>>(p, view);
+      check_launch("pair_hist_cells_kernel");
       count_launch(ctx);
     };
-    // lists that may share atoms tell an atom's own pair by its index
-    const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
-    if (G.same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>);
-    else launch(pair_hist_groups_kernel<PH_SELF_IDS>);
+    const int t = sides - 1;  // list 2's tables
+    const float4 *pos1 = (const float4*)(cb + off[0][4]), *pos2 = (const float4*)(cb + off[t][4]);
+    const int32_t *start2 = (const int32_t*)(cb + off[t][2]), *slot_a = (const int32_t*)(base + o_slot[0]),
+                  *slot_b = (const int32_t*)(base + o_slot[1]), *far = (const int32_t*)(base + o_flag);
+    if (walk) {
+      KernelTimer kt(ctx, "pair_hist_walk_kernel");
+      const PHWalk W{pos1, l1.n, pos2, start2, l2.n, grid[1], slot_a, slot_b, far};
+      const int64_t blocks = ceil_div(l1.n, PH_THREADS / lanes);
+      if (lanes == 32) launch(pair_hist_walk_kernel<32>, W, blocks);
+      else if (lanes == 8) launch(pair_hist_walk_kernel<8>, W, blocks);
+      else launch(pair_hist_walk_kernel<1>, W, blocks);
+    } else {
+      // up to eight groups per warp (one flush of the histograms for them) while the blocks
+      // fill the chip twice over
+      const int64_t groups = ceil_div(l1.n, 32);
+      const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups * (int64_t)n_q / ((int64_t)ctx->n_sm * 8 * PH_WARPS)));
+      const float reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
+      const PHGroups G{pos1, l1.n, per_warp, pos2, start2, l2.n, grid[1], slot_a, slot_b, reach, same ? 1 : 0, far};
+      // lists that may share atoms tell an atom's own pair by its index
+      const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
+      const int64_t blocks = ceil_div(groups, (int64_t)PH_WARPS * per_warp);
+      if (same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>, G, blocks);
+      else launch(pair_hist_groups_kernel<PH_SELF_IDS>, G, blocks);
+    }
   }
   auto all_pairs = [&](const PHUnit* d_units) {
     const bool ids = fa != fb;

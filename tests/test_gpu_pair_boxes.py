@@ -1,5 +1,6 @@
 """The cell pass of ordered pair histograms in boxes that lie anywhere and with wrapped
-coordinates that are not quite in the box: the counts equal the all-pairs pass's."""
+coordinates that are not quite in the box, and lists too sparse for compact groups: the
+counts equal the all-pairs pass's."""
 import numpy as np
 import pytest
 
@@ -63,3 +64,38 @@ def test_vhd_cells_many_cells(eng, monkeypatch, n, box, max_d):
         got = eng.vhd(l1, l2, max_d, 30)
         monkeypatch.setenv("AMDAT_PAIR_CELLS", "off")
         np.testing.assert_array_equal(got, eng.vhd(l1, l2, max_d, 30))
+
+
+@pytest.mark.parametrize("frames,n1,max_d,walk", [(2, 2, 3.0, True), (2, 33, 5.0, True), (40, 200, 1.5, True),
+                                                  (40, 1100, 1.1, True), (2, 30000, 5.0, False), (2, 1, 5.0, False)])
+def test_vhd_few_atoms_to_many(eng, monkeypatch, frames, n1, max_d, walk):
+    """A few atoms among many (32, 8 and 1 lanes each) walk the cells around them: groups of
+    atoms far apart would gather the whole box."""
+    rng = np.random.default_rng(n1)
+    n, L = 30000, 33.0
+    u = (rng.random((1, n, 3)) * L + np.cumsum(rng.normal(0, 0.05, (frames, n, 3)), 0)).astype(np.float32)
+    eng.upload(u, [L] * 3)
+    eng.set_scheme(synth.TimeScheme.linear(frames, 1.0))
+    perm = rng.permutation(n)
+    few, rest = eng.list(np.sort(perm[:n1])), eng.list(np.sort(perm[min(n1, n - 2000):]))
+    for l2 in (rest, 0):
+        eng.profile_reset()
+        eng.vhd(few, l2, max_d, 40)
+        assert (eng.profile_kernel("pair_hist_walk_kernel")[0] == 1) == walk or l2 != 0
+        got, want = _both(eng, monkeypatch, few, l2, max_d, 40)
+        np.testing.assert_array_equal(got, want)
+
+
+def test_vhd_walk_of_one_list(eng, monkeypatch):
+    """One list on both sides: its frames are sorted once; no atom pairs with itself."""
+    rng = np.random.default_rng(5)
+    n, L = 30000, 54.5
+    u = (rng.random((1, n, 3)) * L + np.cumsum(rng.normal(0, 0.1, (2, n, 3)), 0)).astype(np.float32)
+    eng.upload(u, [L] * 3)
+    eng.set_scheme(synth.TimeScheme.linear(2, 1.0))
+    for lst in (0, eng.list(np.arange(0, n, 2))):
+        eng.profile_reset()
+        eng.vhd(lst, lst, 2.0, 26)
+        assert eng.profile_kernel("pair_hist_walk_kernel")[0] == 1
+        got, want = _both(eng, monkeypatch, lst, lst, 2.0, 26)
+        np.testing.assert_array_equal(got, want)
