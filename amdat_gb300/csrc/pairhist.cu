@@ -18,6 +18,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <numeric>
+#include <utility>
 #include <vector>
 
 #include "engine.h"
@@ -608,6 +610,17 @@ static std::vector<PHUnit> pair_units(const amdat_ctx* ctx, int n1, int n2, bool
   return units;
 }
 
+// Cell tables of all frames of both sides stay within this many bytes (AMDAT_PAIR_SCRATCH_MB);
+// beyond, the rows run in batches of frames.
+constexpr size_t PH_TABLE_BYTES = (size_t)4 << 30;
+
+// rows [row0, row0 + rows) of the reordered row tables: their frames are the distinct frames
+// f0[s] .. f0[s] + nf[s] of each side
+struct PHBatch {
+  int32_t f0[2], nf[2];
+  size_t row0, rows;
+};
+
 static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& l2, bool symmetric,
                           const std::vector<int32_t>& fa, const std::vector<int32_t>& fb,
                           const std::vector<int32_t>& row, int32_t n_rows_out, float max_distance,
@@ -636,11 +649,13 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     if (bytes) std::memcpy(host.data() + at, v.data(), bytes);
     return at;
   };
-  const size_t o_fa = table(fa), o_fb = table(fb), o_row = table(row);
+  std::vector<int32_t> qa = fa, qb = fb, qrow = row;  // the rows, in the batches' order
   std::vector<int32_t> fr[2], slot[2];  // the distinct frames of each side and each row's place among them
   size_t o_fr[2] = {0, 0}, o_slot[2] = {0, 0}, o_units = 0;
   std::vector<PHUnit> units;
   int per_thread = 1;
+  std::vector<PHBatch> batches;
+  const ListEntry* lists[2] = {&l1, &l2};
   PHGrid grid[2];
   bool walk = false;
   int lanes = 1;  // of the walk, per list-1 member
@@ -681,15 +696,49 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     lanes = members <= 512 * (int64_t)ctx->n_sm ? 32 : (members <= 2048 * (int64_t)ctx->n_sm ? 8 : 1);
     walk = gw.n.x >= 3 && gw.n.y >= 3 && gw.n.z >= 3 && by_group > (lanes == 32 ? 1.2 : 2.4) * by_walk;
     if (walk) grid[0] = grid[1] = gw;
-    // the walk of one list has one set of tables
-    if (walk && same) sides = 1;
+    auto per_frame = [&](int s) { return (size_t)lists[s]->n * 20 + (size_t)grid[s].n_cells * 12 + 4; };
+    auto distinct = [](std::vector<int32_t> f) {
+      std::sort(f.begin(), f.end());
+      f.erase(std::unique(f.begin(), f.end()), f.end());
+      return f;
+    };
+    const char* mb = std::getenv("AMDAT_PAIR_SCRATCH_MB");
+    const size_t most = mb ? (size_t)std::max(0, std::atoi(mb)) << 20 : PH_TABLE_BYTES;
+    fr[0] = distinct(fa), fr[1] = distinct(fb);
+    if (walk && same) {  // the walk of one list has one set of tables
+      std::vector<int32_t> both = fr[0];
+      both.insert(both.end(), fr[1].begin(), fr[1].end());
+      both = distinct(both);
+      if (both.size() * per_frame(0) <= most) sides = 1, fr[0] = fr[1] = both;
+    }
+    for (int s = 0; s < 2; ++s)
+      for (int32_t x : s ? fb : fa)
+        slot[s].push_back((int32_t)(std::lower_bound(fr[s].begin(), fr[s].end(), x) - fr[s].begin()));
+    // frames per batch and side: all, or what half of the limit holds
+    int32_t step[2] = {(int32_t)fr[0].size(), (int32_t)fr[1].size()};
+    if (sides == 2 && fr[0].size() * per_frame(0) + fr[1].size() * per_frame(1) > most) {
+      for (int s = 0; s < 2; ++s) step[s] = (int32_t)std::max<size_t>(1, std::min<size_t>(fr[s].size(), most / 2 / per_frame(s)));
+      std::vector<int32_t> order(n_q);
+      std::iota(order.begin(), order.end(), 0);
+      auto batch = [&](int32_t q) { return std::make_pair(slot[0][q] / step[0], slot[1][q] / step[1]); };
+      std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return batch(x) < batch(y); });
+      auto reorder = [&](std::vector<int32_t>& v) {
+        const std::vector<int32_t> old = v;
+        for (size_t i = 0; i < n_q; ++i) v[i] = old[order[i]];
+      };
+      for (std::vector<int32_t>* v : {&qa, &qb, &qrow, &slot[0], &slot[1]}) reorder(*v);
+    }
+    for (size_t i = 0; i < n_q; ++i) {
+      const int32_t f0[2] = {slot[0][i] / step[0] * step[0], slot[1][i] / step[1] * step[1]};
+      if (batches.empty() || batches.back().f0[0] != f0[0] || batches.back().f0[1] != f0[1]) {
+        PHBatch B{{f0[0], f0[1]}, {0, 0}, i, 0};
+        for (int s = 0; s < 2; ++s) B.nf[s] = std::min<int32_t>(step[s], (int32_t)fr[s].size() - f0[s]);
+        batches.push_back(B);
+      }
+      ++batches.back().rows;
+      for (int s = 0; s < 2; ++s) slot[s][i] -= f0[s];
+    }
     for (int s = 0; s < 2; ++s) {
-      const std::vector<int32_t>& f = s ? fb : fa;
-      fr[s] = f;
-      if (sides == 1) fr[s].insert(fr[s].end(), s ? fa.begin() : fb.begin(), s ? fa.end() : fb.end());
-      std::sort(fr[s].begin(), fr[s].end());
-      fr[s].erase(std::unique(fr[s].begin(), fr[s].end()), fr[s].end());
-      for (int32_t x : f) slot[s].push_back((int32_t)(std::lower_bound(fr[s].begin(), fr[s].end(), x) - fr[s].begin()));
       o_fr[s] = table(fr[s]);
       o_slot[s] = table(slot[s]);
     }
@@ -697,6 +746,7 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     units = pair_units(ctx, l1.n, l2.n, symmetric, (int64_t)n_q, &per_thread);
     o_units = table(units);
   }
+  const size_t o_fa = table(qa), o_fb = table(qb), o_row = table(qrow);
   const size_t o_flag = host.size(), o_cnt = align(o_flag + 4);
   unsigned char* base = ctx->scratch.reserve(o_cnt + n_out * 8);
   if (!host.empty()) AMDAT_CUDA(cudaMemcpyAsync(base, host.data(), host.size(), cudaMemcpyHostToDevice, ctx->stream));
@@ -722,11 +772,12 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
   p.n_bins = n_bins;
   p.counts = (unsigned long long*)(base + o_cnt);
   if (cells) {
-    const ListEntry* lists[2] = {&l1, &l2};
     size_t need = 0;
     size_t off[2][5];
     for (int s = 0; s < sides; ++s) {
-      const size_t nf = fr[s].size(), n = (size_t)lists[s]->n, nc1 = (size_t)grid[s].n_cells;
+      size_t nf = 0;
+      for (const PHBatch& B : batches) nf = std::max(nf, (size_t)B.nf[s]);
+      const size_t n = (size_t)lists[s]->n, nc1 = (size_t)grid[s].n_cells;
       off[s][0] = need; need = align(need + nf * n * 4);           // cell_of
       off[s][1] = need; need = align(need + nf * nc1 * 4);         // count
       off[s][2] = need; need = align(need + nf * (nc1 + 1) * 4);   // start
@@ -735,54 +786,62 @@ static void run_pair_hist(amdat_ctx* ctx, const ListEntry& l1, const ListEntry& 
     }
     unsigned char* cb = ctx->scratch2.reserve(need);
     cudaStream_t st = ctx->stream;
-    for (int s = 0; s < sides; ++s) {
-      const int nf = (int)fr[s].size();
+    int32_t *far = (int32_t*)(base + o_flag), at[2] = {-1, -1};  // at: first frame of the tables in place
+    auto build = [&](int s, const PHBatch& B) {
+      if (at[s] == B.f0[s]) return;
+      at[s] = B.f0[s];
+      const int nf = B.nf[s];
       const PHList l = phview(*lists[s]);
       const PHGrid& gs = grid[s];
-      const int32_t* frames = (const int32_t*)(base + o_fr[s]);
+      const int32_t* frames = (const int32_t*)(base + o_fr[s]) + B.f0[s];
       AMDAT_CUDA(cudaMemsetAsync(cb + off[s][1], 0, (size_t)nf * gs.n_cells * 4, st));
       const dim3 gn((unsigned)ceil_div(l.n, 256), (unsigned)nf);
       ph_cell_count_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, frames, gs, (int32_t*)(cb + off[s][0]),
-                                               (int32_t*)(cb + off[s][1]), (int32_t*)(base + o_flag));
+                                               (int32_t*)(cb + off[s][1]), far);
       ph_cell_scan_kernel<<<(unsigned)nf, PS_THREADS, 0, st>>>((const int32_t*)(cb + off[s][1]), gs.n_cells,
                                                                (int32_t*)(cb + off[s][2]), (int32_t*)(cb + off[s][3]));
       ph_cell_scatter_kernel<<<gn, 256, 0, st>>>(p.w, p.n_pad, l, frames, gs.n_cells, (const int32_t*)(cb + off[s][0]),
                                                  (int32_t*)(cb + off[s][3]), (float4*)(cb + off[s][4]));
       check_launch("pair cell lists");
       count_launch(ctx, 3);
-    }
-    const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
-    auto launch = [&](auto kern, const auto& view, int64_t blocks) {
-      if (shm > 24 * 1024)
-        AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-      KernelTimer kt(ctx, "pair_hist_cells_kernel");
-      kern<<<dim3((unsigned)blocks, (unsigned)n_q), PH_THREADS, shm, st>>>(p, view);
-      check_launch("pair_hist_cells_kernel");
-      count_launch(ctx);
     };
+    const size_t shm = (size_t)PH_WARPS * (n_bins + 1) * 4;
     const int t = sides - 1;  // list 2's tables
     const float4 *pos1 = (const float4*)(cb + off[0][4]), *pos2 = (const float4*)(cb + off[t][4]);
-    const int32_t *start2 = (const int32_t*)(cb + off[t][2]), *slot_a = (const int32_t*)(base + o_slot[0]),
-                  *slot_b = (const int32_t*)(base + o_slot[1]), *far = (const int32_t*)(base + o_flag);
-    if (walk) {
-      KernelTimer kt(ctx, "pair_hist_walk_kernel");
-      const PHWalk W{pos1, l1.n, pos2, start2, l2.n, grid[1], slot_a, slot_b, far};
-      const int64_t blocks = ceil_div(l1.n, PH_THREADS / lanes);
-      if (lanes == 32) launch(pair_hist_walk_kernel<32>, W, blocks);
-      else if (lanes == 8) launch(pair_hist_walk_kernel<8>, W, blocks);
-      else launch(pair_hist_walk_kernel<1>, W, blocks);
-    } else {
-      // up to eight groups per warp (one flush of the histograms for them) while the blocks
-      // fill the chip twice over
-      const int64_t groups = ceil_div(l1.n, 32);
-      const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups * (int64_t)n_q / ((int64_t)ctx->n_sm * 8 * PH_WARPS)));
-      const float reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
-      const PHGroups G{pos1, l1.n, per_warp, pos2, start2, l2.n, grid[1], slot_a, slot_b, reach, same ? 1 : 0, far};
-      // lists that may share atoms tell an atom's own pair by its index
-      const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
-      const int64_t blocks = ceil_div(groups, (int64_t)PH_WARPS * per_warp);
-      if (same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>, G, blocks);
-      else launch(pair_hist_groups_kernel<PH_SELF_IDS>, G, blocks);
+    const int32_t* start2 = (const int32_t*)(cb + off[t][2]);
+    const float reach = (float)(max_distance * (1.0 + 1e-5) + 2.0 * std::max(1e-4 * max_distance, 2e-6 * edge));
+    // lists that may share atoms tell an atom's own pair by its index
+    const bool apart = l1.contiguous && l2.contiguous && (l1.first + l1.n <= l2.first || l2.first + l2.n <= l1.first);
+    for (const PHBatch& B : batches) {
+      for (int s = 0; s < sides; ++s) build(s, B);
+      PHParams pb = p;
+      pb.frame_a += B.row0, pb.frame_b += B.row0, pb.row_of += B.row0;
+      const int32_t *slot_a = (const int32_t*)(base + o_slot[0]) + B.row0, *slot_b = (const int32_t*)(base + o_slot[1]) + B.row0;
+      auto launch = [&](auto kern, const auto& view, int64_t blocks) {
+        if (shm > 24 * 1024)
+          AMDAT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+        KernelTimer kt(ctx, "pair_hist_cells_kernel");
+        kern<<<dim3((unsigned)blocks, (unsigned)B.rows), PH_THREADS, shm, st>>>(pb, view);
+        check_launch("pair_hist_cells_kernel");
+        count_launch(ctx);
+      };
+      if (walk) {
+        KernelTimer kt(ctx, "pair_hist_walk_kernel");
+        const PHWalk W{pos1, l1.n, pos2, start2, l2.n, grid[1], slot_a, slot_b, far};
+        const int64_t blocks = ceil_div(l1.n, PH_THREADS / lanes);
+        if (lanes == 32) launch(pair_hist_walk_kernel<32>, W, blocks);
+        else if (lanes == 8) launch(pair_hist_walk_kernel<8>, W, blocks);
+        else launch(pair_hist_walk_kernel<1>, W, blocks);
+      } else {
+        // up to eight groups per warp (one flush of the histograms for them) while the blocks
+        // fill the chip twice over
+        const int64_t groups = ceil_div(l1.n, 32);
+        const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(8, groups * (int64_t)B.rows / ((int64_t)ctx->n_sm * 8 * PH_WARPS)));
+        const PHGroups G{pos1, l1.n, per_warp, pos2, start2, l2.n, grid[1], slot_a, slot_b, reach, same ? 1 : 0, far};
+        const int64_t blocks = ceil_div(groups, (int64_t)PH_WARPS * per_warp);
+        if (same || apart) launch(pair_hist_groups_kernel<PH_SELF_LATER>, G, blocks);
+        else launch(pair_hist_groups_kernel<PH_SELF_IDS>, G, blocks);
+      }
     }
   }
   auto all_pairs = [&](const PHUnit* d_units) {

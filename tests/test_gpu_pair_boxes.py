@@ -99,3 +99,41 @@ def test_vhd_walk_of_one_list(eng, monkeypatch):
         assert eng.profile_kernel("pair_hist_walk_kernel")[0] == 1
         got, want = _both(eng, monkeypatch, lst, lst, 2.0, 26)
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("mb", [0, 1, 3])
+@pytest.mark.parametrize("max_d", [1.0, 3.0])
+def test_vhd_cells_in_batches_of_frames(eng, monkeypatch, mb, max_d):
+    """Cell tables over the limit: the time pairs run in batches of frames, one frame of
+    each side at least, and give the same counts."""
+    rng = np.random.default_rng(mb)
+    n, L, T = 9000, 24.0, 11
+    u = (rng.random((1, n, 3)) * L + np.cumsum(rng.normal(0, 0.1, (T, n, 3)), 0)).astype(np.float32)
+    eng.upload(u, [L] * 3)
+    eng.set_scheme(synth.TimeScheme.linear(T, 1.0))
+    half, few = eng.list(np.arange(0, n, 2)), eng.list(np.arange(7, n, 300))
+    for l1, l2 in ((0, 0), (half, 0), (few, 0), (half, half)):
+        monkeypatch.delenv("AMDAT_PAIR_SCRATCH_MB", raising=False)
+        eng.profile_reset()
+        want = eng.vhd(l1, l2, max_d, 40)
+        assert eng.profile_kernel("pair_hist_cells_kernel")[0] == 1 and want.sum() > 0
+        monkeypatch.setenv("AMDAT_PAIR_SCRATCH_MB", str(mb))
+        eng.profile_reset()
+        np.testing.assert_array_equal(eng.vhd(l1, l2, max_d, 40), want)
+        assert mb == 3 or eng.profile_kernel("pair_hist_cells_kernel")[0] > 1
+
+
+def test_vhd_cells_scratch_is_bounded(engine_mod, monkeypatch):
+    import torch
+    monkeypatch.setenv("AMDAT_PAIR_SCRATCH_MB", "64")
+    rng = np.random.default_rng(1)
+    n, L, T = 200000, 62.0, 40
+    eng = engine_mod.Engine(0)
+    try:
+        eng.upload((rng.random((1, n, 3)) * L + rng.normal(0, 0.1, (T, n, 3))).astype(np.float32), [L] * 3)
+        eng.set_scheme(synth.TimeScheme.linear(T, 1.0))
+        free = torch.cuda.mem_get_info()[0]
+        eng.vhd(0, 0, 1.5, 40)
+        assert free - torch.cuda.mem_get_info()[0] < 100 << 20
+    finally:
+        eng.close()
