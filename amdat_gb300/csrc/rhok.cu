@@ -401,40 +401,62 @@ static void run_list_density(amdat_ctx* ctx, Density& d, float period, int32_t p
     // as many vectors per thread as fill a block (four share each staged atom); atom
     // segments until about 24 blocks per SM even out what the SMs get.  5,085 vectors x
     // 100 frames are 500 blocks, four on some SMs and three on the others: 20.7 ms for
-    // 32,000 atoms, 17.5 ms in segments, 16.2 ms with two atoms in flight per vector.  Short lists gain more: of 85 vectors one warp in
-    // eight was busy
-    const int kpt = d.n_k > 2 * RL_THREADS ? 4 : (d.n_k > RL_THREADS ? 2 : 1);
-    const int threads = d.n_k > 128 ? RL_THREADS : (d.n_k > 64 ? 128 : 64);
-    const int64_t kb = ceil_div(d.n_k, (int64_t)threads * kpt);
+    // 32,000 atoms, 17.5 ms in segments, 16.2 ms with two atoms in flight per vector.  Short
+    // lists gain more: of 85 vectors one warp in eight was busy
+    struct Shape {
+      int kpt, threads;
+      int64_t blocks, want;
+    };
+    auto shape = [&](int32_t n) {
+      Shape s{n > 2 * RL_THREADS ? 4 : (n > RL_THREADS ? 2 : 1), n > 128 ? RL_THREADS : (n > 64 ? 128 : 64), 0, 0};
+      s.blocks = ceil_div(n, (int64_t)s.threads * s.kpt);
+      s.want = (int64_t)24 * ctx->n_sm * (RL_THREADS / s.threads);
+      return s;
+    };
     const int64_t folds = ceil_div(e.n, RL_FOLD);
-    const int64_t want = (int64_t)24 * ctx->n_sm * (RL_THREADS / threads);
-    // frame batches keep the folds' sums within 96 MB (they stay in L2 on their way)
-    const size_t fold_bytes = (size_t)folds * d.n_k * sizeof(float2);
-    const bool split = folds > 1 && kb * d.n_frames < want;
-    const int32_t batch = split ? (int32_t)std::max<size_t>(1, std::min<size_t>(d.n_frames, (size_t)(96u << 20) / fold_bytes)) : d.n_frames;
-    const int64_t segs = split ? std::min(folds, ceil_div(want, kb * batch)) : 1;
-    const int seg = (int)(ceil_div(folds, segs) * RL_FOLD);
-    float2* part = split ? (float2*)ctx->scratch.reserve(fold_bytes * batch) : nullptr;
-    for (int32_t f0 = 0; f0 < d.n_frames; f0 += batch) {
-      const int32_t nb = std::min(batch, d.n_frames - f0);
-      float2* rho = d.rho->ptr + (int64_t)f0 * d.n_k;
-      const dim3 grid((unsigned)kb, (unsigned)nb, (unsigned)ceil_div(e.n, seg));
-      auto launch = [&](auto kern) {
-        KernelTimer kt(ctx, "rhok_list_kernel");
-        kern<<<grid, threads, 0, ctx->stream>>>(fx + (int64_t)f0 * e.n, e.n, kv.ptr, d.n_k, seg, rho, part);
-        check_launch("rhok_list_kernel");
-        count_launch(ctx);
-      };
-      if (split) kpt == 4 ? launch(rhok_list_kernel<4, true>) : kpt == 2 ? launch(rhok_list_kernel<2, true>) : launch(rhok_list_kernel<1, true>);
-      else kpt == 4 ? launch(rhok_list_kernel<4, false>) : kpt == 2 ? launch(rhok_list_kernel<2, false>) : launch(rhok_list_kernel<1, false>);
-      if (split) {
-        const int64_t n_out = (int64_t)nb * d.n_k;
-        rhok_list_merge_kernel<<<(unsigned)ceil_div(n_out, 256), 256, 0, ctx->stream>>>(
-            part, e.n / RL_FOLD, e.n % RL_FOLD ? 1 : 0, n_out, rho);
-        check_launch("rhok_list_merge_kernel");
-        count_launch(ctx);
+    const Shape all = shape(d.n_k);
+    bool split = folds > 1 && all.blocks * d.n_frames < all.want;
+    // the folds' sums stay within 96 MB by batches of frames (in L2 on their way); one frame's
+    // may take 1 GB, beyond that even batches of vectors (400,000 atoms x 20,000 vectors, one
+    // frame, 500 MB: 8.6 ms, 10.3 in six batches of 96 MB; 75.7 without segments)
+    const size_t vector_bytes = (size_t)folds * sizeof(float2);
+    int32_t nf = d.n_frames, nk = d.n_k;  // of a batch
+    if (split) {
+      nf = (int32_t)std::max<size_t>(1, std::min<size_t>(d.n_frames, ((size_t)96 << 20) / (vector_bytes * d.n_k)));
+      const size_t fit = ((size_t)1 << 30) / vector_bytes;
+      if (fit < (size_t)d.n_k) {
+        const int64_t unit = fit >= RL_TILE ? RL_TILE : 64;
+        const int64_t n = ceil_div(d.n_k, (int64_t)std::max<size_t>(1, fit / unit * unit));
+        nk = (int32_t)(ceil_div(ceil_div(d.n_k, n), unit) * unit);
+        if (fit < 64) split = false, nk = d.n_k, nf = d.n_frames;  // (beyond 268 million atoms)
       }
     }
+    float2* part = split ? (float2*)ctx->scratch.reserve(vector_bytes * nk * nf) : nullptr;
+    for (int32_t f0 = 0; f0 < d.n_frames; f0 += nf)
+      for (int32_t k0 = 0; k0 < d.n_k; k0 += nk) {  // (vector batches come with one frame)
+        const int32_t nb = std::min(nf, d.n_frames - f0), kn = std::min(nk, d.n_k - k0);
+        const Shape sh = shape(kn);
+        const int64_t segs = split ? std::min(folds, ceil_div(sh.want, sh.blocks * nf)) : 1;
+        const int seg = (int)(ceil_div(folds, segs) * RL_FOLD);
+        float2* rho = d.rho->ptr + (int64_t)f0 * d.n_k + k0;
+        const dim3 grid((unsigned)sh.blocks, (unsigned)nb, (unsigned)ceil_div(e.n, seg));
+        auto launch = [&](auto kern) {
+          KernelTimer kt(ctx, "rhok_list_kernel");
+          kern<<<grid, sh.threads, 0, ctx->stream>>>(fx + (int64_t)f0 * e.n, e.n, kv.ptr + k0, kn, seg, rho, part);
+          check_launch("rhok_list_kernel");
+          count_launch(ctx);
+        };
+        const int kpt = sh.kpt;
+        if (split) kpt == 4 ? launch(rhok_list_kernel<4, true>) : kpt == 2 ? launch(rhok_list_kernel<2, true>) : launch(rhok_list_kernel<1, true>);
+        else kpt == 4 ? launch(rhok_list_kernel<4, false>) : kpt == 2 ? launch(rhok_list_kernel<2, false>) : launch(rhok_list_kernel<1, false>);
+        if (split) {
+          const int64_t n_out = (int64_t)nb * kn;
+          rhok_list_merge_kernel<<<(unsigned)ceil_div(n_out, 256), 256, 0, ctx->stream>>>(
+              part, e.n / RL_FOLD, e.n % RL_FOLD ? 1 : 0, n_out, rho);
+          check_launch("rhok_list_merge_kernel");
+          count_launch(ctx);
+        }
+      }
   }
   AMDAT_CUDA(cudaStreamSynchronize(ctx->stream));
 }
