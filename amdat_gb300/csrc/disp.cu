@@ -1131,6 +1131,7 @@ struct amdat_disp_plan {
   std::vector<int32_t> lu_off, lu_units;  // list -> its units (CSR, ascending)
   amdat::DevBuf<int32_t> class_idx;       // atoms of gathered classes
   int chunk = 0, blocks_per_sm = 0, n_items = 0;
+  int pair_chunk = 0;  // members of an item of several pairs
   int64_t steps1 = 0, steps2 = 0;  // block steps of the items with one and with two atoms per F_s thread
   double tuned_ms = 0.0;
   bool slab = false;  // moments of gathered units together, by slabs of members in atom order
@@ -1172,7 +1173,7 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
   std::vector<int32_t> item_first(n_ug + 1, 0);
   size_t n_rows = 0;         // rows of partials
   std::vector<int64_t> key;  // schedule key per item: (unit, chunk, pair)
-  // moments-only passes give a unit smaller than half a chunk several pairs
+  // moments-only passes give a unit smaller than half of pair_chunk several pairs
   // of one gap per item (the finalize sums a (unit, gap)'s items anyway), so
   // small lists do not pay one item's fixed cost per pair
   const bool multi_pair = pl.S == 0 && pl.NB == 0;
@@ -1198,8 +1199,8 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
   }
   for (int u = 0; u < pl.n_units && !pl.slab; ++u) {
     const int nch = (int)std::max<int64_t>(1, ceil_div(pl.usize[u], chunk));
-    const int ppi = (multi_pair && pl.usize[u] > 0 && 2 * pl.usize[u] <= chunk)
-                        ? std::min(MAX_PAIRS_PER_ITEM, chunk / pl.usize[u])
+    const int ppi = (multi_pair && pl.usize[u] > 0 && 2 * pl.usize[u] <= pl.pair_chunk)
+                        ? std::min(MAX_PAIRS_PER_ITEM, pl.pair_chunk / pl.usize[u])
                         : 1;
     for (int g = 0; g < G; ++g) {
       item_first[(size_t)u * G + g] = (int32_t)items.size();
@@ -1673,11 +1674,12 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     // 500,000 x 1,226 957 / 676, 1,558 / 1,072; 200,000 x 427 176 / 150, 298 / 257; a third
     // of those 200,000 atoms, gathered (196 MB of sectors), 155 / 152, 214 / 232.  32,000
     // atoms x 187 pairs in 2,460 / 4,096 / 8,192 25 / 20 / 23, 42 / 36 / 42.
-    // F_s is compute bound and keeps smaller chunks; so do several small units, whose sums
-    // of a few terms per thread depend on the items' cut.
+    // F_s is compute bound and keeps smaller chunks; so do small units, whose sums of a few
+    // terms per thread depend on the items' cut.
     int64_t chunk = DISP_CHUNK;
     if (P.n_pairs > 0 && unit_atoms > 0) {
-      if (pl->S || pl->bulk || (pl->n_units > 1 && mean_size(pl->usize) < SLAB_MEAN)) {
+      const int32_t largest = *std::max_element(pl->usize.begin(), pl->usize.end());
+      if (pl->S || pl->bulk || largest <= DISP_CHUNK || (pl->n_units > 1 && mean_size(pl->usize) < SLAB_MEAN)) {
         const int64_t want_items = (int64_t)ctx->n_sm * 16;
         chunk = std::max<int64_t>(pl->S ? 128 : 1024,
                                   std::min<int64_t>(DISP_CHUNK, ceil_div(unit_atoms * P.n_pairs, want_items)));
@@ -1694,6 +1696,10 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       }
     }
     if (pl->slab) chunk = SLAB_ENTRIES;  // its one tile
+    // larger chunks are for large units: an item of several pairs gathers its members one by
+    // one, where an item of one pair reads contiguous ones four at a time (4,000 atoms x
+    // 20,000 pairs: 224 us with four pairs per item, 161 with one)
+    pl->pair_chunk = (int)std::min<int64_t>(chunk, DISP_CHUNK);
     // list-mode F_s holds few registers and only its vectors in shared memory:
     // more resident blocks hide the latency of its cosine chain
     int bps = pl->S ? (pl->sh.mode == 1 ? 8 : 4) : 8;
@@ -1704,7 +1710,7 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     const std::string key(keybuf);
     auto hit = tune_cache().find(key);
     if (hit != tune_cache().end()) {
-      chunk = hit->second.first;
+      chunk = pl->pair_chunk = hit->second.first;
       bps = hit->second.second;
     } else if (flags & AMDAT_PLAN_AUTOTUNE) {
       // time each candidate (warm-up + 3 runs, CUDA events) and keep the fastest
@@ -1723,6 +1729,7 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       int bc = (int)chunk, bb = bps;
       for (int c : chunks) {
         for (int bp : bpss) {
+          pl->pair_chunk = c;
           plan_tables(ctx, *pl, P, c, bp);
           plan_launch(ctx, *pl, P);
           AMDAT_CUDA(cudaEventRecord(a, ctx->stream));
@@ -1740,7 +1747,7 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
       }
       cudaEventDestroy(a);
       cudaEventDestroy(b);
-      chunk = bc;
+      chunk = pl->pair_chunk = bc;
       bps = bb;
       pl->tuned_ms = best;
       tune_store(key, bc, bb, best);

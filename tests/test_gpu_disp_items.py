@@ -1,0 +1,32 @@
+"""Items of the moments passes: units of up to 4,096 members keep items of at most 4,096
+members, several pairs to an item only for units of half of that; larger units take
+longer items but never several pairs in one.  The sums are the oracle's to 1e-6."""
+import numpy as np
+import pytest
+
+from amdat_gb300 import engine as E
+from amdat_gb300 import synth
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,frames,chunk,per_item", [(500, 60, 1024, 2), (1000, 200, 4096, 4), (2049, 200, 4096, 1),
+                                                     (4000, 200, 4096, 1), (5000, 200, 16384, 1), (8192, 200, 16384, 1)])
+def test_items_of_one_unit(eng, n, frames, chunk, per_item):
+    sc = synth.TimeScheme.linear(frames, 1.0)
+    traj = synth.random_walk(n, 15.0, sc, 0.3, seed=n, time_scaled=False)
+    eng.upload(traj.unwrapped, traj.box)
+    eng.set_scheme(sc)
+    gaps = np.bincount(E.scheme_pairs(eng.scheme)[0])
+    plan = eng.plan([0])
+    info = plan.info()
+    assert info["chunk"] == chunk
+    assert info["n_items"] == (-(-gaps // per_item)).sum()  # one chunk of members each
+    plan.run()
+    out = plan.read()
+    d2, d4, cnt = orc.disp_moments(orc.scheme(sc), traj.unwrapped, np.arange(n, dtype=np.int32), 0)
+    np.testing.assert_array_equal(out["atom_pairs"][0], cnt)
+    np.testing.assert_allclose(out["sum_d2"][0], d2, rtol=1e-6, atol=1e-12)
+    np.testing.assert_allclose(out["sum_d4"][0], d4, rtol=1e-6, atol=1e-14)
+    plan.close()
