@@ -1130,6 +1130,7 @@ struct amdat_disp_plan {
   std::vector<amdat::ListDev> udev;
   std::vector<int32_t> lu_off, lu_units;  // list -> its units (CSR, ascending)
   amdat::DevBuf<int32_t> class_idx;       // atoms of gathered classes
+  std::vector<int32_t> class_host;        // class_idx while the plan is made
   int chunk = 0, blocks_per_sm = 0, n_items = 0;
   int pair_chunk = 0;  // members of an item of several pairs
   int64_t steps1 = 0, steps2 = 0;  // block steps of the items with one and with two atoms per F_s thread
@@ -1530,6 +1531,7 @@ static void plan_classes(amdat_ctx* ctx, amdat_disp_plan& pl, const int32_t* lis
     for (int l = 0; l < L; ++l)
       if (mask[(size_t)rep * words + l / 64] >> (l % 64) & 1ull) per_list[l].push_back(c);
   }
+  pl.class_host = std::move(members);
   pl.lu_off.assign(L + 1, 0);
   pl.lu_units.clear();
   for (int l = 0; l < L; ++l) {
@@ -1560,32 +1562,39 @@ static double mean_size(const std::vector<int32_t>& sizes) {
 // order, per slab the units' runs there.
 static void plan_slabs(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P) {
   const int64_t N = ctx->n_atoms;
-  std::vector<std::vector<int32_t>> idx(pl.n_units);
-  std::vector<int64_t> at(N + 1, 0);  // first entry of each atom
-  double by_unit = 0.0;               // time of the units one by one, in entries of the slab kernel
   int64_t n = 0;
+  bool gathered = false;
+  for (int u = 0; u < pl.n_units; ++u) {
+    n += pl.usize[u];
+    gathered = gathered || pl.udev[u].idx;
+  }
+  if (!gathered || n == 0) return;
+  // Few pairs and lists that are small on average stay with the units' kernel: its sums are
+  // not error-free (each thread adds its terms by Kahan's scheme, a few in no order of
+  // size), and there the slabs' exact sums differ from them by up to 2e-9, from these sizes
+  // on by less than 6e-10 (as measured; a small list beside large ones does take slabs).
+  if (P.n_pairs < SLAB_PAIRS || mean_size(pl.lsize) < SLAB_MEAN) return;
+  const int64_t slabs = ceil_div(n, SLAB_ENTRIES);
+  const int64_t rows = pl.n_units * slabs * (pl.G + P.n_pairs / slab_pairs(ctx, P.n_pairs, slabs));
+  if (rows > SLAB_ROWS) return;
+  std::vector<std::vector<int32_t>> idx(pl.n_units);
+  double by_unit = 0.0;  // time of the units one by one, in entries of the slab kernel
   for (int u = 0; u < pl.n_units; ++u) {
     const ListDev& L = pl.udev[u];
     idx[u].resize(pl.usize[u]);
-    if (L.idx)
-      AMDAT_CUDA(cudaMemcpy(idx[u].data(), L.idx, (size_t)pl.usize[u] * 4, cudaMemcpyDeviceToHost));
-    else
-      std::iota(idx[u].begin(), idx[u].end(), L.first);
-    n += pl.usize[u];
     if (!L.idx) {
+      std::iota(idx[u].begin(), idx[u].end(), L.first);
       by_unit += 0.75 * pl.usize[u];
     } else if (pl.usize[u]) {
+      if (pl.classes)
+        std::copy_n(pl.class_host.begin() + (L.idx - pl.class_idx.ptr), pl.usize[u], idx[u].begin());
+      else
+        AMDAT_CUDA(cudaMemcpy(idx[u].data(), L.idx, (size_t)pl.usize[u] * 4, cudaMemcpyDeviceToHost));
       by_unit += 0.55 * (idx[u].back() - idx[u].front() + 1);  // lists are ascending
     }
   }
-  const int64_t slabs = ceil_div(n, SLAB_ENTRIES);
-  const int64_t rows = n ? pl.n_units * slabs * (pl.G + P.n_pairs / slab_pairs(ctx, P.n_pairs, slabs)) : 0;
-  if (by_unit <= (double)n || rows > SLAB_ROWS) return;
-  // Small lists and few pairs stay with the units' kernel: its sums are not error-free
-  // (each thread adds its terms by Kahan's scheme, a few in no order of size), and there
-  // the slabs' exact sums differ from them by up to 2e-9, from these sizes on by less
-  // than 6e-10.
-  if (P.n_pairs < SLAB_PAIRS || mean_size(pl.lsize) < SLAB_MEAN) return;
+  if (by_unit <= (double)n) return;
+  std::vector<int64_t> at(N + 1, 0);  // first entry of each atom
   for (int u = 0; u < pl.n_units; ++u)
     for (int32_t a : idx[u]) ++at[a + 1];
   for (int64_t a = 0; a < N; ++a) at[a + 1] += at[a];
@@ -1667,6 +1676,7 @@ static amdat_disp_plan* plan_create(amdat_ctx* ctx, const amdat_disp_request* re
     }
     if (pl->S == 0 && pl->NB == 0 && !pl->bulk && pl->n_units > 1 && pl->n_units <= SLAB_UNITS && P.n_pairs > 0)
       plan_slabs(ctx, *pl, P);
+    pl->class_host = std::vector<int32_t>();
     // Default tile.  Every item ends with a block reduction, so moments take chunks of up
     // to 16,384 members while that leaves ten items per SM and the chunk's atoms in all
     // frames fit half the L2 (its pairs run one after the other).  4,096 / 16,384 members,
