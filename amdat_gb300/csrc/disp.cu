@@ -1378,7 +1378,7 @@ static void plan_launch(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P)
     };
     if (pl.slab) {
       const unsigned char* sb = pl.slab_dev.ptr;
-      KernelTimer kt(ctx, "disp_mixed_kernel");
+      KernelTimer kt(ctx, "disp_mixed_kernel"), slab(ctx, "disp_slab_kernel");  // of all moments, and of this route
       disp_slab_kernel<<<(unsigned)pl.n_items, DISP_THREADS, 0, ctx->stream>>>(
           p.u, p.n_pad, p.desc, p.frames, (const int32_t*)sb, (const uint16_t*)(sb + pl.o_place),
           (const uint16_t*)(sb + pl.o_run), pl.n_units, pl.n_items, p.part);
