@@ -247,6 +247,15 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
     if (GS) __syncthreads();
 
     KSum m2 = {0.f, 0.f}, m4 = {0.f, 0.f};
+    // Kahan's sums are not error-free, and longer ones are further off: a thread's terms are
+    // summed 16 at a time, as many as an item of 4,096 members brings, and these sums merged
+    // error-free
+    KSum M2 = {0.f, 0.f}, M4 = {0.f, 0.f};
+    auto merge16 = [&] {
+      M2 = kmerge(M2, m2);
+      M4 = kmerge(M4, m4);
+      m2 = m4 = KSum{0.f, 0.f};
+    };
     KSum fs[MAX_FS];
 #pragma unroll
     for (int s = 0; s < MAX_FS; ++s) fs[s] = KSum{0.f, 0.f};
@@ -305,11 +314,12 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
     } else if (MODE == 0 && !L.idx && (L.first + it.a1) / 4 > (L.first + it.a0 + 3) / 4) {
       // contiguous members: one 16-byte load per plane and frame brings four
       // consecutive atoms (planes start on 128-atom boundaries); the < 4 atoms
-      // before the first and after the last whole quad go one per thread
+      // before the first and after the last whole quad go one per thread.  The sums of
+      // |dr|^2 and |dr|^4 run packed
+      KSum2 k = {0ull, 0ull}, K = {0ull, 0ull};
       auto term = [&](float dx, float dy, float dz) {
         const float e = sq3(dx, dy, dz);
-        kadd(m2, e);
-        kadd(m4, e * e);
+        kadd2(k, pk2(e, e * e));
         if (GS) gs_count(p, hist, dx, dy, dz);
       };
       const int lo = L.first + it.a0, hi = L.first + it.a1;
@@ -317,7 +327,8 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
       const float4* A0 = reinterpret_cast<const float4*>(X0);
       const float4* A1 = reinterpret_cast<const float4*>(X1);
       const int64_t qp = p.n_pad >> 2;  // quads per plane
-      for (int v = v0 + tid; v < v1; v += nthr) {
+      int v = v0 + tid;
+      auto quad = [&] {
         const float4 x0 = __ldg(A0 + v), x1 = __ldg(A1 + v);
         const float4 y0 = __ldg(A0 + qp + v), y1 = __ldg(A1 + qp + v);
         const float4 z0 = __ldg(A0 + 2 * qp + v), z1 = __ldg(A1 + 2 * qp + v);
@@ -325,6 +336,25 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
         term(__fsub_rn(x1.y, x0.y), __fsub_rn(y1.y, y0.y), __fsub_rn(z1.y, z0.y));
         term(__fsub_rn(x1.z, x0.z), __fsub_rn(y1.z, y0.z), __fsub_rn(z1.z, z0.z));
         term(__fsub_rn(x1.w, x0.w), __fsub_rn(y1.w, y0.w), __fsub_rn(z1.w, z0.w));
+        v += nthr;
+      };
+      auto merge_quads = [&] {
+        K = kmerge2(K, k);
+        k = KSum2{0ull, 0ull};
+      };
+      // moments alone wait for their loads: four quads as straight code (64,000 atoms x 1,226
+      // pairs 98 -> 89 us); with G_s the straight code overflows the instruction cache
+      // (32,000 atoms x 187 pairs 29 -> 37 us)
+      while (!GS && v + 3 * nthr < v1) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) quad();
+        if (v < v1) merge_quads();
+      }
+      while (v < v1) {
+        const int stop = min(v1, v + 4 * nthr);
+#pragma unroll 1
+        while (v < stop) quad();
+        if (v < v1) merge_quads();
       }
       const int n_head = 4 * v0 - lo, n_tail = hi - 4 * v1;
       if (tid < n_head + n_tail) {
@@ -333,12 +363,15 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
              __fsub_rn(__ldg(X1 + p.n_pad + atom), __ldg(X0 + p.n_pad + atom)),
              __fsub_rn(__ldg(X1 + 2 * p.n_pad + atom), __ldg(X0 + 2 * p.n_pad + atom)));
       }
+      K = kmerge2(K, k);
+      upk2(K.s, m2.s, m4.s);
+      upk2(K.c, m2.c, m4.c);
       a_start = it.a1;  // nothing left for the loops below
     } else if (MODE == 0 && !GS) {
       // gathered members (index lists): MSD_BATCH atoms' six loads each are
       // issued before any of them is used (the pass is load-latency bound)
       constexpr int MSD_BATCH = 4;  // 8 costs occupancy (registers) and is slower
-      for (; a_start + (MSD_BATCH - 1) * nthr < it.a1; a_start += MSD_BATCH * nthr) {
+      for (int n = 1; a_start + (MSD_BATCH - 1) * nthr < it.a1; a_start += MSD_BATCH * nthr, ++n) {
         int at[MSD_BATCH];
 #pragma unroll
         for (int k = 0; k < MSD_BATCH; ++k)
@@ -357,7 +390,24 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
             kadd(m2, d2);
             kadd(m4, d2 * d2);
           }
+          if (n % (16 / MSD_BATCH) == 0 && a_start + MSD_BATCH * nthr < it.a1) merge16();
         }
+      }
+    } else if (MODE == 0) {
+      // gathered members with G_s
+      while (a_start < it.a1) {
+        const int stop = min(it.a1, a_start + 16 * nthr);
+        for (; a_start < stop; a_start += nthr) {
+          const int atom = L.idx ? __ldg(L.idx + a_start) : L.first + a_start;
+          const float dx = __fsub_rn(__ldg(X1 + atom), __ldg(X0 + atom));
+          const float dy = __fsub_rn(__ldg(X1 + p.n_pad + atom), __ldg(X0 + p.n_pad + atom));
+          const float dz = __fsub_rn(__ldg(X1 + 2 * p.n_pad + atom), __ldg(X0 + 2 * p.n_pad + atom));
+          const float d2 = sq3(dx, dy, dz);
+          kadd(m2, d2);
+          kadd(m4, d2 * d2);
+          gs_count(p, hist, dx, dy, dz);
+        }
+        if (a_start < it.a1) merge16();
       }
     }
     if (MODE == 1 && !GS) {
@@ -477,6 +527,10 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
       }
     }
 
+    if (MODE == 0) {
+      m2 = kmerge(M2, m2);
+      m4 = kmerge(M4, m4);
+    }
     // block reduction of the compensated sums
     const int n_red = 2 + n_fs;
     for (int k = 0; k < n_red; ++k) {

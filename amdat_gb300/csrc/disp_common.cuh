@@ -38,6 +38,21 @@ __device__ __forceinline__ KSum kshfl(KSum v, int off) {
   return o;
 }
 
+// two compensated sums at once (packed FP32): kadd and kmerge of each, bit for bit
+struct KSum2 {
+  uint64_t s, c;
+};
+__device__ __forceinline__ void kadd2(KSum2& k, uint64_t v) {
+  const uint64_t y = sub2(v, k.c), t = add2(k.s, y);
+  k.c = sub2(sub2(t, k.s), y);
+  k.s = t;
+}
+__device__ __forceinline__ KSum2 kmerge2(KSum2 a, KSum2 b) {
+  const uint64_t s = add2(a.s, b.s), bb = sub2(s, a.s);
+  const uint64_t err = add2(sub2(a.s, sub2(s, bb)), sub2(b.s, bb));
+  return KSum2{s, sub2(add2(a.c, b.c), err)};
+}
+
 // fraction of a turn dr/L, as int32 in units of 2^-31 turns (exact wrap)
 __device__ __forceinline__ int32_t turns_fixed(float d, float period) {
   float t = __fdiv_rn(d, period);
