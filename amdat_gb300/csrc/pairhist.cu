@@ -420,8 +420,10 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
     const bool all_y = ny >= g.n.y, all_z = nz >= g.n.z;
     if (all_y) ya = 0, ny = g.n.y;
     if (all_z) za = 0, nz = g.n.z;
-    const float xm = 0.5f * (x0 + x1), ym = 0.5f * (y0 + y1), zm = 0.5f * (z0 + z1);  // the box's centre and half edges
-    const float xh = 0.5f * (x1 - x0), yh = 0.5f * (y1 - y0), zh = 0.5f * (z1 - z0);
+    // the box's centre as members' coordinates round, and its half edges from there
+    const float xm = g.lo.x + 0.5f * (x0 + x1), ym = g.lo.y + 0.5f * (y0 + y1), zm = g.lo.z + 0.5f * (z0 + z1);
+    const float xh = fmaxf(x1 - (xm - g.lo.x), xm - g.lo.x - x0), yh = fmaxf(y1 - (ym - g.lo.y), ym - g.lo.y - y0),
+                zh = fmaxf(z1 - (zm - g.lo.z), zm - g.lo.z - z0);
     int cnt = 0;  // gathered members
     auto go = [&](int n) {  // lanes against the first n gathered members (a multiple of four)
       __syncwarp();
@@ -435,9 +437,8 @@ __global__ void __launch_bounds__(PH_THREADS) pair_hist_groups_kernel(PHParams p
       for (int k = k0; k < k1; k += 32) {
         // only members within reach of the group's box are kept
         const float4 c = k + lane < k1 ? __ldg(P2 + k + lane) : make_float4(nan, nan, nan, 0.f);
-        const float gx = fmaxf(0.f, fabsf(min_image(c.x - g.lo.x - xm, p.box.x)) - xh),
-                    gy = fmaxf(0.f, fabsf(min_image(c.y - g.lo.y - ym, p.box.y)) - yh),
-                    gz = fmaxf(0.f, fabsf(min_image(c.z - g.lo.z - zm, p.box.z)) - zh);
+        const float gx = fmaxf(0.f, fabsf(min_image(c.x - xm, p.box.x)) - xh), gy = fmaxf(0.f, fabsf(min_image(c.y - ym, p.box.y)) - yh),
+                    gz = fmaxf(0.f, fabsf(min_image(c.z - zm, p.box.z)) - zh);
         const bool keep = k + lane < k1 && fmaf(gz, gz, fmaf(gy, gy, gx * gx)) <= G.reach * G.reach;
         const unsigned kept = __ballot_sync(0xffffffffu, keep);
         if (keep) {
