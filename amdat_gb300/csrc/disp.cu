@@ -1213,8 +1213,8 @@ namespace amdat {
 
 // Pairs per item of the slab route.  An item's units are summed once, so items are as
 // large as still fills the chip's three blocks per SM: 12 / 8 / 4 / 2 items per SM give
-// 24 / 23 / 17 / 16 us for 6,474 atoms of 2 types over 289 pairs, 65 / 51 / 44 / 40 for 64
-// nested lists of 15,000 out of 60,000.
+// 27 / 25 / 23 / 21 us for 20,000 atoms of 2 types over 286 pairs, 63 / 60 / 58 / 58 for 64
+// nested lists of up to 30,000 out of 60,000 atoms over 427 pairs.
 static int slab_pairs(const amdat_ctx* ctx, int64_t n_pairs, int64_t n_slabs) {
   const int64_t want = (int64_t)ctx->n_sm * 2;
   return (int)std::min<int64_t>(MAX_PAIRS_PER_ITEM, std::max<int64_t>(1, n_pairs * n_slabs / want));

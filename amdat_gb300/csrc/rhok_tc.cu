@@ -48,7 +48,8 @@
 //                16-column blocks 2 i + warp / 4), then the epilogue
 //   warp 8       producer: bulk copies (cp.async.bulk) of the Z parts and the X/Y
 //                tables of each chunk into a shared-memory ring
-//   warp 9       MMA issuer: 12 tcgen05.mma per chunk, A read from tensor memory
+//   warps 9-10   MMA issuers, one per accumulator (even and odd groups of chunks): 12
+//                tcgen05.mma per chunk, A read from tensor memory
 //   warps 12-19  builders: the A operand of the chunk (W products, FP16 split)
 //                stored into tensor memory (lane quadrant warp % 4; warps 12-15 the
 //                even, 16-19 the odd chunks)

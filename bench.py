@@ -510,11 +510,12 @@ def structure_bench(torch, stream, device, args, n_atoms=100000, box=48.9, frame
         peak = measured_peaks().get("bf16_tflops_sustained", 1700.0)
         out["sk_adjoint_atom_k_per_s"] = r
         out["sk_adjoint_roofline"] = {
-            "bound": "tensor", "achieved": 16 * r / 1e12, "peak": peak, "unit": "TFLOP/s",
-            "frac": 16 * r / 1e12 / peak,
-            "rule": "16 flops per atom x vector (one complex MAC for T and one for the nz-weighted T'); "
-                    "the kernel issues 3 FP16 split passes over whole tiles; peak = measured sustained "
-                    "bf16/fp16 dense rate"}
+            "bound": "tensor", "achieved": 8 * r / 1e12, "peak": peak, "unit": "TFLOP/s",
+            "frac": 8 * r / 1e12 / peak,
+            "rule": "8 flops per atom x vector: eight real multiply-adds (P, Q and the nz-weighted P', "
+                    "Q') per atom and pair of vectors (nx, ny, nz), (-nx, -ny, nz); the kernel issues "
+                    "3 FP16 split passes over whole tiles; peak = measured sustained bf16/fp16 dense "
+                    "rate"}
     if "sk_adjoint_columns_kernel" in kern:
         r = frames * n_atoms * nk / (kern["sk_adjoint_columns_kernel"] / 1e3)
         out["sk_adjoint_atom_k_per_s"] = r
@@ -1061,7 +1062,8 @@ def main():
                  "achieved_rule": "algorithmic: 8 flops (one complex MAC) per atom*vector",
                  "issued_tensor_tflops": r["issued"],
                  "issued_rule": "3 fp16 split passes x 8 flops x atoms x frames x tile entries "
-                                "(64 complex rows x up to 128 nz per tile, incl. tile padding)",
+                                "(64 rows of the half plane x both sign images x up to 96 nz per "
+                                "tile, incl. tile padding)",
                  "peak_source": "bf16_tflops_sustained of MEASURED_PEAKS.json (fp16 and bf16 "
                                 "dense rates are equal; the kernel runs inside a seconds-long step)",
                  "fp32_pipe_peak_tflops": r["fp32_peak_max"]}
