@@ -342,9 +342,12 @@ __global__ void __launch_bounds__(MODE == 0 ? DISP_THREADS : FS_THREADS)
         K = kmerge2(K, k);
         k = KSum2{0ull, 0ull};
       };
-      // moments alone wait for their loads: four quads as straight code (64,000 atoms x 1,226
-      // pairs 98 -> 89 us); with G_s the straight code overflows the instruction cache
-      // (32,000 atoms x 187 pairs 29 -> 37 us)
+      // moments alone wait for their loads: a round of four quads as straight code (64,000
+      // atoms x 1,226 pairs 98 -> 89 us), a plain loop in items of one round at most (32,000 x
+      // 187 pairs 18.7 -> 17.3 us).  With G_s straight code overflows the instruction cache
+      // (32,000 x 187 pairs 29 -> 37 us)
+      if (!GS && v1 - v0 <= 4 * nthr)
+        while (v < v1) quad();
       while (!GS && v + 3 * nthr < v1) {
 #pragma unroll
         for (int n = 0; n < 4; ++n) quad();
@@ -1253,7 +1256,16 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
     n_rows = (size_t)pl.n_units * items.size();
   }
   for (int u = 0; u < pl.n_units && !pl.slab; ++u) {
-    const int nch = (int)std::max<int64_t>(1, ceil_div(pl.usize[u], chunk));
+    int nch = (int)std::max<int64_t>(1, ceil_div(pl.usize[u], chunk));
+    // long items of moments and G_s hold whole rounds of 16 terms per thread, but for a
+    // unit's last (200,000 atoms x 427 pairs 153 us in 13 even items per pair, 140 so)
+    int64_t step = 0;
+    if (pl.S == 0 && !pl.bulk && nch > 1 && chunk > DISP_CHUNK) {
+      step = std::max<int64_t>(1, (pl.usize[u] / nch + DISP_CHUNK / 2) / DISP_CHUNK) * DISP_CHUNK;
+      // not many more items, where the chunk allows longer ones
+      if (4 * ceil_div(pl.usize[u], step) > 5 * nch && step + DISP_CHUNK <= chunk) step += DISP_CHUNK;
+      nch = (int)ceil_div(pl.usize[u], step);
+    }
     const int ppi = (multi_pair && pl.usize[u] > 0 && 2 * pl.usize[u] <= pl.pair_chunk)
                         ? std::min(MAX_PAIRS_PER_ITEM, pl.pair_chunk / pl.usize[u])
                         : 1;
@@ -1263,8 +1275,8 @@ static void plan_tables(amdat_ctx* ctx, amdat_disp_plan& pl, const PairTable& P,
       for (int pr = P.gap_first[g]; pr < P.gap_first[g + 1]; pr += ppi) {
         const int np = std::min(ppi, P.gap_first[g + 1] - pr);
         for (int c = 0; c < nch; ++c) {
-          const int a0 = (int)((int64_t)pl.usize[u] * c / nch);
-          const int a1 = (int)((int64_t)pl.usize[u] * (c + 1) / nch);
+          const int a0 = (int)(step ? c * step : (int64_t)pl.usize[u] * c / nch);
+          const int a1 = (int)(step ? std::min<int64_t>(pl.usize[u], (c + 1) * step) : (int64_t)pl.usize[u] * (c + 1) / nch);
           items.push_back(DispItem{u, pr, a0, a1, np});
           key.push_back(((int64_t)u << 40) | ((int64_t)c << 20) | (int64_t)pr);
         }

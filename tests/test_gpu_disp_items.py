@@ -36,11 +36,11 @@ def test_items_of_one_unit(eng, n, frames, chunk, per_item):
 @pytest.mark.parametrize("gathered", [False, True])
 @pytest.mark.parametrize("bins", [0, 20])
 def test_long_items_keep_small_terms(eng, gathered, bins):
-    """The first 4,096 members of each item of 16,000 move by 2^-15, the others by 1, in
-    every pair of odd gap.  One Kahan sum per thread and item would drop the small terms
-    (3e-10 of the sum); sums of 16 terms merged error-free keep them."""
+    """Items are whole multiples of 4,096 members.  One such round in four moves by 2^-15,
+    the others by 1, in every pair of odd gap.  One Kahan sum per thread and item would drop
+    small terms (3e-10 of the sum); sums of 16 terms merged error-free keep them."""
     n, T = 64000, 40
-    far = np.arange(n) % 16000 >= 4096
+    far = np.arange(n) // 4096 % 4 > 0
     u = np.zeros((T, 2 * n if gathered else n, 3), np.float32)
     members = np.arange(n) * 2 if gathered else np.arange(n)
     u[1::2, members, 0] = np.where(far, np.float32(1.0), np.float32(2.0 ** -15))
