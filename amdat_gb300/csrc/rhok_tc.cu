@@ -547,6 +547,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // host: tile plan over the shell-sorted vector list, launches per frame batch
 // ---------------------------------------------------------------------------
 HalfPlan* half_plan_build(amdat_ctx* ctx, const std::vector<int32_t>& kvec) {
+  // the register split draws on what the block is launched with: a kernel compiled to fewer
+  // would wait for registers that never come
+  cudaFuncAttributes attr;
+  AMDAT_CUDA(cudaFuncGetAttributes(&attr, rhok_tc_kernel));
+  if (attr.numRegs * TC_THREADS < 256 * TC_REG_DRAIN + 128 * TC_REG_MISC + 256 * TC_REG_BUILD)
+    throw Error(AMDAT_ERR_CUDA, "rhok_tc_kernel was compiled to too few registers for its split");
   int nmax = 0;
   for (int v : kvec) nmax = std::max(nmax, std::abs(v));
   const LatticeIndex index(kvec, nmax);
