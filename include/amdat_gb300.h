@@ -105,7 +105,8 @@ amdat_status amdat_scheme_pairs(const amdat_scheme* s, int32_t fullblock, int32_
 amdat_status amdat_create(int32_t device, amdat_ctx** out);
 amdat_status amdat_destroy(amdat_ctx* ctx);
 /* Issue work on an existing cudaStream_t (passed as void*); NULL restores the
- * context's own stream. */
+ * context's own stream, which waits for no other: for inputs made on the default
+ * stream pass cudaStreamLegacy. */
 amdat_status amdat_set_stream(amdat_ctx* ctx, void* cuda_stream);
 amdat_status amdat_synchronize(amdat_ctx* ctx);
 /* number of kernels this context has launched (for launch accounting) */
@@ -113,9 +114,11 @@ amdat_status amdat_launch_count(amdat_ctx* ctx, int64_t* count);
 /* Per-kernel timing: with enable != 0 every hot kernel launch is bracketed by
  * CUDA events on the context's stream; amdat_profile_kernel returns the number
  * of launches and their total device time (ms) since the last reset.  Kernel
- * names: disp_mixed_kernel, disp_plain_kernel, rhok_list_kernel,
- * rhok_lattice_kernel, rhok_tc_kernel, rhok_plain_kernel, isf_pairs_kernel,
- * sk_frames_kernel, pair_hist_kernel, gsmooth_kernel, gsmooth_adjoint_kernel,
+ * names: disp_mixed_kernel (of those the slab launches also as disp_slab_kernel),
+ * disp_plain_kernel, rhok_list_kernel, rhok_lattice_kernel, rhok_tc_kernel,
+ * rhok_plain_kernel, isf_pairs_kernel, sk_frames_kernel, pair_hist_kernel,
+ * pair_hist_cells_kernel (of those the walks also as pair_hist_walk_kernel),
+ * gsmooth_kernel, gsmooth_adjoint_kernel, sk_adjoint_tc_kernel,
  * sk_adjoint_columns_kernel, sk_adjoint_direct_kernel, disp_axes_kernel, disp_bins_kernel.  (No counterpart in the reference, which times commands
  * with time(NULL), e.g. src/control.cpp:2190-2196.) */
 amdat_status amdat_profile_reset(amdat_ctx* ctx, int32_t enable);
